@@ -304,7 +304,7 @@ def run_ours(args):
     elif args.ddadi:
         chosen = "DDADI k, i, j line sweeps, one thread per line"
     elif lk % 100 == 1:
-        chosen = f"cluster lines, {lk // 100} CTAs"
+        chosen = f"warp line wavefront, {lk // 100} CTAs"
     elif lk % 100 == 3:
         chosen = f"pipelined tile wavefront, {lk // 100} tiles"
     else:
@@ -644,7 +644,7 @@ def run_large(args):
         "gpu_launches": per_cycle * args.steps,
         # the dominant kernel of the cycle (profiles/launches_large8blk_512x256x128.md):
         # the LU-SGS line-wavefront sweep; one lower sweep of the largest block, timed alone
-        "roofline": {"bound": "hbm", "kernel": "k_lusgs_lines<double,7> (lower sweep, largest block)",
+        "roofline": {"bound": "hbm", "kernel": "k_flow_sweep<double,7> (upper sweep, largest block)",
                      "achieved": achieved_sweep, "peak": peak, "peak_kind": pkind, "unit": "GB/s",
                      "frac": achieved_sweep / peak,
                      "traffic": None if fp32 else SWEEP_TRAFFIC_PER_CELL * fine_cells[big], "ms_per_launch": ms_sweep,

@@ -28,18 +28,23 @@ struct BlockCtx {
   ff_patch* d_patch = nullptr;
   std::vector<ff_patch> h_patch;
   ff_params prm{};
-  // LU-SGS data in the sweep layout (SW_N x ns) of the upper (sw) and the
-  // lower (swl) sweep, and the increments in it (7 x ns), FP64 or FP32 as
-  // the block's lusgs_fp32 asks.  sw_static: the metric-only part of both
-  // layouts is filled (1 FP64, 2 FP32; 0 after the metrics change).
+  // LU-SGS, warp wavefront (the default sweep): the records of the upper and
+  // the lower sweep, the edge words between tiles and the tile counters, in
+  // the precision lusgs_fp32 asks.  flow_static: the records' face normals
+  // are filled (0 after an allocation or a change of the metrics).
+  void *fup = nullptr, *flo = nullptr, *fedge = nullptr;
+  unsigned* fticket = nullptr;
+  FlowGeom fg{};
+  int flow_static = 0;
+  // LU-SGS, the pipelined and the hyperplane sweep (FINFLO_LUSGS): data in
+  // the sweep layout (SW_N x ns) of the upper (sw) and the lower (swl)
+  // sweep, and the increments in it (7 x ns).  sw_static: the metric-only
+  // part of both layouts is filled (1 FP64, 2 FP32; 0 after the metrics
+  // change).
   double* sw = nullptr;
   double* swl = nullptr;
   double* dwp = nullptr;
   int sw_static = 0;
-  // a second stream of the block: the second sweep's coefficient pass runs
-  // on it beside the first sweep (fork / join events)
-  cudaStream_t aux = nullptr;
-  cudaEvent_t aux_fork = nullptr, aux_join = nullptr;
   // DDADI kernel form per direction (index 1..3 = i, j, k): index into
   // DD_CFG, or -1 for one thread per line; the tuner's time of the chosen
   // form per direction
@@ -51,8 +56,7 @@ struct BlockCtx {
   size_t ns = 0;
   unsigned long long* d_red = nullptr;   // per-block reduction word (FUN1KO CDMAX)
   int coop_threads = 128;       // threads per CTA of the hyperplane sweep (tune_sweep)
-  int use_lines = 0;            // 1: cluster line-wavefront LU-SGS
-  int can_lines = 0;            // the line sweep fits one cluster
+  int use_lines = 1;            // 1: warp line-wavefront LU-SGS
   int can_pipe = 0, use_pipe = 0;   // pipelined tile wavefront possible / chosen
   int pipe_tk = 0;              // its tile height along k (8, 16 or 32 lines)
   bool pipe_stage = false;
@@ -62,8 +66,6 @@ struct BlockCtx {
   int res_shape = 0;            // residual tile shape (RES_SHAPES), chosen by tune_residual
   int res_tuned = 0;
   float sweep_ms[2] = {0.f, 0.f};   // measured upper sweep: lines, best hyperplane
-  LineGeom lg{};
-  bool lines_stage = false;     // the staged line sweep fits (one tile per thread group)
   DevBlock db{};
   cudaGraphExec_t graph = nullptr;
   int graph_fp32 = -1;
@@ -89,7 +91,6 @@ struct Ctx {
   char errmsg[256] = {0};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   long nlaunch = 0;                     // kernel launches issued so far
-  bool side_by_side = false;            // inside fork_join's concurrent chains
   // multi-block: per-block streams for the concurrent chains inside a
   // captured cycle, the device block table and the connection work-list
   std::vector<cudaStream_t> side;
@@ -426,23 +427,46 @@ bool res_batch_ok(Ctx* c) {
 inline double* swd(const BlockCtx* b, int upper) { return upper ? b->sw : b->swl; }
 inline float* swf(const BlockCtx* b, int upper) { return upper ? b->sw32 : b->swl32; }
 
-// Sweep-layout buffers in the block's LU-SGS precision (the other
-// precision's are freed).
+template <typename T>
+void drop(T*& p) {
+  cudaFree((void*)p);
+  p = nullptr;
+}
+
+// The buffers of the block's LU-SGS sweep in its precision and equation
+// count (none for DDADI, whose sweeps work in place).  Records start as
+// zeros (slots without a cell stay so), edge words as the mark of a word not
+// yet there (all bits set).
 int alloc_sweep(Ctx* c, BlockCtx* b) {
   const size_t ns = b->ns;
   b->sw_static = 0;
-  if (b->prm.lusgs_fp32) {
-    cudaFree(b->sw); cudaFree(b->swl); cudaFree(b->dwp);
-    b->sw = nullptr; b->swl = nullptr; b->dwp = nullptr;
-    if (!b->sw32) CK(cudaMalloc(&b->sw32, sizeof(float) * SW_N * ns));
-    if (!b->swl32) CK(cudaMalloc(&b->swl32, sizeof(float) * SW_N * ns));
-    if (!b->dwp32) CK(cudaMalloc(&b->dwp32, sizeof(float) * 7 * ns));
+  b->flow_static = 0;
+  drop(b->sw); drop(b->swl); drop(b->dwp); drop(b->sw32); drop(b->swl32); drop(b->dwp32);
+  drop(b->fup); drop(b->flo); drop(b->fedge);
+  if (b->prm.ddadi) return 0;
+  const bool f32 = b->prm.lusgs_fp32 != 0;
+  if (b->use_lines) {
+    const int nv = b->prm.iturb >= 3 ? 7 : 5;
+    const size_t el = f32 ? sizeof(float) : sizeof(double);
+    const size_t nr = flow_rec_len(b->fg, nv) * el, ne = flow_edge_len(b->fg, nv) * el;
+    CK(cudaMalloc(&b->fup, nr));
+    CK(cudaMalloc(&b->flo, nr));
+    CK(cudaMalloc(&b->fedge, ne));
+    if (!b->fticket) CK(cudaMalloc(&b->fticket, 2 * sizeof(unsigned)));
+    CK(cudaMemsetAsync(b->fup, 0, nr, c->stream));
+    CK(cudaMemsetAsync(b->flo, 0, nr, c->stream));
+    CK(cudaMemsetAsync(b->fedge, 0xff, ne, c->stream));
+    CK(cudaMemsetAsync(b->fticket, 0, 2 * sizeof(unsigned), c->stream));
+    return 0;
+  }
+  if (f32) {
+    CK(cudaMalloc(&b->sw32, sizeof(float) * SW_N * ns));
+    CK(cudaMalloc(&b->swl32, sizeof(float) * SW_N * ns));
+    CK(cudaMalloc(&b->dwp32, sizeof(float) * 7 * ns));
   } else {
-    cudaFree(b->sw32); cudaFree(b->swl32); cudaFree(b->dwp32);
-    b->sw32 = nullptr; b->swl32 = nullptr; b->dwp32 = nullptr;
-    if (!b->sw) CK(cudaMalloc(&b->sw, sizeof(double) * SW_N * ns));
-    if (!b->swl) CK(cudaMalloc(&b->swl, sizeof(double) * SW_N * ns));
-    if (!b->dwp) CK(cudaMalloc(&b->dwp, sizeof(double) * 7 * ns));
+    CK(cudaMalloc(&b->sw, sizeof(double) * SW_N * ns));
+    CK(cudaMalloc(&b->swl, sizeof(double) * SW_N * ns));
+    CK(cudaMalloc(&b->dwp, sizeof(double) * 7 * ns));
   }
   return 0;
 }
@@ -491,244 +515,55 @@ int coop_sweep(Ctx* c, BlockCtx* b, int upper, bool fp32) {
   return coop_sweep_n(c, b, upper, fp32, b->coop_threads);
 }
 
-template <typename CT, int NV>
-cudaError_t launch_lines(cudaLaunchConfig_t* cfg, BlockCtx* b, const CT* sw, CT* dwp, int upper, bool stage) {
-  return stage ? cudaLaunchKernelEx(cfg, k_lusgs_lines<CT, NV, true>, b->db, sw, dwp, upper, b->lg)
-               : cudaLaunchKernelEx(cfg, k_lusgs_lines<CT, NV, false>, b->db, sw, dwp, upper, b->lg);
-}
+constexpr int kMaxDev = 64;
 
-// The staged line sweep for a block swept alone; the unstaged one when
-// several blocks' sweeps run side by side (fork_join).
-int lines_sweep(Ctx* c, BlockCtx* b, int upper, bool fp32) {
-  const bool stage = b->lines_stage && !c->side_by_side;
-  const int nv = b->prm.iturb >= 3 ? 7 : 5;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(b->lg.cs);
-  cfg.blockDim = dim3(LTHREADS * b->lg.ng);
-  cfg.dynamicSmemBytes = lines_smem_bytes(nv, b->lg.tpc, fp32 ? sizeof(float) : sizeof(double), stage);
-  cfg.stream = c->stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = b->lg.cs;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  static const int prio = [] {
-    const char* e = getenv("FINFLO_SWEEP_PRIO");
-    int lo = 0, hi = 0;
-    if (!e || !strcmp(e, "0") || cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess) return 1;
-    return hi;
-  }();
-  if (c->side_by_side && prio <= 0) {   // side by side: the sweeps' CTAs first
-    attr[1].id = cudaLaunchAttributePriority;
-    attr[1].val.priority = prio;
-    cfg.numAttrs = 2;
+// ---- warp wavefront (k_flow_sweep) ------------------------------------------
+// One sweep: one CTA per tile of 16 x 8 lines.
+template <typename CT, int NV>
+int flow_sweep_t(Ctx* c, BlockCtx* b, int upper) {
+  constexpr int sm = (int)flow_smem_bytes(NV, sizeof(CT));
+  static bool set[kMaxDev];
+  if (c->device < 0 || c->device >= kMaxDev) return fail(c, FF_ERR_ARG, "device id");
+  if (!set[c->device]) {
+    CK(cudaFuncSetAttribute(k_flow_sweep<CT, NV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    CK(cudaFuncSetAttribute(k_flow_sweep<CT, NV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    set[c->device] = true;
   }
-  cudaError_t e;
-  if (nv == 7)
-    e = fp32 ? launch_lines<float, 7>(&cfg, b, swf(b, upper), b->dwp32, upper, stage)
-             : launch_lines<double, 7>(&cfg, b, swd(b, upper), b->dwp, upper, stage);
+  CT *up = (CT*)b->fup, *lo = (CT*)b->flo, *ed = (CT*)b->fedge;
+  // PREDGS drops the i+1 coupling of row JMAX unless predgs_full asks for
+  // it; PRKEGS does not drop it
+  if (upper)
+    k_flow_sweep<CT, NV, true><<<b->fg.nb, FTHREADS, sm, c->stream>>>(up, lo, ed, b->fg, b->imax, b->jmax, b->kmax,
+                                                                    !b->prm.predgs_full, b->fticket, c->d_err);
   else
-    e = fp32 ? launch_lines<float, 5>(&cfg, b, swf(b, upper), b->dwp32, upper, stage)
-             : launch_lines<double, 5>(&cfg, b, swd(b, upper), b->dwp, upper, stage);
-  if (e != cudaSuccess) return fail(c, FF_ERR_CUDA, "cluster sweep launch", e);
+    k_flow_sweep<CT, NV, false><<<b->fg.nb, FTHREADS, sm, c->stream>>>(lo, lo, ed, b->fg, b->imax, b->jmax, b->kmax, 0,
+                                                                     b->fticket + 1, c->d_err);
   c->nlaunch++;
   return 0;
 }
 
-constexpr int kMaxDev = 64;
-int g_lines_smem[kMaxDev][4];   // dynamic shared memory granted to k_lusgs_lines<f64|f32, 5|7, *>
+int flow_sweep(Ctx* c, BlockCtx* b, int upper) {
+  const bool f32 = b->prm.lusgs_fp32 != 0;
+  if (b->prm.iturb >= 3) return f32 ? flow_sweep_t<float, 7>(c, b, upper) : flow_sweep_t<double, 7>(c, b, upper);
+  return f32 ? flow_sweep_t<float, 5>(c, b, upper) : flow_sweep_t<double, 5>(c, b, upper);
+}
 
 template <typename CT, int NV>
-int lines_attr_set(Ctx* c, size_t smem) {
-  CK(cudaFuncSetAttribute(k_lusgs_lines<CT, NV, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  CK(cudaFuncSetAttribute(k_lusgs_lines<CT, NV, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  CK(cudaFuncSetAttribute(k_lusgs_lines<CT, NV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  CK(cudaFuncSetAttribute(k_lusgs_lines<CT, NV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  return 0;
+void flow_fill_t(Ctx* c, BlockCtx* b, int what) {
+  const int nb = nblk((long)b->fg.ntiles * b->fg.ns * 32, 256);
+  CT *up = (CT*)b->fup, *lo = (CT*)b->flo;
+  if (what == 0) k_flow_static<CT, NV><<<nb, 256, 0, c->stream>>>(b->db, b->fg, up, lo);
+  else if (what == 1) k_flow_coef<CT, NV><<<nb, 256, 0, c->stream>>>(b->db, b->prm, b->fg, up, lo, b->fticket);
+  else k_flow_out<CT, NV><<<nb, 256, 0, c->stream>>>(b->db, b->fg, lo);
+  c->nlaunch++;
 }
 
-// Kernel attributes are per device, shared by all blocks: only raise them.
-template <int NV>
-int lines_attrs(Ctx* c, size_t sm64, size_t sm32) {
-  int* g = g_lines_smem[c->device] + (NV == 7 ? 2 : 0);
-  if ((int)sm64 > g[0]) {
-    int rc = lines_attr_set<double, NV>(c, sm64);
-    if (rc) return rc;
-    g[0] = (int)sm64;
-  }
-  if ((int)sm32 > g[1]) {
-    int rc = lines_attr_set<float, NV>(c, sm32);
-    if (rc) return rc;
-    g[1] = (int)sm32;
-  }
-  return 0;
-}
-
-// Choose the LU-SGS sweep kernel of a block: the cluster line wavefront
-// when the (j,k) line tiles fit one cluster, else the cooperative hyperplane
-// kernel.  The largest cluster that fits is taken; a smaller cluster only
-// means more tiles per CTA.
-int setup_lines(Ctx* c, BlockCtx* b) {
-  LineGeom lg{};
-  lg.ntj = (b->jmax + LTJ - 1) / LTJ;
-  lg.ntk = (b->kmax + LTK - 1) / LTK;
-  lg.ntiles = lg.ntj * lg.ntk;
-  const int nv = b->prm.iturb >= 3 ? 7 : 5;
-  if (c->device < 0 || c->device >= kMaxDev) return fail(c, FF_ERR_ARG, "device id");
-  // FINFLO_LINES_CS caps the cluster size (16 by default): smaller clusters
-  // let more blocks' sweeps run side by side in a multi-block cycle
-  static const int cs_max = [] {
-    const char* e = getenv("FINFLO_LINES_CS");
-    const int v = e ? atoi(e) : 16;
-    return (v == 1 || v == 2 || v == 4 || v == 8) ? v : 16;
-  }();
-  for (int cs = cs_max; cs >= 1; cs /= 2) {
-    int csz = min(cs, lg.ntiles);
-    int tpc = (lg.ntiles + csz - 1) / csz;
-    int ng = min(tpc, LMAX_TPC);
-    // staging needs one tile per thread group and room for the stage
-    bool stage = tpc == ng && tpc <= LMAX_TPC_STAGE &&
-                 lines_smem_bytes(nv, tpc, sizeof(double), true) <= (size_t)c->smem_optin;
-    size_t sm64 = lines_smem_bytes(nv, tpc, sizeof(double), stage);
-    size_t sm32 = lines_smem_bytes(nv, tpc, sizeof(float), stage);
-    if (sm64 > (size_t)c->smem_optin) continue;
-    int rc = nv == 7 ? lines_attrs<7>(c, sm64, sm32) : lines_attrs<5>(c, sm64, sm32);
-    if (rc) return rc;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(csz);
-    cfg.blockDim = dim3(LTHREADS * ng);
-    cfg.dynamicSmemBytes = sm64;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = csz; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int nclusters = 0;
-    cudaError_t e;
-    if (nv == 7)
-      e = stage ? cudaOccupancyMaxActiveClusters(&nclusters, k_lusgs_lines<double, 7, true>, &cfg)
-                : cudaOccupancyMaxActiveClusters(&nclusters, k_lusgs_lines<double, 7, false>, &cfg);
-    else
-      e = stage ? cudaOccupancyMaxActiveClusters(&nclusters, k_lusgs_lines<double, 5, true>, &cfg)
-                : cudaOccupancyMaxActiveClusters(&nclusters, k_lusgs_lines<double, 5, false>, &cfg);
-    if (e != cudaSuccess || nclusters < 1) {
-      cudaGetLastError();
-      continue;
-    }
-    lg.cs = csz;
-    lg.tpc = tpc;
-    lg.ng = ng;
-    b->lg = lg;
-    b->lines_stage = stage;
-    b->use_lines = 1;
-    b->can_lines = 1;
-    return 0;
-  }
-  b->use_lines = 0;
-  b->can_lines = 0;
-  return 0;
-}
-// ---- all blocks' line sweeps in one launch ----------------------------------
-// The blocks of one multigrid level, swept together by k_lusgs_lines_batch:
-// one cluster per block, every cluster of the launch the same size (the
-// smallest of the blocks' own), so a block with a larger own cluster gets
-// more tiles per CTA.  Returns false when a block cannot be swept this way.
-struct LinesBatchShape {
-  int cs = 0, threads = 0;
-  size_t smem = 0;
-};
-
-bool lines_batch_shape(Ctx* c, const std::vector<BlockCtx*>& v, size_t elem, LinesBatchShape& sh,
-                       std::vector<LineGeom>* geoms = nullptr) {
-  sh = LinesBatchShape{};
-  int cs = 16;
-  for (auto* b : v) {
-    if (!b->can_lines || b->prm.ddadi) return false;
-    cs = min(cs, b->lg.cs);
-  }
-  if (geoms) geoms->clear();
-  int ng_max = 1;
-  for (auto* b : v) {
-    LineGeom g = b->lg;
-    if (g.cs != cs) {
-      g.cs = cs;
-      g.tpc = (g.ntiles + cs - 1) / cs;
-      g.ng = min(g.tpc, LMAX_TPC);
-    }
-    const int nv = b->prm.iturb >= 3 ? 7 : 5;
-    sh.smem = max(sh.smem, lines_smem_bytes(nv, g.tpc, elem, false));
-    ng_max = max(ng_max, g.ng);
-    if (geoms) geoms->push_back(g);
-  }
-  sh.cs = cs;
-  sh.threads = LTHREADS * ng_max;
-  return sh.smem <= (size_t)c->smem_optin;
-}
-
-int g_lb_smem[kMaxDev][4];   // dynamic shared memory granted to k_lusgs_lines_batch<f64|f32, 5|7>
-
-template <typename CT, int NV>
-int lines_batch_launch(Ctx* c, const std::vector<BlockCtx*>& v, int upper) {
-  const bool fp32 = sizeof(CT) == 4;
-  for (size_t s0 = 0; s0 < v.size(); s0 += LB_MAX) {
-    std::vector<BlockCtx*> part(v.begin() + s0, v.begin() + min(v.size(), s0 + LB_MAX));
-    LinesBatchShape sh;
-    std::vector<LineGeom> geoms;
-    if (!lines_batch_shape(c, part, sizeof(CT), sh, &geoms))
-      return fail(c, FF_ERR_ARG, "batched line sweep: a block does not fit");
-    int& granted = g_lb_smem[c->device][(fp32 ? 1 : 0) + (NV == 7 ? 2 : 0)];
-    if ((int)sh.smem > granted) {
-      CK(cudaFuncSetAttribute(k_lusgs_lines_batch<CT, NV>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-      CK(cudaFuncSetAttribute(k_lusgs_lines_batch<CT, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sh.smem));
-      granted = (int)sh.smem;
-    }
-    static LinesBatch lb;   // ~15 KB: kept off the host stack
-    lb = LinesBatch{};
-    lb.n = (int)part.size();
-    for (int n = 0; n < lb.n; n++) {
-      BlockCtx* b = part[n];
-      lb.upper[n] = upper ? (b->prm.predgs_full ? 3 : 1) : 0;
-      lb.lg[n] = geoms[n];
-      lb.sw[n] = fp32 ? (const void*)swf(b, upper) : (const void*)swd(b, upper);
-      lb.dwp[n] = fp32 ? (void*)b->dwp32 : (void*)b->dwp;
-      lb.b[n] = b->db;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(lb.n * sh.cs);
-    cfg.blockDim = dim3(sh.threads);
-    cfg.dynamicSmemBytes = sh.smem;
-    cfg.stream = c->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = sh.cs;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k_lusgs_lines_batch<CT, NV>, lb);
-    if (e != cudaSuccess) return fail(c, FF_ERR_CUDA, "batched line sweep launch", e);
-    c->nlaunch++;
-  }
-  return 0;
-}
-
-// One sweep (upper = 1: PREDGS order, 0: CORRGS) of every block of v, one
-// launch per equation count and precision.
-int lines_batch(Ctx* c, const std::vector<BlockCtx*>& v, int upper) {
-  for (int nv : {5, 7})
-    for (int fp32 : {0, 1}) {
-      std::vector<BlockCtx*> g;
-      for (auto* b : v)
-        if ((b->prm.iturb >= 3 ? 7 : 5) == nv && (b->prm.lusgs_fp32 != 0) == (fp32 != 0)) g.push_back(b);
-      if (g.empty()) continue;
-      int rc = nv == 7 ? (fp32 ? lines_batch_launch<float, 7>(c, g, upper) : lines_batch_launch<double, 7>(c, g, upper))
-                       : (fp32 ? lines_batch_launch<float, 5>(c, g, upper) : lines_batch_launch<double, 5>(c, g, upper));
-      if (rc) return rc;
-    }
-  return 0;
+// what: 0 the records' face normals, 1 their coefficients and right-hand
+// side, 2 the results back into DRO..DE(,DRK,DEPS).
+void flow_fill(Ctx* c, BlockCtx* b, int what) {
+  const bool f32 = b->prm.lusgs_fp32 != 0;
+  if (b->prm.iturb >= 3) f32 ? flow_fill_t<float, 7>(c, b, what) : flow_fill_t<double, 7>(c, b, what);
+  else f32 ? flow_fill_t<float, 5>(c, b, what) : flow_fill_t<double, 5>(c, b, what);
 }
 
 // ---- pipelined tile wavefront (k_lusgs_pipe) ------------------------------
@@ -864,25 +699,38 @@ int setup_pipe(Ctx* c, BlockCtx* b) {
   return 0;
 }
 
-// The metric-only part of both sweep layouts (k_sweep_static), once per
-// block and precision and again after the metrics change.  Inside a stream
-// capture the fill goes into the graph and the layouts stay marked unfilled.
+// The metric-only part of the sweep data, once per block and allocation and
+// again after the metrics change.  Inside a stream capture the fill goes into
+// the graph and the data stays marked unfilled: what captures calls
+// fill_static first.
 void sweep_static(Ctx* c, BlockCtx* b, bool fp32) {
-  const int want = fp32 ? 2 : 1;
-  if (b->sw_static == want) return;
-  for (int up = 0; up < 2; up++) {
-    if (fp32) k_sweep_static<float><<<nblk((long)b->ns, 128), 128, 0, c->stream>>>(b->db, swf(b, up), up);
-    else k_sweep_static<double><<<nblk((long)b->ns, 128), 128, 0, c->stream>>>(b->db, swd(b, up), up);
-    c->nlaunch++;
+  const int want = b->use_lines ? 1 : (fp32 ? 2 : 1);
+  int& have = b->use_lines ? b->flow_static : b->sw_static;
+  if (have == want) return;
+  if (b->use_lines) {
+    flow_fill(c, b, 0);
+  } else {
+    for (int up = 0; up < 2; up++) {
+      if (fp32) k_sweep_static<float><<<nblk((long)b->ns, 128), 128, 0, c->stream>>>(b->db, swf(b, up), up);
+      else k_sweep_static<double><<<nblk((long)b->ns, 128), 128, 0, c->stream>>>(b->db, swd(b, up), up);
+      c->nlaunch++;
+    }
   }
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(c->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) b->sw_static = want;
+  if (cudaStreamIsCapturing(c->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) have = want;
+}
+
+// Before a capture: the metric-only sweep data of every block that lacks it.
+void fill_static(Ctx* c) {
+  for (auto* b : c->blocks)
+    if (!b->prm.ddadi) sweep_static(c, b, b->prm.lusgs_fp32 != 0);
 }
 
 // The metrics of a block changed: its sweep layouts' static part is stale,
 // and so is every captured graph that skipped refilling it.
 void metrics_changed(Ctx* c, BlockCtx* b) {
   b->sw_static = 0;
+  b->flow_static = 0;
   for (auto* x : c->blocks)
     if (x->graph) { cudaGraphExecDestroy(x->graph); x->graph = nullptr; }
   for (auto& g : c->phase_graph)
@@ -894,6 +742,10 @@ void metrics_changed(Ctx* c, BlockCtx* b) {
 // right-hand side copied into it).
 void sweep_coef(Ctx* c, BlockCtx* b, int upper, bool fp32) {
   sweep_static(c, b, fp32);
+  if (b->use_lines) {   // one pass for both sweeps
+    if (upper) flow_fill(c, b, 1);
+    return;
+  }
   if (fp32)
     k_sweep_coef<float><<<nblk((long)b->ns, 128), 128, 0, c->stream>>>(b->db, b->prm, swf(b, upper), b->dwp32, upper);
   else
@@ -901,15 +753,12 @@ void sweep_coef(Ctx* c, BlockCtx* b, int upper, bool fp32) {
   c->nlaunch++;
 }
 
-// Sweep autotuner.  Candidates: the pipelined tile wavefront and the cluster
-// line sweep (each in one cluster of at most 16 CTAs), and the cooperative
-// hyperplane sweep over the whole GPU at 64/128/256 threads per CTA.  Which
-// is fastest depends on the block's shape.  Each candidate is timed (upper
-// sweep in the block's precision, on its current state, in the block's own
-// sweep buffers, which hold nothing between implicit stages) and the
-// fastest is kept.  FINFLO_LUSGS=pipe|lines|hyperplane restricts the choice.
-// Blocks that run side by side in a multi-block cycle use cluster sweeps
-// (see fork_join).
+// The sweep's kernel.  The warp wavefront serves every block; the pipelined
+// tile wavefront (one cluster) and the cooperative hyperplane sweep (the whole
+// GPU, at the fastest of 64/128/256 threads per CTA, timed here) run only
+// where FINFLO_LUSGS=pipe|hyperplane asks for them: both were slower on every
+// block shape tried (128x64x64 SST, FP64, one sweep: warp wavefront
+// 0.150 ms, pipelined 0.74 ms, hyperplanes 2.2 ms).
 // DDADI kernel shapes: the prefetch depth and CTA size of the one thread
 // per line kernels, and the (lines per CTA, cells per chunk) of the
 // producer/consumer kernels the autotuner chooses from.
@@ -1034,77 +883,50 @@ int tune_sweep(Ctx* c, BlockCtx* b) {
   const TuneKey key{c->device, b->imax, b->jmax, b->kmax, b->prm.iturb >= 3 ? 7 : 5, b->prm.lusgs_fp32 != 0,
                     b->prm.ddadi != 0};
   if (b->prm.ddadi) return tune_ddadi(c, b, key);
-  const char* env = getenv("FINFLO_LUSGS");
-  if (!env) {
+  if (b->use_lines || b->use_pipe) return 0;
+  const bool fp32 = b->prm.lusgs_fp32 != 0;
+  {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune_cache.find(key);
-    if (it != g_tune_cache.end() && (!it->second.use_pipe || b->can_pipe) && (!it->second.use_lines || b->can_lines)) {
-      const TuneVal& v = it->second;
-      b->use_pipe = v.use_pipe; b->use_lines = v.use_lines; b->coop_threads = v.coop_threads;
-      b->pipe_ms = v.pipe_ms; b->sweep_ms[0] = v.lines_ms; b->sweep_ms[1] = v.hyp_ms;
+    if (it != g_tune_cache.end()) {
+      b->coop_threads = it->second.coop_threads;
+      b->sweep_ms[1] = it->second.hyp_ms;
       return 0;
     }
   }
-  const bool fp32 = b->prm.lusgs_fp32 != 0;
   const int threads[3] = {64, 128, 256};
-  const bool only = env && (!strcmp(env, "pipe") || !strcmp(env, "lines") || !strcmp(env, "hyperplane"));
-  const bool try_pipe = b->can_pipe && (!only || !strcmp(env, "pipe"));
-  const bool try_lines = b->can_lines && (!only || !strcmp(env, "lines"));
-  bool try_hyp = !only || !strcmp(env, "hyperplane");
-  if (!try_pipe && !try_lines) try_hyp = true;   // nothing else fits
   sweep_coef(c, b, 1, fp32);
-  float best_k[3] = {0.f, 0.f, 0.f};   // pipe, lines, hyperplane
+  float best = 0.f;
   int best_t = b->coop_threads;
-  int rc = 0;
-  b->use_pipe = 0;
-  for (int kind = 0; kind < 5 && !rc; kind++) {
-    if (kind == 0 && !try_pipe) continue;
-    if (kind == 1 && !try_lines) continue;
-    if (kind > 1 && !try_hyp) continue;
-    float best = 0.f;
-    for (int rep = 0; rep < 4 && !rc; rep++) {   // rep 0 warms up
-      cudaEventRecord(c->ev0, c->stream);
-      rc = kind == 0 ? pipe_sweep(c, b, 1, fp32)
-                     : (kind == 1 ? lines_sweep(c, b, 1, fp32) : coop_sweep_n(c, b, 1, fp32, threads[kind - 2]));
-      if (rc) break;
-      cudaEventRecord(c->ev1, c->stream);
-      cudaError_t s2 = cudaEventSynchronize(c->ev1);
-      if (s2 != cudaSuccess) { rc = fail(c, FF_ERR_CUDA, "sweep autotune", s2); break; }
+  for (int k = 0; k < 3; k++) {
+    float bt = 0.f;
+    for (int rep = 0; rep < 4; rep++) {   // rep 0 warms up
+      CK(cudaEventRecord(c->ev0, c->stream));
+      int rc = coop_sweep_n(c, b, 1, fp32, threads[k]);
+      if (rc) return rc;
+      CK(cudaEventRecord(c->ev1, c->stream));
+      CK(cudaEventSynchronize(c->ev1));
       float ms = 0.f;
-      cudaEventElapsedTime(&ms, c->ev0, c->ev1);
-      if (rep > 0) best = rep == 1 ? ms : fminf(best, ms);
+      CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+      if (rep > 0) bt = rep == 1 ? ms : fminf(bt, ms);
     }
-    if (kind < 2) best_k[kind] = best;
-    else if (best_k[2] == 0.f || best < best_k[2]) { best_k[2] = best; best_t = threads[kind - 2]; }
+    if (k == 0 || bt < best) { best = bt; best_t = threads[k]; }
   }
-  if (rc) return rc;
   int herr = 0;
   CK(cudaMemcpy(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (herr) return fail(c, FF_ERR_TIMEOUT, "sweep autotune: a bounded wait gave up");
-  b->pipe_ms = best_k[0];
-  b->sweep_ms[0] = best_k[1];
-  b->sweep_ms[1] = best_k[2];
+  b->sweep_ms[1] = best;
   b->coop_threads = best_t;
-  // the fastest measured candidate
-  int pick = -1;
-  float bt = 0.f;
-  for (int k = 0; k < 3; k++)
-    if (best_k[k] > 0.f && (pick < 0 || best_k[k] < bt)) { pick = k; bt = best_k[k]; }
-  b->use_pipe = pick == 0;
-  b->use_lines = pick == 1 ? 1 : 0;
-  if (pick == 0) b->use_lines = 0;
-  if (!env) {
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune_cache[key] = TuneVal{b->use_pipe, b->use_lines, b->coop_threads, 0, b->pipe_ms, b->sweep_ms[0], b->sweep_ms[1]};
-  }
+  std::lock_guard<std::mutex> lk(g_tune_mu);
+  g_tune_cache[key] = TuneVal{0, 0, best_t, 0, 0.f, 0.f, best};
   return 0;
 }
 
 int sweep(Ctx* c, BlockCtx* b, int upper, bool fp32) {
   // bit 2 of the lower (PREDGS) sweep's flag keeps the row-JMAX i+1 coupling
   if (upper && b->prm.predgs_full) upper |= 2;
-  if (b->use_pipe) return pipe_sweep(c, b, upper, fp32);
-  return b->use_lines ? lines_sweep(c, b, upper, fp32) : coop_sweep(c, b, upper, fp32);
+  if (b->use_lines) return flow_sweep(c, b, upper);
+  return b->use_pipe ? pipe_sweep(c, b, upper, fp32) : coop_sweep(c, b, upper, fp32);
 }
 
 // DDADI (LUSGS=0): the k, i and j lines in turn (imps3.f:320-356), each a
@@ -1180,6 +1002,7 @@ void st_imps_pre(Ctx* c, BlockCtx* b, int level) {
 }
 
 void st_sweep_out(Ctx* c, BlockCtx* b) {
+  if (b->use_lines) return flow_fill(c, b, 2);
   int ncell = b->imax * b->jmax * b->kmax;
   if (b->prm.lusgs_fp32)
     k_sweep_out<float><<<nblk(ncell, 128), 128, 0, c->stream>>>(b->db, b->dwp32, b->prm.iturb >= 3 ? 7 : 5);
@@ -1205,29 +1028,8 @@ int st_imps(Ctx* c, BlockCtx* b, int level, bool divide_cp) {
     if ((rc = ddadi_sweeps(c, b))) return rc;
   } else {
     sweep_coef(c, b, 1, fp32);
-    if (b->use_lines || b->use_pipe) {
-      // the second sweep's coefficients (their own layout buffer; they read
-      // the state, which the first sweep does not change) beside the first
-      // sweep, whose one cluster leaves most SMs free.  Not beside the
-      // cooperative hyperplane sweep, which needs every CTA resident.
-      if (!b->aux) {
-        CK(cudaStreamCreateWithFlags(&b->aux, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&b->aux_fork, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&b->aux_join, cudaEventDisableTiming));
-      }
-      cudaStream_t main = c->stream;
-      CK(cudaEventRecord(b->aux_fork, main));
-      CK(cudaStreamWaitEvent(b->aux, b->aux_fork, 0));
-      c->stream = b->aux;
-      sweep_coef(c, b, 0, fp32);
-      c->stream = main;
-      CK(cudaEventRecord(b->aux_join, b->aux));
-      if ((rc = sweep(c, b, 1, fp32))) return rc;
-      CK(cudaStreamWaitEvent(main, b->aux_join, 0));
-    } else {
-      if ((rc = sweep(c, b, 1, fp32))) return rc;
-      sweep_coef(c, b, 0, fp32);
-    }
+    if ((rc = sweep(c, b, 1, fp32))) return rc;
+    sweep_coef(c, b, 0, fp32);
     if ((rc = sweep(c, b, 0, fp32))) return rc;
     st_sweep_out(c, b);
   }
@@ -1437,7 +1239,6 @@ int fork_join(Ctx* c, int nb, F fn) {
   cudaStream_t main = c->stream;
   CK(cudaEventRecord(c->fork_ev, main));
   int rc = 0;
-  c->side_by_side = true;
   for (int n = 0; n < nb && !rc; n++) {
     CK(cudaStreamWaitEvent(c->side[n], c->fork_ev, 0));
     c->stream = c->side[n];
@@ -1445,7 +1246,6 @@ int fork_join(Ctx* c, int nb, F fn) {
     c->stream = main;
     CK(cudaEventRecord(c->side_ev[n], c->side[n]));
   }
-  c->side_by_side = false;
   c->stream = main;
   for (int n = 0; n < nb; n++) CK(cudaStreamWaitEvent(main, c->side_ev[n], 0));
   return rc;
@@ -1460,7 +1260,6 @@ int fork_n(Ctx* c, int cnt, F fn) {
   cudaStream_t main = c->stream;
   CK(cudaEventRecord(c->fork_ev, main));
   int rc = 0;
-  c->side_by_side = true;
   for (int n = 0; n < cnt && !rc; n++) {
     CK(cudaStreamWaitEvent(c->side[n], c->fork_ev, 0));
     c->stream = c->side[n];
@@ -1468,60 +1267,28 @@ int fork_n(Ctx* c, int cnt, F fn) {
     c->stream = main;
     CK(cudaEventRecord(c->side_ev[n], c->side[n]));
   }
-  c->side_by_side = false;
   c->stream = main;
   for (int n = 0; n < cnt; n++) CK(cudaStreamWaitEvent(main, c->side_ev[n], 0));
   return rc;
 }
 
 // Multi-block cycles in lockstep (the reference's order: each stage of
-// CYCLES over all blocks, ns3c.f:1400-2130) with every level's LU-SGS sweeps
-// as one batched launch, with FINFLO_MB_LOCKSTEP=1.  Needs the cluster line
-// sweep on every block and level.  Not the default: the per-block branches
-// overlap one block's latency-bound sweeps (16 SMs each) with the other
-// blocks' residual work, which lockstep cannot (8-block SST case,
-// 512x256x128 cells: 64.2 ms per V-cycle as branches, 71.8 ms in lockstep).
+// CYCLES over all blocks, ns3c.f:1400-2130) with FINFLO_MB_LOCKSTEP=1, each
+// stage's kernels of the blocks side by side.  Not the default: the per-block
+// branches overlap the latency-bound end of one block's sweeps with the other
+// blocks' residual work.
 bool ls_ok(Ctx* c) {
   const char* env = getenv("FINFLO_MB_LOCKSTEP");
-  const char* kind = getenv("FINFLO_LUSGS");
-  if (!env || strcmp(env, "1") || (kind && strcmp(kind, "lines")) || c->tops.size() < 2) return false;
-  std::vector<std::vector<BlockCtx*>> lv;
-  for (auto* t : c->tops) {
-    size_t m = 0;
-    for (BlockCtx* x = t; x; x = x->coarse, m++) {
-      if (lv.size() <= m) lv.resize(m + 1);
-      lv[m].push_back(x);
-    }
-  }
-  for (auto& v : lv) {
-    LinesBatchShape sh;
-    for (size_t s0 = 0; s0 < v.size(); s0 += LB_MAX) {
-      std::vector<BlockCtx*> part(v.begin() + s0, v.begin() + min(v.size(), s0 + LB_MAX));
-      if (!lines_batch_shape(c, part, sizeof(double), sh)) return false;
-    }
-  }
+  if (!env || strcmp(env, "1") || c->tops.size() < 2) return false;
+  for (auto* t : c->tops)
+    for (BlockCtx* x = t; x; x = x->coarse)
+      if (!x->use_lines || x->prm.ddadi) return false;
   return true;
 }
 
-// IMPS of the blocks v (one level) in lockstep: both sweeps batched.
+// IMPS of the blocks v (one level) in lockstep.
 int ls_imps(Ctx* c, const std::vector<BlockCtx*>& v, int level, bool divide_cp) {
-  const int n = (int)v.size();
-  int rc = fork_n(c, n, [&](int i) {
-    st_imps_pre(c, v[i], level);
-    sweep_coef(c, v[i], 1, v[i]->prm.lusgs_fp32 != 0);
-    return 0;
-  });
-  if (rc || (rc = lines_batch(c, v, 1))) return rc;
-  rc = fork_n(c, n, [&](int i) {
-    sweep_coef(c, v[i], 0, v[i]->prm.lusgs_fp32 != 0);
-    return 0;
-  });
-  if (rc || (rc = lines_batch(c, v, 0))) return rc;
-  return fork_n(c, n, [&](int i) {
-    st_sweep_out(c, v[i]);
-    st_imps_post(c, v[i], divide_cp);
-    return 0;
-  });
+  return fork_n(c, (int)v.size(), [&](int i) { return st_imps(c, v[i], level, divide_cp); });
 }
 
 // mg_body of every level-1 block in lockstep, stage by stage in mg_body's
@@ -1635,7 +1402,7 @@ int mb_cycle(Ctx* c, int icycle) {
   k_reset_acc<<<1, 32, 0, c->stream>>>(c->d_resi, c->d_dromax);
   c->nlaunch++;
   const bool batch = res_batch_ok(c), lockstep = ls_ok(c);
-  if (lockstep) {   // lockstep: RESIDI, RESL2, IMPSDI (batched sweeps), FIN
+  if (lockstep) {   // lockstep: RESIDI, RESL2, IMPSDI, FIN
     rc = fork_n(c, nb, [&](int n) {
       BlockCtx* b = c->tops[n];
       int r;
@@ -1861,8 +1628,8 @@ int ff_destroy(void* ctx) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
     cudaFree(b->base); cudaFree(b->d_patch);
     cudaFree(b->sw); cudaFree(b->swl); cudaFree(b->dwp); cudaFree(b->sw32); cudaFree(b->swl32); cudaFree(b->dwp32);
+    cudaFree(b->fup); cudaFree(b->flo); cudaFree(b->fedge); cudaFree(b->fticket);
     cudaFree(b->d_red);
-    if (b->aux) { cudaStreamDestroy(b->aux); cudaEventDestroy(b->aux_fork); cudaEventDestroy(b->aux_join); }
     delete b;
   }
   drop_phase_graphs(c);
@@ -1890,6 +1657,23 @@ static const char* flux_check(const ff_params* prm) {
   return nullptr;
 }
 
+// The block's sweep kernel: the warp wavefront, or what FINFLO_LUSGS asks for
+// where it fits (the pipelined tile wavefront needs its tiles in one cluster).
+static int pick_sweep(Ctx* c, BlockCtx* b) {
+  const char* env = getenv("FINFLO_LUSGS");
+  b->use_lines = 1;
+  b->use_pipe = 0;
+  if (!env) return 0;
+  if (!strcmp(env, "hyperplane")) b->use_lines = 0;
+  if (!strcmp(env, "pipe")) {
+    int rc = setup_pipe(c, b);
+    if (rc) return rc;
+    b->use_pipe = b->can_pipe;
+    b->use_lines = !b->can_pipe;
+  }
+  return 0;
+}
+
 // The body of ff_block_add: 0 and the new block's id in *id, or an error code.
 static int block_add(Ctx* c, int imax, int jmax, int kmax, int npatch, const ff_patch* patches,
                      const ff_params* prm, int* id) {
@@ -1915,19 +1699,15 @@ static int block_add(Ctx* c, int imax, int jmax, int kmax, int npatch, const ff_
     CK(cudaMemcpyAsync(b->d_patch, patches, sizeof(ff_patch) * npatch, cudaMemcpyHostToDevice, c->stream));
   }
   b->ns = sw_size(imax, jmax, kmax);
-  { int rc = alloc_sweep(c, b); if (rc) return rc; }
+  b->fg = flow_geom(imax, jmax, kmax);
   CK(cudaMalloc(&b->d_red, sizeof(unsigned long long) * 2));
   b->db.imax = imax; b->db.jmax = jmax; b->db.kmax = kmax;
   b->db.is = imax + 4; b->db.il = (imax + 4) * (jmax + 4); b->db.ntot = b->ntot;
   b->db.npatch = npatch; b->db.patch = b->d_patch;
   for (int s = 0; s < FF_NSLOTS; s++) b->db.a[s] = b->base + (size_t)s * b->slot_stride;
   {
-    int rc = setup_lines(c, b);
-    if (rc) return rc;
-    if ((rc = setup_pipe(c, b))) return rc;
-    const char* env = getenv("FINFLO_LUSGS");
-    if (env && strcmp(env, "hyperplane") == 0) b->use_lines = 0;
-    if (env && strcmp(env, "pipe") == 0 && b->can_pipe) { b->use_pipe = 1; b->use_lines = 0; }
+    int rc = pick_sweep(c, b);
+    if (rc || (rc = alloc_sweep(c, b))) return rc;
   }
   b->tuned = 0;
   c->blocks.push_back(b);
@@ -1961,20 +1741,12 @@ int ff_block_params(void* ctx, int blk, const ff_params* prm) {
   if (const char* why = flux_check(prm)) return fail(c, FF_ERR_ARG, why);
   bool nv_changed = (b->prm.iturb >= 3) != (prm->iturb >= 3);
   bool fp_changed = (b->prm.lusgs_fp32 != 0) != (prm->lusgs_fp32 != 0);
-  if ((b->prm.ddadi != 0) != (prm->ddadi != 0)) b->tuned = 0;
+  bool dd_changed = (b->prm.ddadi != 0) != (prm->ddadi != 0);
+  if (dd_changed) b->tuned = 0;
   b->prm = *prm;
-  if (nv_changed) {   // the line sweep's shared memory depends on the equation count
-    int rc = setup_lines(c, b);
-    if (rc) return rc;
-  }
-  if (fp_changed) {
-    int rc = alloc_sweep(c, b);
-    if (rc) return rc;
-  }
-  if (nv_changed || fp_changed) {   // the pipelined sweep's instantiation and shared memory
-    int rc = setup_pipe(c, b);
-    if (rc) return rc;
-    if (!b->can_pipe) b->use_pipe = 0;
+  if (nv_changed || fp_changed || dd_changed) {   // the sweep's kernel and buffers
+    int rc = pick_sweep(c, b);
+    if (rc || (rc = alloc_sweep(c, b))) return rc;
   }
   if (nv_changed || fp_changed) b->tuned = 0;
   // captured cycles of any block may include this one (multigrid levels)
@@ -1989,7 +1761,7 @@ int ff_upload(void* ctx, int blk, int slot, const double* host) {
   BlockCtx* b = getb(c, blk);
   if (!b || slot < 0 || slot >= FF_NSLOTS || !host) return fail(c, FF_ERR_ARG, "ff_upload");
   CK(cudaMemcpyAsync(b->db.a[slot], host, sizeof(double) * b->ntot, cudaMemcpyHostToDevice, c->stream));
-  if (slot >= FF_A1 && slot <= FF_VOL && b->sw_static) metrics_changed(c, b);
+  if (slot >= FF_A1 && slot <= FF_VOL && (b->sw_static || b->flow_static)) metrics_changed(c, b);
   return 0;
 }
 
@@ -2032,7 +1804,13 @@ int ff_synchronize(void* ctx) {
   if (err) {
     cudaMemset(c->d_err, 0, sizeof(int));
     cudaMemset(c->d_bar, 0, 2 * sizeof(unsigned));
-    return fail(c, FF_ERR_TIMEOUT, "LU-SGS grid barrier timed out");
+    for (auto* b : c->blocks)   // edge words of an unfinished warp wavefront
+      if (b->fedge) {
+        const size_t el = b->prm.lusgs_fp32 ? sizeof(float) : sizeof(double);
+        cudaMemset(b->fedge, 0xff, flow_edge_len(b->fg, b->prm.iturb >= 3 ? 7 : 5) * el);
+        cudaMemset(b->fticket, 0, 2 * sizeof(unsigned));
+      }
+    return fail(c, FF_ERR_TIMEOUT, "LU-SGS sweep: a bounded wait timed out");
   }
   return 0;
 }
@@ -2312,6 +2090,7 @@ int ff_cycles(void* ctx, int blk, int ncycles, int icycle0, double* hist, int us
     if (!b->graph || b->graph_fp32 != want) {
       if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
       cudaGraph_t g;
+      fill_static(c);
       CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
       long n0 = c->nlaunch;
       rc = run_cycle(c, b, 2);
@@ -2362,7 +2141,7 @@ int ff_lusgs_kind(void* ctx, int blk) {
   if (b->prm.ddadi)
     return b->dd_cfg[1] < 0 ? 4 : 4 + 100 * (1000 + 100 * b->dd_cfg[3] + 10 * b->dd_cfg[1] + b->dd_cfg[2]);
   if (b->use_pipe) return 3 + 100 * b->pg.ntj * b->pg.ntk;
-  return b->use_lines ? 1 + b->lg.cs * 100 : 2 + b->coop_threads * 100;
+  return b->use_lines ? 1 + b->fg.nb * 100 : 2 + b->coop_threads * 100;
 }
 
 int ff_residual_shape(void* ctx, int blk) {
@@ -2429,6 +2208,7 @@ int ff_mb_phase(void* ctx, int phase, int icycle, int use_graph) {
   } else {
     if (!c->phase_graph[gi]) {
       cudaGraph_t g;
+      fill_static(c);
       CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
       rc = mb_phase(c, phase, 2);
       cudaError_t e = cudaStreamEndCapture(c->stream, &g);
@@ -2485,6 +2265,7 @@ int ff_cycles_all(void* ctx, int ncycles, int icycle0, double* hist, int use_gra
     if (!c->mb_graph || c->mb_graph_n != nb) {
       if (c->mb_graph) { cudaGraphExecDestroy(c->mb_graph); c->mb_graph = nullptr; }
       cudaGraph_t g;
+      fill_static(c);
       CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
       long n0 = c->nlaunch;
       rc = mb_cycle(c, 2);

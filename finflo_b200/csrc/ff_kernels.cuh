@@ -11,8 +11,8 @@
 //                                     layout, then a cooperative persistent
 //                                     kernel marching the i+j+k hyperplanes
 //                                     with a bounded grid barrier
-//   k_lusgs_lines                     the same sweep as a line wavefront in
-//                                     one thread-block cluster (DSMEM)
+//   k_flow_coef + k_flow_sweep        the same sweep as a wavefront of warps
+//                                     (the default, ff_flow.cuh)
 #pragma once
 #include "ff_device.cuh"
 #include <cooperative_groups.h>
@@ -1539,54 +1539,8 @@ __global__ void k_time_levels(DevBlock b, int nv, int mode) {
 
 }  // namespace ff
 
-// ---------------------------------------------------------------------------
-// LU-SGS sweep as a line wavefront inside one thread-block cluster.
-//
-// Thread (lj, lk) of tile t owns the i-line (J, K); at hyperplane m it
-// handles the cell I = m - J - K of its line.  Like the reference (PREDGS
-// imps4.f:345 / CORRGS imps4.f:76) each cell, once solved, produces the
-// split-Jacobian products for its three downstream neighbours: the i
-// neighbour is on the same line (kept in shared memory), the j and k
-// neighbours are the lines (J -/+ 1, K) and (J, K -/+ 1), read at the next
-// plane from shared memory -- from another CTA's shared memory (DSMEM) when
-// the line belongs to another tile.  The triangular system is the
-// reference's (incl. the dropped i+1 coupling in row J = JMAX of PREDGS), so
-// the result equals the hyperplane and slab orders up to rounding.
-//
-// A CTA of the cluster holds tpc tiles, ng = min(tpc, 4) of them side by
-// side (ng x 128 threads; a thread group takes every ng-th tile).  One split
-// cluster barrier per plane: a thread arrives once its products are
-// published and waits only before the next plane.  With STAGE (one tile per
-// thread group) the thread starts, between arrive and wait, the
-// asynchronous copy (cp.async) of its next cell's sweep data (the SW_N
-// values of the sweep layout and the right-hand side) into its own
-// shared-memory slots, so the memory latency of the next plane overlaps the
-// barrier.  Without STAGE the cell data is read from global memory where it
-// is used: the variant for many blocks' sweeps running side by side, where
-// the other blocks' warps hide the latency and the smaller shared-memory
-// footprint keeps more CTAs resident.  The published values are
-// double-buffered, so a plane reads only the previous plane's outputs.
-// ---------------------------------------------------------------------------
-// 16x4-line tiles (two warps, each 16 consecutive J of two K rows, so a
-// warp's sweep-layout loads are two 128-byte runs): a 16-CTA cluster then
-// holds up to 160 tiles in one pass (10 per CTA, 640 threads), enough for
-// the ~9,000 i-lines of a 2.4M-cell block.
-constexpr int LTJ = 16, LTK = 4, LTHREADS = LTJ * LTK;
-constexpr int LMAX_TPC = 10;         // tile groups per CTA (threads per CTA <= 640)
-constexpr int LMAX_TPC_STAGE = 4;    // staged: <= 256 threads, so up to 255 registers a thread
-constexpr int LSTAGE = SW_N + 7;     // staged values per thread: sweep data + right-hand side
-
-struct LineGeom {
-  int ntj, ntk, ntiles, cs, tpc;   // tiles in j/k, cluster size, tiles per CTA
-  int ng;                          // thread groups of 128 per CTA (tiles in parallel)
-};
-
-// Shared memory of k_lusgs_lines: pub [2][tpc][2*NV][128] (j and k
-// products), ydb [tpc][NV][128] (i products), with STAGE (one tile per
-// thread group, ng == tpc) stage [LSTAGE][tpc*128].
-__host__ __device__ inline size_t lines_smem_bytes(int nv, int tpc, size_t elem, bool stage) {
-  return ((size_t)5 * nv + (stage ? LSTAGE : 0)) * tpc * LTHREADS * elem;
-}
+// Staged values per thread of the pipelined sweep: sweep data + right-hand side
+constexpr int LSTAGE = SW_N + 7;
 
 FF_DI void cp_async_ca(void* smem, const double* g) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -1597,8 +1551,6 @@ FF_DI void cp_async_ca(void* smem, const float* g) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(g) : "memory");
 }
 FF_DI void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-FF_DI void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
-FF_DI void cluster_wait_acquire() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
 
 // Start the copy of one cell's sweep data into the thread's stage slots
 // (stride = threads per CTA).
@@ -1615,211 +1567,6 @@ FF_DI void lines_stage(CT* stg, int stride, const CT* __restrict__ sw, const CT*
   for (int v = 0; v < NV; v++) cp_async_ca(stg + (SW_N + v) * stride, dwp + v * ns + S);
 }
 
-FF_DI void prefetch_l2(const void* g) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(g)); }
-
-// The sweep data and right-hand side of one cell into L2 (the values
-// lines_stage copies, without a destination).
-template <typename CT, int NV>
-FF_DI void lines_prefetch_l2(const CT* __restrict__ sw, const CT* dwp, size_t ns, size_t S, int upper) {
-#pragma unroll
-  for (int c = 0; c < SW_N; c++) {
-    if (c == SW_FD && upper) continue;
-    if (NV == 5 && (c == SW_RO || c == SW_SC + 3 || c == SW_SC + 4)) continue;
-    prefetch_l2(sw + c * ns + S);
-  }
-#pragma unroll
-  for (int v = 0; v < NV; v++) prefetch_l2(dwp + v * ns + S);
-}
-
-// A lane's line in one tile slot of its CTA, with the DSMEM sources of its
-// j and k neighbours' products (offsets within one pub buffer).
-template <typename CT>
-struct LineDesc {
-  bool ok, hj, hk;
-  int J, K;
-  const CT* srcj;
-  const CT* srck;
-};
-
-template <typename CT, int NV>
-FF_DI LineDesc<CT> line_desc(const cooperative_groups::cluster_group& cluster, CT* pub, const LineGeom& lg,
-                             int JMAX, int KMAX, int upper, int rank, int q, int lj, int lk) {
-  LineDesc<CT> d;
-  d.ok = false;
-  d.hj = d.hk = false;
-  d.J = d.K = 0;
-  d.srcj = d.srck = pub;
-  const int t = q * lg.cs + rank;
-  if (t >= lg.ntiles) return d;
-  const int tj = t % lg.ntj, tk = t / lg.ntj;
-  d.J = tj * LTJ + lj + 1;
-  d.K = tk * LTK + lk + 1;
-  d.ok = d.J <= JMAX && d.K <= KMAX;
-  d.hj = upper ? (d.J < JMAX) : (d.J > 1);
-  d.hk = upper ? (d.K < KMAX) : (d.K > 1);
-  if (d.ok && d.hj) {   // line (J -/+ 1, K)
-    const int Jn = upper ? d.J + 1 : d.J - 1;
-    const int tn = tk * lg.ntj + (Jn - 1) / LTJ, ln = lk * LTJ + (Jn - 1) % LTJ;
-    d.srcj = cluster.map_shared_rank(pub, tn % lg.cs) + (tn / lg.cs) * 2 * NV * LTHREADS + ln;
-  }
-  if (d.ok && d.hk) {   // line (J, K -/+ 1)
-    const int Kn = upper ? d.K + 1 : d.K - 1;
-    const int tn = ((Kn - 1) / LTK) * lg.ntj + tj, ln = ((Kn - 1) % LTK) * LTJ + lj;
-    d.srck = cluster.map_shared_rank(pub, tn % lg.cs) + ((tn / lg.cs) * 2 * NV + NV) * LTHREADS + ln;
-  }
-  return d;
-}
-
-// The sweep of one block by one cluster.  The CTA may hold more thread
-// groups than lg.ng (a batched launch sized for its largest block): the
-// extra groups own no tile and only take part in the cluster barriers.
-template <typename CT, int NV, bool STAGE>
-FF_DI void lines_body(const DevBlock& b, const CT* __restrict__ sw, CT* dwp, int upper, const LineGeom& lg) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int tpc = lg.tpc, ng = lg.ng, nthr = ng * LTHREADS;
-  CT* pub = reinterpret_cast<CT*>(smem_raw);        // [2][tpc][2*NV][LTHREADS]: bd(NV), ck(NV)
-  CT* ydb = pub + 2 * tpc * 2 * NV * LTHREADS;      // [tpc][NV][LTHREADS]
-  CT* my = ydb + tpc * NV * LTHREADS + threadIdx.x; // stage [LSTAGE][nthr] (STAGE: ng == tpc)
-  const int IMAX = b.imax, JMAX = b.jmax, KMAX = b.kmax;
-  const int W = IMAX + JMAX - 1;
-  const size_t ns = sw_size(IMAX, JMAX, KMAX);
-  const int rank = (int)cluster.block_rank();
-  const int g0 = threadIdx.x / LTHREADS, lane = threadIdx.x % LTHREADS, lj = lane % LTJ, lk = lane / LTJ;
-  const int nplanes = IMAX + JMAX + KMAX - 2;
-  const int pstride = tpc * 2 * NV * LTHREADS;   // one buffer of pub
-  auto plane_cell = [&](int s, int J, int K, int& I, size_t& S) {
-    const int m = upper ? IMAX + JMAX + KMAX - s : 3 + s;
-    I = m - J - K;
-    S = ((size_t)(K - 1) * W + (m - K - 2)) * JMAX + (J - 1);
-    return I >= 1 && I <= IMAX;
-  };
-  for (int q = g0; q < tpc; q += ng)
-#pragma unroll
-    for (int v = 0; v < NV; v++) ydb[(q * NV + v) * LTHREADS + lane] = CT(0);
-  // the thread group's first tile (its only one with STAGE), computed once
-  const LineDesc<CT> d0 = line_desc<CT, NV>(cluster, pub, lg, JMAX, KMAX, upper, rank, g0, lj, lk);
-  if (STAGE) {
-    int I;
-    size_t S;
-    if (d0.ok && plane_cell(0, d0.J, d0.K, I, S)) lines_stage<CT, NV>(my, nthr, sw, dwp, ns, S, upper);
-  }
-  cluster.sync();
-  for (int s = 0; s < nplanes; s++) {
-    const int bin = s & 1, bout = bin ^ 1;
-    for (int q = g0; q < (STAGE ? g0 + 1 : tpc); q += ng) {
-      const LineDesc<CT> ld =
-          STAGE || q == g0 ? d0 : line_desc<CT, NV>(cluster, pub, lg, JMAX, KMAX, upper, rank, q, lj, lk);
-      const int J = ld.J;
-      int I;
-      size_t S;
-      if (!ld.ok || !plane_cell(s, J, ld.K, I, S)) continue;
-      if (STAGE) cp_async_wait_all();
-      // value c of the cell's sweep data (c >= SW_N: right-hand side)
-      auto cd_ = [&](int c) -> CT {
-        if (STAGE) return my[c * nthr];
-        return c < SW_N ? __ldg(sw + c * ns + S) : dwp[(c - SW_N) * ns + S];
-      };
-      // PREDGS drops the i+1 coupling of row J = JMAX unless bit 2 of upper
-      // (predgs_full) asks for it; PRKEGS does not drop it
-      const bool hy = upper ? (I < IMAX && (NV == 7 || J < JMAX || (upper & 2))) : (I > 1);
-      // ---- consume: neighbour contributions of the previous plane ----
-      CT yd[NV], bd[NV], ck[NV];
-#pragma unroll
-      for (int v = 0; v < NV; v++) {
-        yd[v] = hy ? ydb[(q * NV + v) * LTHREADS + lane] : CT(0);
-        bd[v] = ld.hj ? ld.srcj[bin * pstride + v * LTHREADS] : CT(0);
-        ck[v] = ld.hk ? ld.srck[bin * pstride + v * LTHREADS] : CT(0);
-      }
-      // ---- solve the cell ----
-      const CT dt1 = cd_(SW_DT1), vol = cd_(SW_VOL), fd = upper ? CT(1) : cd_(SW_FD);
-      const CT a1 = cd_(SW_A1), a2 = cd_(SW_A2), a3 = cd_(SW_A3);
-      const CT scinv = cd_(SW_SCINV), scinp = cd_(SW_SCINP);
-      CT res[NV];
-#pragma unroll
-      for (int v = 0; v < NV; v++) {
-        CT cd = cd_(SW_N + v) * fd;
-        CT x = upper ? (-dt1 * a3 * ck[v] + vol * cd) : (dt1 * a3 * ck[v] + vol * cd);
-        x = upper ? x - dt1 * (a1 * yd[v] + a2 * bd[v]) : x + dt1 * (a1 * yd[v] + a2 * bd[v]);
-        res[v] = x * (v == 4 ? scinp : scinv);
-        dwp[v * ns + S] = res[v];
-      }
-      // ---- produce: contributions to the three downstream neighbours ----
-      CT sc[5];
-#pragma unroll
-      for (int c = 0; c < (NV == 7 ? 5 : 3); c++) sc[c] = cd_(SW_SC + c);
-      const CT ro = NV == 7 ? cd_(SW_RO) : CT(0);
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        CT f[3], l[3];
-#pragma unroll
-        for (int c = 0; c < 3; c++) f[c] = cd_(SW_F + 3 * d + c);
-#pragma unroll
-        for (int e = 0; e < 3; e++) l[e] = cd_(SW_L + 3 * d + e);
-        CT out[NV];
-        nb_product_pre<CT, NV>(out, res, f, sc, ro, l[0], l[1], l[2]);
-        if (d == 0) {
-#pragma unroll
-          for (int v = 0; v < NV; v++) ydb[(q * NV + v) * LTHREADS + lane] = out[v];
-        } else {
-#pragma unroll
-          for (int v = 0; v < NV; v++)
-            pub[bout * pstride + (q * 2 * NV + (d == 1 ? 0 : NV) + v) * LTHREADS + lane] = out[v];
-        }
-      }
-    }
-    cluster_arrive_release();
-    // the next plane's sweep data, in flight while the other CTAs finish
-    if (STAGE && s + 1 < nplanes && d0.ok) {
-      int I;
-      size_t S;
-      if (plane_cell(s + 1, d0.J, d0.K, I, S)) lines_stage<CT, NV>(my, nthr, sw, dwp, ns, S, upper);
-    }
-    if (!STAGE && s + 1 < nplanes) {
-      // unstaged: pull the next plane's cells of every tile of the thread
-      // group into L2 (a hint: no registers or shared memory held)
-      for (int q = g0; q < tpc; q += ng) {
-        const int t = q * lg.cs + rank;
-        if (t >= lg.ntiles) break;
-        const int J = (t % lg.ntj) * LTJ + lj + 1, K = (t / lg.ntj) * LTK + lk + 1;
-        int I;
-        size_t S;
-        if (J > JMAX || K > KMAX || !plane_cell(s + 1, J, K, I, S)) continue;
-        lines_prefetch_l2<CT, NV>(sw, dwp, ns, S, upper);
-      }
-    }
-    cluster_wait_acquire();
-  }
-}
-
-template <typename CT, int NV, bool STAGE>
-__global__ void __launch_bounds__(LTHREADS * (STAGE ? LMAX_TPC_STAGE : LMAX_TPC))
-    k_lusgs_lines(DevBlock b, const CT* __restrict__ sw, CT* dwp, int upper, LineGeom lg) {
-  lines_body<CT, NV, STAGE>(b, sw, dwp, upper, lg);
-}
-
-// Several blocks' sweeps in one launch (a block work-list): cluster e of
-// the grid sweeps entry e.  All entries share the cluster size; each has its
-// own tile geometry and sweep flags.
-constexpr int LB_MAX = 16;
-struct LinesBatch {
-  int n;
-  int upper[LB_MAX];
-  LineGeom lg[LB_MAX];
-  const void* sw[LB_MAX];
-  void* dwp[LB_MAX];
-  DevBlock b[LB_MAX];
-};
-
-template <typename CT, int NV>
-__global__ void __launch_bounds__(LTHREADS * LMAX_TPC)
-    k_lusgs_lines_batch(const __grid_constant__ LinesBatch lb) {
-  const int e = blockIdx.x / lb.lg[0].cs;
-  if (e >= lb.n) return;   // whole clusters only: the launch has n * cs CTAs
-  lines_body<CT, NV, false>(lb.b[e], static_cast<const CT*>(lb.sw[e]), static_cast<CT*>(lb.dwp[e]), lb.upper[e],
-                            lb.lg[e]);
-}
-
 #include "ff_pipe.cuh"
+#include "ff_flow.cuh"
 #include "ff_ddadi.cuh"

@@ -223,15 +223,16 @@ int ff_time_cycles_all(void *ctx, int ncycles, float *ms, int *launches_per_cycl
 /* Timing helpers (CUDA events on the context stream); ff_cycle_launches is
  * the number of kernel launches in one graph-captured cycle. */
 int ff_cycle_launches(void *ctx, int blk);
-/* LU-SGS sweep kernel of a block: 1 + 100*cluster_size = cluster line
- * wavefront, 2 + 100*threads_per_CTA = cooperative hyperplane kernel. */
-/* The autotuner's measured upper-sweep times in ms {cluster lines, fastest
- * cooperative hyperplane} of a block (zeros until its first ff_cycles call
- * or sweep stage timing; lines 0 where the lines do not fit a cluster). */
+/* LU-SGS sweep kernel of a block: 1 + 100*CTAs = line wavefront of warps
+ * (the default), 2 + 100*threads_per_CTA = cooperative hyperplane kernel. */
+/* The measured upper-sweep times in ms {lines, fastest cooperative
+ * hyperplane} of a block, zero for a kernel that was not timed: the line
+ * wavefront is taken without timing it, the hyperplane kernel's CTA size is
+ * timed at the first ff_cycles call where FINFLO_LUSGS asks for it. */
 int ff_sweep_tuning(void *ctx, int blk, float *ms2);
-/* The autotuner's measured upper-sweep times in ms {pipelined tile
- * wavefront, cluster lines, fastest cooperative hyperplane} (zero where not
- * tried).  LU-SGS kind 3 + 100*tiles = the pipelined tile wavefront.
+/* The measured upper-sweep times in ms {pipelined tile wavefront, lines,
+ * fastest cooperative hyperplane} (zero where not timed).  LU-SGS kind 3 +
+ * 100*tiles = the pipelined tile wavefront.
  * DDADI blocks (prm->ddadi = 1): the tuned PRED+CORR time per direction
  * {k, i, j}, and kind 4 + 100*(1000 + 100*fk + 10*fi + fj) with f the
  * chosen producer/consumer form per direction (0: 32 lines x 4 cells per
