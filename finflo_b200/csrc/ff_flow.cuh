@@ -15,14 +15,17 @@
 // the cluster barrier.  Here nothing waits for a whole plane: a CTA starts as
 // soon as its two upstream CTAs have passed its first cells and then runs at
 // their pace.  A step of the chain is a warp's instructions for one cell a
-// lane and a CTA barrier (0.36 us in FP64, 0.32 us in FP32), and each CTA on
-// the way adds the lag of its edge words, 1.5 to 4 us.  With one warp per CTA
-// (8 x 4 lines) the lags were two thirds of the sweep of a 128x64x64 block,
-// 0.164 ms against 0.046 ms with the edges left out; 16 x 8 lines halve the
-// CTAs on the way and are what fits the shared memory in FP64 with seven
-// equations.  One sweep, B200, 128x64x64 cells with seven equations: 0.150 ms
-// in FP64 and 0.113 ms in FP32 (cluster lines 0.588 ms); 64x32x32 with five:
-// 0.063 ms (0.223 ms); 248x136x72 with seven: 0.272 ms.
+// lane and a CTA barrier, 0.25 us in FP64 (a dependent multiply-add alone is
+// ~25 cycles) and 0.21 us in FP32, and each CTA on the way adds the lag of its
+// edge words, ~3 us.  The CTA's shape weighs the two: with 8 x 4 lines the
+// lags cost more, with 16 x 8 lines the step, whose four warps then share the
+// shared memory's bandwidth (one sweep of a 128x64x64 block with seven
+// equations, FP64: 8 x 4 0.129 ms, 8 x 8 0.114 ms, 16 x 4 0.150 ms, 16 x 8
+// 0.134 ms).  Loading the next record into registers a step ahead made the
+// step longer (0.156 ms at 16 x 8), as did a step barrier split into arrival
+// and wait on an mbarrier.  One sweep, B200: 128x64x64 cells, seven equations,
+// 0.114 ms in FP64 and 0.099 ms in FP32 (cluster lines 0.588 ms); 64x32x32,
+// five equations, 0.046 ms (0.223 ms); 248x136x72, seven, 0.249 ms.
 //
 // Between CTAs the products of the edge lines go through global memory (L2)
 // and carry their own arrival: every word of the edge buffer holds a mark (all
@@ -49,11 +52,11 @@
 #pragma once
 
 constexpr int FTJ = 8, FTK = 4;     // lines of a warp tile along j and k (32 lanes)
-constexpr int FWJ = 2, FWK = 2;     // warp tiles of a CTA along j and k
+constexpr int FWJ = 1, FWK = 2;     // warp tiles of a CTA along j and k
 constexpr int FW = FWJ * FWK, FBJ = FTJ * FWJ, FBK = FTK * FWK;   // its warps, its lines along j and k
 constexpr int FIO = 64;             // threads that fetch, and that publish, the edge words
 constexpr int FTHREADS = FW * 32 + 2 * FIO;
-constexpr int FD = 6;               // ring slots: up to FD - 2 steps of record copies in flight
+constexpr int FD = 6;               // ring slots: up to FD - 1 steps of record copies in flight
 constexpr int FPF = 2;              // steps between an edge request and its use
 constexpr int FHS = FW * 32 + (FBJ > FBK ? FBJ : FBK);   // products of one value: the CTA's lines + the incoming edge
 
@@ -267,8 +270,8 @@ FF_DI void flow_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar
 // sweep, its own for the lower one).  grid = CTA tiles.  The first FW warps
 // compute and do nothing else: with one warp doing everything its own
 // instruction stream was the chain, 0.55 us a step.  The next FIO threads
-// fetch the incoming edge words one step ahead and wait for the records two
-// steps ahead; the last FIO publish the outgoing edge words of the step before and start the
+// fetch the incoming edge words and wait for the records, one step ahead; the
+// last FIO publish the outgoing edge words of the step before and start the
 // record copies.
 template <typename CT, int NV, bool UP>
 __global__ void __launch_bounds__(FTHREADS) k_flow_sweep(const CT* rec, CT* res, CT* edge, FlowGeom g, int imax,
@@ -326,60 +329,39 @@ __global__ void __launch_bounds__(FTHREADS) k_flow_sweep(const CT* rec, CT* res,
     CT* nj = pj + warp * 32 + lane;
     CT* nk = pk + warp * 32 + lane;
     CT* o = res + ((size_t)max(wt, 0) * ns + (UP ? ns - 1 : 0)) * ROW + lane;
-    // The record of a step is read, and the part of the solve that waits for no other line done, in the step before.
-    CT base[NV], l[3], f[9], b2, b3, sp, k0, hr, k4, y, h3, h2;
-    auto load = [&](int T, const CT* yi) {
-      if (wt < 0 || (unsigned)(T - off) >= (unsigned)ns) return;
-      const CT* my = ring + ((T % FD) * FW + warp) * ROW + lane;
-      const CT al = my[R::AL * 32], b1 = my[R::B * 32];
-      sp = my[R::SP * 32];
-#pragma unroll
-      for (int v = 0; v < NV; v++) base[v] = al * my[v * 32] + b1 * yi[v];
-      base[4] = base[4] * sp;
-      b2 = my[(R::B + 1) * 32];
-      b3 = my[(R::B + 2) * 32];
-#pragma unroll
-      for (int d = 0; d < 3; d++) l[d] = my[(R::L + d) * 32];
-#pragma unroll
-      for (int d = 0; d < 9; d++) f[d] = my[(R::F + d) * 32];
-      k0 = my[R::K0 * 32];
-      hr = my[R::HR * 32];
-      k4 = my[R::K4 * 32];
-      if constexpr (NV == 7) {
-        y = my[R::Y * 32];
-        h3 = my[R::H3 * 32];
-        h2 = my[R::H2 * 32];
-      }
-    };
     CT yi[NV];
 #pragma unroll
-    for (int v = 0; v < NV; v++) yi[v] = base[v] = CT(0);
-    __syncthreads();   // the records of steps 0 and 1, the incoming words of step 0
-    load(0, yi);
+    for (int v = 0; v < NV; v++) yi[v] = CT(0);
+    __syncthreads();   // the record and the incoming words of step 0
     for (int T = 0; T < nbs; T++) {
-      const bool act = wt >= 0 && (unsigned)(T - off) < (unsigned)ns;
-      CT x[NV];
-      if (act) {
+      if (wt >= 0 && (unsigned)(T - off) < (unsigned)ns) {
+        const CT* my = ring + ((T % FD) * FW + warp) * ROW + lane;
         const int bi = (T & 1) * PB, bo = PB - bi;
-        const CT s2 = b2 * sp, s3 = b3 * sp;
+        const CT al = my[R::AL * 32], b1 = my[R::B * 32], b2 = my[(R::B + 1) * 32], b3 = my[(R::B + 2) * 32];
+        CT x[NV];
 #pragma unroll
-        for (int v = 0; v < NV; v++)
-          x[v] = (base[v] + (v == 4 ? s3 : b3) * qk[bi + v * FHS]) + (v == 4 ? s2 : b2) * qj[bi + v * FHS];
-        const CT p = hr * x[4];
+        for (int v = 0; v < NV; v++) x[v] = al * my[v * 32] + b1 * yi[v];
+#pragma unroll
+        for (int v = 0; v < NV; v++) x[v] = (x[v] + b3 * qk[bi + v * FHS]) + b2 * qj[bi + v * FHS];
+        x[4] = x[4] * my[R::SP * 32];
+        const CT k0 = my[R::K0 * 32], k4 = my[R::K4 * 32], p = my[R::HR * 32] * x[4];
         CT w = x[4];
-        if constexpr (NV == 7) w = (y * x[4] - h3 * x[5]) - h2 * x[0];
+        if constexpr (NV == 7) w = (my[R::Y * 32] * x[4] - my[R::H3 * 32] * x[5]) - my[R::H2 * 32] * x[0];
         // the k and j products first: other lines wait for them
 #pragma unroll
         for (int d = 2; d >= 0; d--) {
-          const CT z = f[3 * d] * x[1] + f[3 * d + 1] * x[2] + f[3 * d + 2] * x[3];
+          const CT l = my[(R::L + d) * 32];
+          const CT nx = my[(R::F + 3 * d) * 32], ny = my[(R::F + 3 * d + 1) * 32], nz = my[(R::F + 3 * d + 2) * 32];
+          const CT z = nx * x[1] + ny * x[2] + nz * x[3];
           CT out[NV];
-          out[0] = l[d] * x[0] + k0 * z;
-#pragma unroll
-          for (int v = 0; v < 3; v++) out[1 + v] = l[d] * x[1 + v] + f[3 * d + v] * p;
-          out[4] = l[d] * w + k4 * z;
+          out[0] = l * x[0] + k0 * z;
+          out[1] = l * x[1] + nx * p;
+          out[2] = l * x[2] + ny * p;
+          out[3] = l * x[3] + nz * p;
+          out[4] = l * w + k4 * z;
           if constexpr (NV == 7) {
-            out[5] = l[d] * x[5];
-            out[6] = l[d] * x[6];
+            out[5] = l * x[5];
+            out[6] = l * x[6];
           }
 #pragma unroll
           for (int v = 0; v < NV; v++) {
@@ -391,9 +373,6 @@ __global__ void __launch_bounds__(FTHREADS) k_flow_sweep(const CT* rec, CT* res,
         if (any_drop && J == jmax)   // PREDGS's dropped i+1 coupling (imps4.f:1460-1466)
 #pragma unroll
           for (int v = 0; v < NV; v++) yi[v] = CT(0);
-      }
-      load(T + 1, yi);
-      if (act) {
         if (line && (unsigned)(T - mj - mk) < (unsigned)imax)
 #pragma unroll
           for (int v = 0; v < NV; v++) o[v * 32] = x[v];
@@ -484,7 +463,6 @@ __global__ void __launch_bounds__(FTHREADS) k_flow_sweep(const CT* rec, CT* res,
 #pragma unroll
     for (int u = 1; u <= FPF; u++) request(u, ew[u % FPF]);
     record(0);
-    record(1);
     __syncthreads();
     for (int tb = 0; tb < nbs; tb += FPF) {
 #pragma unroll
@@ -493,7 +471,7 @@ __global__ void __launch_bounds__(FTHREADS) k_flow_sweep(const CT* rec, CT* res,
         if (T >= nbs) break;
         take(T + 1, ew[(u + 1) % FPF]);
         request(T + 1 + FPF, ew[(u + 1) % FPF]);
-        record(T + 2);
+        record(T + 1);
         __syncthreads();
       }
     }
@@ -544,8 +522,7 @@ __global__ void __launch_bounds__(FTHREADS) k_flow_sweep(const CT* rec, CT* res,
   for (int T = 0; T < nbs; T++) {
     if (T > 0) {
       publish(T - 1);
-      if (T == 1) copy(FD);   // step T's record is in registers since step T - 1, step 0's since step 0
-      copy(T + FD);
+      copy(T - 1 + FD);
     }
     __syncthreads();
   }

@@ -518,7 +518,7 @@ int coop_sweep(Ctx* c, BlockCtx* b, int upper, bool fp32) {
 constexpr int kMaxDev = 64;
 
 // ---- warp wavefront (k_flow_sweep) ------------------------------------------
-// One sweep: one CTA per tile of 16 x 8 lines.
+// One sweep: one CTA per tile of 8 x 8 lines.
 template <typename CT, int NV>
 int flow_sweep_t(Ctx* c, BlockCtx* b, int upper) {
   constexpr int sm = (int)flow_smem_bytes(NV, sizeof(CT));
@@ -758,7 +758,7 @@ void sweep_coef(Ctx* c, BlockCtx* b, int upper, bool fp32) {
 // GPU, at the fastest of 64/128/256 threads per CTA, timed here) run only
 // where FINFLO_LUSGS=pipe|hyperplane asks for them: both were slower on every
 // block shape tried (128x64x64 SST, FP64, one sweep: warp wavefront
-// 0.150 ms, pipelined 0.74 ms, hyperplanes 2.2 ms).
+// 0.114 ms, pipelined 0.74 ms, hyperplanes 2.2 ms).
 // DDADI kernel shapes: the prefetch depth and CTA size of the one thread
 // per line kernels, and the (lines per CTA, cells per chunk) of the
 // producer/consumer kernels the autotuner chooses from.
