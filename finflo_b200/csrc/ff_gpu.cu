@@ -109,6 +109,9 @@ struct Ctx {
   bool halo_pack = false, halo_unpack = false;
   double *halo_send = nullptr, *halo_recv = nullptr;
   cudaGraphExec_t phase_graph[2] = {nullptr, nullptr};
+  // scratch of the set-up calls (synchronous, so one buffer serves them all)
+  void* setup = nullptr;
+  size_t setup_bytes = 0;
 };
 
 int fail(Ctx* c, int code, const char* what, cudaError_t e = cudaSuccess) {
@@ -1636,6 +1639,7 @@ int ff_destroy(void* ctx) {
   cudaFree(c->d_halo);
   for (size_t n = 0; n < c->side.size(); n++) { cudaStreamDestroy(c->side[n]); cudaEventDestroy(c->side_ev[n]); }
   if (c->fork_ev) cudaEventDestroy(c->fork_ev);
+  cudaFree(c->setup);
   cudaFree(c->d_blocks); cudaFree(c->d_conn);
   cudaFree(c->d_bar); cudaFree(c->d_err); cudaFree(c->d_resi); cudaFree(c->d_dromax);
   cudaFree(c->d_hist); cudaFree(c->d_hist_pos);
@@ -1915,6 +1919,31 @@ int ff_resl2(void* ctx, int blk, double* out5) {
   return 0;
 }
 
+// Device scratch of a set-up call: kept from call to call up to SETUP_KEEP
+// (three cudaMalloc / cudaFree pairs took most of a 128x64x64 block's
+// metrics, 5.0 ms of which 0.29 ms were kernels), a larger one is given
+// back by setup_done.
+static constexpr size_t SETUP_KEEP = 256u << 20;
+static cudaError_t setup_buf(Ctx* c, size_t bytes, double** p) {
+  *p = nullptr;
+  if (bytes > c->setup_bytes) {
+    cudaFree(c->setup);
+    c->setup = nullptr;
+    c->setup_bytes = 0;
+    cudaError_t e = cudaMalloc(&c->setup, bytes);
+    if (e != cudaSuccess) return e;
+    c->setup_bytes = bytes;
+  }
+  *p = (double*)c->setup;
+  return cudaSuccess;
+}
+static void setup_done(Ctx* c) {
+  if (c->setup_bytes <= SETUP_KEEP) return;
+  cudaFree(c->setup);
+  c->setup = nullptr;
+  c->setup_bytes = 0;
+}
+
 int ff_block_metrics(void* ctx, int blk, const double* xyz) {
   Ctx* c = (Ctx*)ctx;
   BlockCtx* b = getb(c, blk);
@@ -1922,18 +1951,17 @@ int ff_block_metrics(void* ctx, int blk, const double* xyz) {
   metrics_changed(c, b);
   const GridDims g{b->imax + 1, b->jmax + 1, b->kmax + 1};
   const size_t nn = (size_t)g.ni * g.nj * g.nk, ne = (size_t)(g.ni + 4) * (g.nj + 4) * (g.nk + 4);
-  double *dn = nullptr, *de = nullptr;
-  CK(cudaMalloc(&dn, 3 * nn * sizeof(double)));
-  if (cudaMalloc(&de, 3 * ne * sizeof(double)) != cudaSuccess) { cudaFree(dn); return fail(c, FF_ERR_CUDA, "ff_block_metrics"); }
+  double* dn = nullptr;
+  CK(setup_buf(c, 3 * (nn + ne) * sizeof(double), &dn));
+  double* de = dn + 3 * nn;
   cudaError_t e = cudaMemcpyAsync(dn, xyz, 3 * nn * sizeof(double), cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) {
     k_extend_nodes<<<nblk((long)ne, 256), 256, 0, c->stream>>>(dn, de, g);
-    k_cell_metrics<<<nblk((long)b->ntot, 256), 256, 0, c->stream>>>(b->db, de);
+    k_cell_metrics<<<nblk((long)b->ntot, 256), 256, 0, c->stream>>>(b->db, de, 2);
     c->nlaunch += 2;
     e = cudaStreamSynchronize(c->stream);
   }
-  cudaFree(dn);
-  cudaFree(de);
+  setup_done(c);
   if (e != cudaSuccess) return fail(c, FF_ERR_CUDA, "ff_block_metrics", e);
   CK(cudaGetLastError());
   return 0;
@@ -1951,45 +1979,35 @@ int ff_block_metrics_levels(void* ctx, int blk, int nlev, const double* xyz) {
   const GridDims g{b->imax + 1, b->jmax + 1, b->kmax + 1};
   const size_t nn = (size_t)g.ni * g.nj * g.nk;
   RawDims r{b->imax + 2 * ng, b->jmax + 2 * ng, b->kmax + 2 * ng};
-  const size_t ne = (size_t)(r.ci + 1) * (r.cj + 1) * (r.ck + 1);
-  double *dn = nullptr, *de = nullptr, *raw = nullptr, *raw2 = nullptr;
-  auto cleanup = [&]() { cudaFree(dn); cudaFree(de); cudaFree(raw); cudaFree(raw2); };
-  if (cudaMalloc(&dn, 3 * nn * sizeof(double)) != cudaSuccess || cudaMalloc(&de, 3 * ne * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&raw, RW_N * r.n() * sizeof(double)) != cudaSuccess) {
-    cleanup();
-    return fail(c, FF_ERR_CUDA, "ff_block_metrics_levels: device memory");
+  for (int l = 0, lng = ng; l + 1 < nlev; l++, lng /= 2) {
+    const RawDims rc{r.ci >> (l + 1), r.cj >> (l + 1), r.ck >> (l + 1)};
+    if (lv[l + 1]->imax + lng != rc.ci || lv[l + 1]->jmax + lng != rc.cj || lv[l + 1]->kmax + lng != rc.ck)
+      return fail(c, FF_ERR_ARG, "ff_block_metrics_levels: a coarse level does not halve the finer one");
   }
+  const size_t ne = (size_t)(r.ci + 1) * (r.cj + 1) * (r.ck + 1);
+  // the nodes, the extended nodes, and the raw metrics of two coarse levels in turn
+  const RawDims r2{r.ci / 2, r.cj / 2, r.ck / 2}, r3{r.ci / 4, r.cj / 4, r.ck / 4};
+  const size_t n2 = nlev > 1 ? RW_N * r2.n() : 0, n3 = nlev > 2 ? RW_N * r3.n() : 0;
+  double* dn = nullptr;
+  CK(setup_buf(c, (3 * (nn + ne) + n2 + n3) * sizeof(double), &dn));
+  double *de = dn + 3 * nn, *raw[2] = {de + 3 * ne, de + 3 * ne + n2};
   cudaError_t e = cudaMemcpyAsync(dn, xyz, 3 * nn * sizeof(double), cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) {
     k_extend_nodes<<<nblk((long)ne, 256), 256, 0, c->stream>>>(dn, de, g, ng);
-    k_raw_metrics<<<nblk((long)r.n(), 256), 256, 0, c->stream>>>(de, raw, r);
+    k_cell_metrics<<<nblk((long)b->ntot, 256), 256, 0, c->stream>>>(b->db, de, ng);
     c->nlaunch += 2;
-    int lng = ng;
-    for (int l = 0; l < nlev && e == cudaSuccess; l++) {
-      BlockCtx* x = lv[l];
-      k_finish_metrics<<<nblk((long)x->ntot, 256), 256, 0, c->stream>>>(x->db, raw, r, lng);
-      c->nlaunch++;
-      if (l + 1 < nlev) {
-        RawDims rc{r.ci / 2, r.cj / 2, r.ck / 2};
-        if (lv[l + 1]->imax + 2 * (lng / 2) != rc.ci || lv[l + 1]->jmax + 2 * (lng / 2) != rc.cj ||
-            lv[l + 1]->kmax + 2 * (lng / 2) != rc.ck) {
-          cleanup();
-          return fail(c, FF_ERR_ARG, "ff_block_metrics_levels: a coarse level does not halve the finer one");
-        }
-        if (cudaMalloc(&raw2, RW_N * rc.n() * sizeof(double)) != cudaSuccess) { e = cudaErrorMemoryAllocation; break; }
-        k_lump<<<nblk((long)rc.n(), 256), 256, 0, c->stream>>>(raw, r, raw2, rc);
-        c->nlaunch++;
-        e = cudaStreamSynchronize(c->stream);
-        cudaFree(raw);
-        raw = raw2;
-        raw2 = nullptr;
-        r = rc;
-        lng /= 2;
-      }
+    RawDims f = r;
+    for (int l = 1, lng = ng / 2; l < nlev; l++, lng /= 2) {
+      const RawDims q{f.ci / 2, f.cj / 2, f.ck / 2};
+      if (l == 1) k_raw_lump<<<nblk((long)q.n(), 64), 64, 0, c->stream>>>(de, f, raw[0], q);
+      else k_lump<<<nblk((long)q.n(), 256), 256, 0, c->stream>>>(raw[l & 1], f, raw[(l - 1) & 1], q);
+      k_finish_metrics<<<nblk((long)lv[l]->ntot, 256), 256, 0, c->stream>>>(lv[l]->db, raw[(l - 1) & 1], q, lng);
+      c->nlaunch += 2;
+      f = q;
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    e = cudaStreamSynchronize(c->stream);
   }
-  cleanup();
+  setup_done(c);
   if (e != cudaSuccess) return fail(c, FF_ERR_CUDA, "ff_block_metrics_levels", e);
   CK(cudaGetLastError());
   return 0;
@@ -1999,15 +2017,23 @@ int ff_wall_distance(void* ctx, int blk, const double* pts, int npts) {
   Ctx* c = (Ctx*)ctx;
   BlockCtx* b = getb(c, blk);
   if (!b || npts < 0 || (npts > 0 && !pts)) return fail(c, FF_ERR_ARG, "ff_wall_distance");
+  // points, then the boxes of their groups and super-groups
+  const int ng = (npts + WD_C - 1) / WD_C, nsup = (ng + WD_S - 1) / WD_S;
+  const size_t np3 = (size_t)npts * 3;
   double* dp = nullptr;
-  if (npts > 0) CK(cudaMalloc(&dp, (size_t)npts * 3 * sizeof(double)));
-  cudaError_t e = npts > 0 ? cudaMemcpyAsync(dp, pts, (size_t)npts * 3 * sizeof(double), cudaMemcpyHostToDevice, c->stream)
-                           : cudaSuccess;
+  if (npts > 0) CK(setup_buf(c, np3 * sizeof(double) + (size_t)(ng + nsup) * sizeof(WdBox), &dp));
+  WdBox *group = (WdBox*)(dp + np3), *super = group + ng;
+  cudaError_t e = cudaSuccess;
+  if (npts > 0) {
+    e = cudaMemcpyAsync(dp, pts, np3 * sizeof(double), cudaMemcpyHostToDevice, c->stream);
+    k_wd_boxes<<<nsup, WD_C * WD_S, 0, c->stream>>>(dp, npts, group, super);
+    c->nlaunch++;
+  }
   // the block, then each coarser level: every cell's nearest point, and
   // the interior cells again as the mean of their children (LUMP_DIST)
   BlockCtx* fine = nullptr;
   for (BlockCtx* x = b; x && e == cudaSuccess; fine = x, x = x->coarse) {
-    k_wall_distance<<<nblk((long)x->ntot, WD_THREADS), WD_THREADS, 0, c->stream>>>(x->db, dp, npts);
+    k_wall_distance<<<nblk((long)x->ntot, WD_THREADS), WD_THREADS, 0, c->stream>>>(x->db, dp, npts, group, super);
     c->nlaunch++;
     if (fine) {
       k_lump_distw<<<nblk((long)x->imax * x->jmax * x->kmax, 256), 256, 0, c->stream>>>(fine->db, x->db);
@@ -2016,7 +2042,7 @@ int ff_wall_distance(void* ctx, int blk, const double* pts, int npts) {
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (dp) cudaFree(dp);
+  setup_done(c);
   if (e != cudaSuccess) return fail(c, FF_ERR_CUDA, "ff_wall_distance", e);
   return 0;
 }

@@ -164,15 +164,16 @@ FF_DI double thickness(double vol, double alo, double ahi) {
   return dmin(1e4, rm(rq(ra(vol, eps), ra(ra(alo, ahi), eps)), 2.0));
 }
 
-// Metrics of every storage cell (ghosts included) of the block from the
-// extended nodes with 2 ghost layers.
-__global__ void k_cell_metrics(DevBlock b, const double* __restrict__ ext) {
+// Metrics of every storage cell (two ghost layers included) of the block from
+// the extended nodes with ng >= 2 ghost layers.
+__global__ void k_cell_metrics(DevBlock b, const double* __restrict__ ext, int ng) {
   const int is = b.imax + 4, js = b.jmax + 4, ks = b.kmax + 4;
   const size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= (size_t)b.ntot) return;
   const int i = (int)(n % is), j = (int)((n / is) % js), k = (int)(n / ((size_t)is * js));
-  const ExtNodes E{ext, (size_t)(is + 1) * (js + 1) * (ks + 1), is + 1, js + 1};
-  const CellGeom g = arevc1_cell(E, i, j, k);
+  const int o = ng - 2, ei = is + 2 * o + 1, ej = js + 2 * o + 1, ek = ks + 2 * o + 1;
+  const ExtNodes E{ext, (size_t)ei * ej * ek, ei, ej};
+  const CellGeom g = arevc1_cell(E, i + o, j + o, k + o);
   b.a[FF_XC][n] = g.cen.x;
   b.a[FF_YC][n] = g.cen.y;
   b.a[FF_ZC][n] = g.cen.z;
@@ -203,30 +204,77 @@ struct RawDims {
 // high face's; RW_VOL; RW_C + c
 enum : int { RW_ALO = 0, RW_NLO = 3, RW_AHI = 12, RW_NHI = 15, RW_VOL = 24, RW_C = 25, RW_N = 28 };
 
-__global__ void k_raw_metrics(const double* __restrict__ ext, double* __restrict__ raw, RawDims r) {
-  const size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nr = r.n();
-  if (n >= nr) return;
-  const int i = (int)(n % r.ci), j = (int)((n / r.ci) % r.cj), k = (int)(n / ((size_t)r.ci * r.cj));
-  const ExtNodes E{ext, (size_t)(r.ci + 1) * (r.cj + 1) * (r.ck + 1), r.ci + 1, r.cj + 1};
-  const CellGeom g = arevc1_cell(E, i, j, k);
-  for (int d = 0; d < 3; d++) {
-    double a, ah;
-    V3 nr_, nh;
-    area_normal(g.lo[d], a, nr_);
-    area_normal(g.hi[d], ah, nh);
-    raw[(size_t)(RW_ALO + d) * nr + n] = a;
-    raw[(size_t)(RW_NLO + 3 * d + 0) * nr + n] = nr_.x;
-    raw[(size_t)(RW_NLO + 3 * d + 1) * nr + n] = nr_.y;
-    raw[(size_t)(RW_NLO + 3 * d + 2) * nr + n] = nr_.z;
-    raw[(size_t)(RW_AHI + d) * nr + n] = ah;
-    raw[(size_t)(RW_NHI + 3 * d + 0) * nr + n] = nh.x;
-    raw[(size_t)(RW_NHI + 3 * d + 1) * nr + n] = nh.y;
-    raw[(size_t)(RW_NHI + 3 * d + 2) * nr + n] = nh.z;
+// LUMPA1's result for one face: the summed area + 1e-20, the normalised sum of the area-weighted normals.
+FF_DI void lump_face(double al, V3 v, double* __restrict__ cr, size_t nc, size_t n, int acomp, int ncomp) {
+  const double axyzl = vnorm(v), den = ra(axyzl, 1.0e-20);
+  double nx = rq(v.x, den);
+  const double ny = rq(v.y, den), nz = rq(v.z, den);
+  if (axyzl < 1.0e-20) nx = 1.;
+  cr[(size_t)acomp * nc + n] = ra(al, 1.0e-20);
+  cr[(size_t)(ncomp + 0) * nc + n] = nx;
+  cr[(size_t)(ncomp + 1) * nc + n] = ny;
+  cr[(size_t)(ncomp + 2) * nc + n] = nz;
+}
+
+// The first coarsening step straight from the extended nodes (RawDims f the
+// fine cells): a thread makes its eight children's geometry in registers and
+// adds it up, instead of writing the 28 raw values of every fine cell (206 MB
+// for a 128x64x64 block with three levels) and reading them twice.  Children
+// in LUMPVS's order; every sum below in the order k_lump takes it, for which
+// LUMPA1's k faces wait with the second child until the third is in.
+__global__ void __launch_bounds__(64) k_raw_lump(const double* __restrict__ ext, RawDims f, double* __restrict__ cr,
+                                                 RawDims c) {
+  const size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nc = c.n();
+  if (n >= nc) return;
+  const int i = (int)(n % c.ci), j = (int)((n / c.ci) % c.cj), k = (int)(n / ((size_t)c.ci * c.cj));
+  const ExtNodes E{ext, (size_t)(f.ci + 1) * (f.cj + 1) * (f.ck + 1), f.ci + 1, f.cj + 1};
+  struct Face {
+    double a;
+    V3 v;   // area and area-weighted normal
+  };
+  Face acc[3][2], held[2];
+  double vl = 0.;
+  V3 sc{0., 0., 0.};
+  auto add = [](Face& s, const Face& t, bool first) {
+    s.a = first ? t.a : ra(s.a, t.a);
+    s.v.x = first ? t.v.x : ra(s.v.x, t.v.x);
+    s.v.y = first ? t.v.y : ra(s.v.y, t.v.y);
+    s.v.z = first ? t.v.z : ra(s.v.z, t.v.z);
+  };
+#pragma unroll
+  for (int q = 0; q < 8; q++) {   // (di, dj, dk): 000, 010, 001, 011, 100, 110, 101, 111
+    const int di = q >> 2, dj = q & 1, dk = (q >> 1) & 1;
+    const CellGeom g = arevc1_cell(E, 2 * i + di, 2 * j + dj, 2 * k + dk);
+    vl = q == 0 ? g.vol : ra(vl, g.vol);
+    const V3 t{rm(g.vol, g.cen.x), rm(g.vol, g.cen.y), rm(g.vol, g.cen.z)};
+    sc = q == 0 ? t : V3{ra(sc.x, t.x), ra(sc.y, t.y), ra(sc.z, t.z)};
+    const int side[3] = {di, dj, dk};
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      Face w;
+      V3 nr;
+      area_normal(side[d] ? g.hi[d] : g.lo[d], w.a, nr);
+      w.v = V3{rm(w.a, nr.x), rm(w.a, nr.y), rm(w.a, nr.z)};
+      // how many children of this side came before: d = 0 pairs (j, k), d = 1 (k, i), both met in their own
+      // order; d = 2 pairs (i, j), met as (0,0), (0,1), (1,0), (1,1) and added as (0,0), (1,0), (0,1), (1,1)
+      const int o1 = d == 0 ? dj : (d == 1 ? dk : di), o2 = d == 0 ? dk : (d == 1 ? di : dj);
+      if (d == 2 && o1 == 0 && o2 == 1) {
+        held[side[d]] = w;
+      } else {
+        add(acc[d][side[d]], w, o1 == 0 && o2 == 0);
+        if (d == 2 && o1 == 1 && o2 == 0) add(acc[d][side[d]], held[side[d]], false);
+      }
+    }
   }
-  raw[(size_t)RW_VOL * nr + n] = g.vol;
-  raw[(size_t)(RW_C + 0) * nr + n] = g.cen.x;
-  raw[(size_t)(RW_C + 1) * nr + n] = g.cen.y;
-  raw[(size_t)(RW_C + 2) * nr + n] = g.cen.z;
+  cr[(size_t)RW_VOL * nc + n] = vl;
+  cr[(size_t)(RW_C + 0) * nc + n] = rq(sc.x, vl);
+  cr[(size_t)(RW_C + 1) * nc + n] = rq(sc.y, vl);
+  cr[(size_t)(RW_C + 2) * nc + n] = rq(sc.z, vl);
+#pragma unroll
+  for (int d = 0; d < 3; d++)
+#pragma unroll
+    for (int s = 0; s < 2; s++) lump_face(acc[d][s].a, acc[d][s].v, cr, nc, n, s ? RW_AHI + d : RW_ALO + d,
+                                          (s ? RW_NHI : RW_NLO) + 3 * d);
 }
 
 // One coarsening step: coarse cell (i, j, k) from the fine children
@@ -270,16 +318,7 @@ __global__ void k_lump(const double* __restrict__ fr, RawDims f, double* __restr
       }
       double al = F(acomp + d, m4[0]);
       for (int q = 1; q < 4; q++) al = ra(al, F(acomp + d, m4[q]));
-      al = ra(al, 1.0e-20);
-      const double axyzl = __dsqrt_rn(ra(ra(rm(v[0], v[0]), rm(v[1], v[1])), rm(v[2], v[2])));
-      const double den = ra(axyzl, 1.0e-20);
-      double nx = rq(v[0], den);
-      const double ny = rq(v[1], den), nz = rq(v[2], den);
-      if (axyzl < 1.0e-20) nx = 1.;
-      cr[(size_t)(acomp + d) * nc + n] = al;
-      cr[(size_t)(ncomp + 3 * d + 0) * nc + n] = nx;
-      cr[(size_t)(ncomp + 3 * d + 1) * nc + n] = ny;
-      cr[(size_t)(ncomp + 3 * d + 2) * nc + n] = nz;
+      lump_face(al, V3{v[0], v[1], v[2]}, cr, nc, n, acomp + d, ncomp + 3 * d);
     }
   }
 }
@@ -307,28 +346,107 @@ __global__ void k_finish_metrics(DevBlock b, const double* __restrict__ raw, Raw
   }
 }
 
-// WALL_DIST: DISTW of every storage cell, the distance to the nearest of
-// the wall points (3 values each), squared distances (dx^2 + dy^2) + dz^2
-// compared starting from 1e8 (the least kept), then the root.  One thread
-// per cell; the points staged through shared memory in tiles.
-constexpr int WD_THREADS = 256, WD_TP = 512;
-__global__ void __launch_bounds__(WD_THREADS) k_wall_distance(DevBlock b, const double* __restrict__ pts, int np) {
-  __shared__ double sp[WD_TP * 3];
+// WALL_DIST: DISTW of every storage cell, the distance to the nearest of the
+// wall points (3 values each), squared distances (dx^2 + dy^2) + dz^2
+// compared starting from 1e8 (the least kept), then the root.
+//
+// Every cell against every point is cells x points: 9e9 distances for a
+// 128x64x64 block and its 16384 points, 4.4 ms of FP64 work.  The points come
+// in patch order, so WD_C consecutive ones lie close together: each such
+// group gets its bounding box (k_wd_boxes), each WD_S groups a box of theirs,
+// and a cell only looks at groups whose box is not farther than the nearest
+// point it has.  A box distance is taken 1e-12 short, far more than the
+// rounding of either side, so no group that holds the least rounded distance
+// is passed over and the result is the same to the bit.  The walk is a warp's
+// (32 consecutive cells, nearly the same groups): a group is looked at when
+// any of the 32 needs it, its points read once for all.
+constexpr int WD_THREADS = 256, WD_C = 32, WD_S = 32;
+
+struct WdBox {
+  double lo[3], hi[3];
+};
+
+// boxes of the groups, one warp each, and of WD_S groups, one block of 32 warps each
+__global__ void __launch_bounds__(WD_C* WD_S) k_wd_boxes(const double* __restrict__ pts, int np, WdBox* group,
+                                                       WdBox* super) {
+  __shared__ WdBox sb[WD_S];
+  const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int g = blockIdx.x * WD_S + w, t = g * WD_C + lane, ng = (np + WD_C - 1) / WD_C;
+  double lo[3], hi[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const double x = t < np ? pts[(size_t)t * 3 + c] : 0.;
+    lo[c] = t < np ? x : __longlong_as_double(0x7ff0000000000000LL);
+    hi[c] = t < np ? x : -__longlong_as_double(0x7ff0000000000000LL);
+    for (int o = 16; o > 0; o >>= 1) {   // fmin / fmax leave a NaN out, as the comparison of distances does
+      lo[c] = fmin(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+      hi[c] = fmax(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+    }
+    if (lane == 0) {
+      sb[w].lo[c] = lo[c];
+      sb[w].hi[c] = hi[c];
+      if (g < ng) { group[g].lo[c] = lo[c]; group[g].hi[c] = hi[c]; }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double a = sb[0].lo[threadIdx.x], b = sb[0].hi[threadIdx.x];
+    for (int q = 1; q < WD_S; q++) {
+      a = fmin(a, sb[q].lo[threadIdx.x]);
+      b = fmax(b, sb[q].hi[threadIdx.x]);
+    }
+    super[blockIdx.x].lo[threadIdx.x] = a;
+    super[blockIdx.x].hi[threadIdx.x] = b;
+  }
+}
+
+// a squared distance no point of the box is nearer than
+FF_DI double wd_bound(const WdBox* b, double x, double y, double z) {
+  const double dx = fmax(fmax(__ldg(b->lo) - x, x - __ldg(b->hi)), 0.);
+  const double dy = fmax(fmax(__ldg(b->lo + 1) - y, y - __ldg(b->hi + 1)), 0.);
+  const double dz = fmax(fmax(__ldg(b->lo + 2) - z, z - __ldg(b->hi + 2)), 0.);
+  return (dx * dx + dy * dy + dz * dz) * (1. - 1.e-12);
+}
+FF_DI void wd_group(const double* __restrict__ pts, int np, int g, double x, double y, double z, double& best) {
+  const int t1 = min(np, (g + 1) * WD_C);
+#pragma unroll 4
+  for (int t = g * WD_C; t < t1; t++) {
+    const double dx = rs(x, __ldg(pts + 3 * (size_t)t)), dy = rs(y, __ldg(pts + 3 * (size_t)t + 1)),
+                 dz = rs(z, __ldg(pts + 3 * (size_t)t + 2));
+    const double r = ra(ra(rm(dx, dx), rm(dy, dy)), rm(dz, dz));
+    if (r < best) best = r;
+  }
+}
+
+__global__ void __launch_bounds__(WD_THREADS) k_wall_distance(DevBlock b, const double* __restrict__ pts, int np,
+                                                              const WdBox* __restrict__ group,
+                                                              const WdBox* __restrict__ super) {
   const size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool ok = n < (size_t)b.ntot;
-  const double x = ok ? b.a[FF_XC][n] : 0., y = ok ? b.a[FF_YC][n] : 0., z = ok ? b.a[FF_ZC][n] : 0.;
+  const size_t m = ok ? n : (size_t)b.ntot - 1;   // whole warps take part in the votes
+  const double x = b.a[FF_XC][m], y = b.a[FF_YC][m], z = b.a[FF_ZC][m];
+  const int ng = (np + WD_C - 1) / WD_C, nsup = (ng + WD_S - 1) / WD_S;
   double best = 1.e8;
-  for (int t0 = 0; t0 < np; t0 += WD_TP) {
-    const int nt = min(WD_TP, np - t0);
-    __syncthreads();
-    for (int q = threadIdx.x; q < nt * 3; q += blockDim.x) sp[q] = pts[(size_t)t0 * 3 + q];
-    __syncthreads();
-    if (ok)
-      for (int t = 0; t < nt; t++) {
-        const double dx = rs(x, sp[3 * t]), dy = rs(y, sp[3 * t + 1]), dz = rs(z, sp[3 * t + 2]);
-        const double r = ra(ra(rm(dx, dx), rm(dy, dy)), rm(dz, dz));
-        if (r < best) best = r;
-      }
+  if (np > 0) {
+    // a first guess: the nearest group of the nearest super-group
+    int s0 = 0, g0;
+    double near = __longlong_as_double(0x7ff0000000000000LL);
+    for (int s = 0; s < nsup; s++) {
+      const double d = wd_bound(super + s, x, y, z);
+      if (d < near) { near = d; s0 = s; }
+    }
+    near = __longlong_as_double(0x7ff0000000000000LL);
+    g0 = s0 * WD_S;
+    for (int g = s0 * WD_S; g < min(ng, (s0 + 1) * WD_S); g++) {
+      const double d = wd_bound(group + g, x, y, z);
+      if (d < near) { near = d; g0 = g; }
+    }
+    wd_group(pts, np, g0, x, y, z, best);
+    for (int s = 0; s < nsup; s++) {
+      if (!__any_sync(0xffffffffu, wd_bound(super + s, x, y, z) <= best)) continue;
+      for (int g = s * WD_S; g < min(ng, (s + 1) * WD_S); g++)
+        if (__any_sync(0xffffffffu, wd_bound(group + g, x, y, z) <= best)) wd_group(pts, np, g, x, y, z, best);
+    }
   }
   if (ok) b.a[FF_DISTW][n] = __dsqrt_rn(best);
 }
