@@ -168,7 +168,7 @@ int st_statim(Ctx* c, BlockCtx* b, int npass = 2) {
 }
 
 int st_boundi(Ctx* c, BlockCtx* b) {
-  k_refcor<<<nblk(b->ntot, 256), 256, 0, c->stream>>>(b->db);
+  k_refcor<<<nblk(refcor_threads(b->imax, b->jmax, b->kmax), 128), 128, 0, c->stream>>>(b->db);
   c->nlaunch++;
   if (b->npatch) {
     int maxn = 1;
@@ -1379,7 +1379,7 @@ int mb_boundi(Ctx* c) {
   int nb = (int)c->tops.size(), rc;
   rc = fork_join(c, nb, [&](int n) {
     BlockCtx* b = c->tops[n];
-    k_refcor<<<nblk(b->ntot, 256), 256, 0, c->stream>>>(b->db);
+    k_refcor<<<nblk(refcor_threads(b->imax, b->jmax, b->kmax), 128), 128, 0, c->stream>>>(b->db);
     c->nlaunch++;
     if (b->npatch) {
       int maxn = 1;
@@ -1534,7 +1534,7 @@ int mb_phase(Ctx* c, int phase, int icycle) {
   if (phase == FF_PHASE_CYCLE_A || phase == FF_PHASE_BOUNDI_A) {
     rc = fork_join(c, nb, [&](int n) {
       BlockCtx* b = c->tops[n];
-      k_refcor<<<nblk(b->ntot, 256), 256, 0, c->stream>>>(b->db);
+      k_refcor<<<nblk(refcor_threads(b->imax, b->jmax, b->kmax), 128), 128, 0, c->stream>>>(b->db);
       c->nlaunch++;
       if (b->npatch) {
         int maxn = 1;

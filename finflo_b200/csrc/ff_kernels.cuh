@@ -28,46 +28,56 @@ constexpr int NCOEF = 13;                 // LU-SGS coefficients per cell
 // ---------------------------------------------------------------------------
 // STATIM: PDTOP state.f:1690, PERFGA state.f:159, CONSVA base3c.f:489, and the
 // laminar TURBDI (ADJUIN res3c.f:9447: EPS2 = 1, VIST = 0 on interior cells).
-FF_DI void state_cell(const DevBlock& b, const ff_params& p, size_t n) {
-  double* a_P = b.a[FF_P];
+struct StateV {
+  double P, drdp, ro, vis, drdh, cp, ch, c, e, u, v, w;
+};
+
+FF_DI StateV state_eval(const DevBlock& b, const ff_params& p, size_t n) {
+  StateV s;
   double pd = b.a[FF_PDIFF][n], T = b.a[FF_TEMP][n];
-  double P = pd + p.frspre;
+  s.u = b.a[FF_U][n]; s.v = b.a[FF_V][n]; s.w = b.a[FF_W][n];
+  const double rk = p.iturb < 3 ? 0. : b.a[FF_RK][n];
+  s.P = pd + p.frspre;
   const double gm1 = p.gamma - 1., cp2 = p.gamma / gm1 * p.rgas;
   double trgs = T * p.rgas;
-  double drdp = 1. / trgs;
-  double ro = P * drdp;
-  double vis = p.visu0 * T * sqrt(T) / (T + p.tsu0);
+  s.drdp = 1. / trgs;
+  s.ro = s.P * s.drdp;
+  s.vis = p.visu0 * T * sqrt(T) / (T + p.tsu0);
   double e = trgs / gm1;
-  double drdh = -ro / e / p.gamma;
-  double u = b.a[FF_U][n], v = b.a[FF_V][n], w = b.a[FF_W][n];
-  double rkin = (u * u + v * v + w * w) * .5;
-  double c, rk = 0.;
+  s.drdh = -s.ro / e / p.gamma;
+  double rkin = (s.u * s.u + s.v * s.v + s.w * s.w) * .5;
   if (p.iturb < 3) {
-    c = sqrt(dmax(1. / (drdh / ro + drdp), 1.0));
+    s.c = sqrt(dmax(1. / (s.drdh / s.ro + s.drdp), 1.0));
   } else {   // CONSVA two-equation branch: k in the sound speed and E
-    rk = b.a[FF_RK][n];
-    double ypro = 1. / ro;
-    double xturb = 1. + (2. / 3.) * rk * ypro * drdp;
-    c = sqrt(dmax(xturb / (drdh * ypro + drdp), 1.0));
+    double ypro = 1. / s.ro;
+    double xturb = 1. + (2. / 3.) * rk * ypro * s.drdp;
+    s.c = sqrt(dmax(xturb / (s.drdh * ypro + s.drdp), 1.0));
   }
-  a_P[n] = P;
-  b.a[FF_DRDP][n] = drdp;
-  b.a[FF_RO][n] = ro;
-  b.a[FF_VIS][n] = vis;
-  b.a[FF_DRDH][n] = drdh;
-  b.a[FF_CP][n] = cp2;
-  b.a[FF_CH][n] = vis * cp2 / p.pr;
-  b.a[FF_C][n] = c;
-  b.a[FF_E][n] = p.iturb < 3 ? (e + rkin) * ro : (e + rkin) * ro + rk;
-  b.a[FF_RM][n] = ro * u;
-  b.a[FF_RN][n] = ro * v;
-  b.a[FF_RW][n] = ro * w;
+  s.cp = cp2;
+  s.ch = s.vis * cp2 / p.pr;
+  s.e = p.iturb < 3 ? (e + rkin) * s.ro : (e + rkin) * s.ro + rk;
+  return s;
+}
+
+FF_DI void state_store(const DevBlock& b, size_t n, const StateV& s) {
+  b.a[FF_P][n] = s.P;
+  b.a[FF_DRDP][n] = s.drdp;
+  b.a[FF_RO][n] = s.ro;
+  b.a[FF_VIS][n] = s.vis;
+  b.a[FF_DRDH][n] = s.drdh;
+  b.a[FF_CP][n] = s.cp;
+  b.a[FF_CH][n] = s.ch;
+  b.a[FF_C][n] = s.c;
+  b.a[FF_E][n] = s.e;
+  b.a[FF_RM][n] = s.ro * s.u;
+  b.a[FF_RN][n] = s.ro * s.v;
+  b.a[FF_RW][n] = s.ro * s.w;
 }
 
 __global__ void k_state(DevBlock b, ff_params p) {
   size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= (size_t)b.ntot) return;
-  state_cell(b, p, n);
+  state_store(b, n, state_eval(b, p, n));
   if (p.iturb >= 3) return;   // TURBEQ, not ADJUIN, sets EPS2 and VIST
   int i = (int)(n % b.is), j = (int)((n / b.is) % (b.jmax + 4)), k = (int)(n / b.il);
   if (i >= 2 && i < b.imax + 2 && j >= 2 && j < b.jmax + 2 && k >= 2 && k < b.kmax + 2) {
@@ -105,6 +115,12 @@ FF_DI size_t face_cell(const DevBlock& b, const FaceG& f, int a, int c) {
   (void)ls;                                                                    \
   size_t L = face_cell((b), fg, pa1, pa2);
 
+// The patch kernels below read everything a cell needs before the first
+// store: a slot's store may alias the next slot's load as far as the compiler
+// knows, so load-store pairs in turn cost one L2 round trip each (k_reflec
+// 10.8, k_mir 12.1, k_refcor 12.0, k_refcen 8.6 and k_inlet_outlet 7.7 us a
+// launch on a 16x8x8 block; 6.3, 4.4, 3.7, 4.9 and 6.0 us now).
+
 // REFLEC turb3.f:5294: solid walls (viscous, wall at rest) and the inlet
 // pressure extrapolation.  mode 0: REFLEC; mode 1: re-evaluate the equation of
 // state in the two ghost cells first (the second STATIM pass).
@@ -113,34 +129,42 @@ __global__ void k_reflec(DevBlock b, ff_params p, int mode) {
   size_t LB = L - ls, LT = L + ls, LC = L - 2 * ls;
   bool wall = pa.ityp >= 7 && pa.ityp <= 10;
   if (!wall && pa.ityp != FF_BC_INL) return;
-  if (mode == 1) { state_cell(b, p, LB); state_cell(b, p, LC); }
   double* P = b.a[FF_P]; double* PD = b.a[FF_PDIFF];
+  double *T = b.a[FF_TEMP], *RO = b.a[FF_RO];
+  const double pl = P[L], pdl = PD[L];
+  StateV sB, sC;
+  if (mode == 1) { sB = state_eval(b, p, LB); sC = state_eval(b, p, LC); }
   if (pa.ityp == FF_BC_INL) {
-    P[LB] = P[L]; PD[LB] = PD[L]; P[LC] = P[L]; PD[LC] = PD[L];
+    if (mode == 1) { state_store(b, LB, sB); state_store(b, LC, sC); }
+    P[LB] = pl; PD[LB] = pdl; P[LC] = pl; PD[LC] = pdl;
     return;
   }
-  double *T = b.a[FF_TEMP], *RO = b.a[FF_RO];
+  const double tl = T[L], vis = b.a[FF_VIS][L], ch = b.a[FF_CH][L], cc = b.a[FF_C][L], drdp = b.a[FF_DRDP][L];
+  const double drdh = b.a[FF_DRDH][L], u = -b.a[FF_U][L], v = -b.a[FF_V][L], w = -b.a[FF_W][L], rol = RO[L];
+  const double plt = P[LT], pdlt = PD[LT], e = b.a[FF_E][L];
+  double rk = 0., re = 0., ret = 0.;
+  if (p.iturb >= 3) { rk = b.a[FF_RK][L]; re = b.a[FF_REPS][L]; ret = b.a[FF_REPS][LT]; }
+  if (mode == 1) { state_store(b, LB, sB); state_store(b, LC, sC); }
   int ihfl = pa.iheat == 1 ? 1 : 0;
   double tsurf = pa.iheat == 1 ? pa.bount : 0.0;
-  double tb = (1 - ihfl) * T[L] + ihfl * (2. * tsurf - T[L]);
+  double tb = (1 - ihfl) * tl + ihfl * (2. * tsurf - tl);
   tb = dmax(dmin(tb, p.tuplim), p.tlolim);
   T[LB] = tb; T[LC] = tb;
-  b.a[FF_VIS][LB] = b.a[FF_VIS][L]; b.a[FF_CH][LB] = b.a[FF_CH][L]; b.a[FF_C][LB] = b.a[FF_C][L];
-  b.a[FF_DRDP][LB] = b.a[FF_DRDP][L]; b.a[FF_DRDH][LB] = b.a[FF_DRDH][L];
-  double u = -b.a[FF_U][L], v = -b.a[FF_V][L], w = -b.a[FF_W][L];
+  b.a[FF_VIS][LB] = vis; b.a[FF_CH][LB] = ch; b.a[FF_C][LB] = cc;
+  b.a[FF_DRDP][LB] = drdp; b.a[FF_DRDH][LB] = drdh;
   b.a[FF_U][LB] = u; b.a[FF_V][LB] = v; b.a[FF_W][LB] = w;
   b.a[FF_U][LC] = u; b.a[FF_V][LC] = v; b.a[FF_W][LC] = w;
-  double ro = dmax(0.001 * p.frsden, RO[L]);
-  double pb = dmax(0.001 * p.frspre, 2. * P[L] - P[LT]);
-  double pdb = dmax(-0.999 * p.frspre, 2. * PD[L] - PD[LT]);
+  double ro = dmax(0.001 * p.frsden, rol);
+  double pb = dmax(0.001 * p.frspre, 2. * pl - plt);
+  double pdb = dmax(-0.999 * p.frspre, 2. * pdl - pdlt);
   RO[LB] = ro; RO[LC] = ro; P[LB] = pb; P[LC] = pb; PD[LB] = pdb; PD[LC] = pdb;
   b.a[FF_EPS2][LB] = 1.; b.a[FF_VIST][LB] = 0.; b.a[FF_EPS2][LC] = 1.; b.a[FF_VIST][LC] = 0.;
   b.a[FF_RM][LB] = ro * u; b.a[FF_RN][LB] = ro * v; b.a[FF_RW][LB] = ro * w;
   b.a[FF_RM][LC] = ro * u; b.a[FF_RN][LC] = ro * v; b.a[FF_RW][LC] = ro * w;
-  b.a[FF_E][LB] = b.a[FF_E][L]; b.a[FF_E][LC] = b.a[FF_E][L];
+  b.a[FF_E][LB] = e; b.a[FF_E][LC] = e;
   if (p.iturb >= 3) {   // turb3.f:5646-5658 (ITURB = 6)
-    b.a[FF_RK][LB] = -b.a[FF_RK][L];
-    b.a[FF_REPS][LB] = dmax(0., 2. * b.a[FF_REPS][L] - b.a[FF_REPS][LT]);
+    b.a[FF_RK][LB] = -rk;
+    b.a[FF_REPS][LB] = dmax(0., 2. * re - ret);
   }
 }
 
@@ -149,18 +173,16 @@ __global__ void k_refcen(DevBlock b, ff_params p) {
   FF_PATCH_LOOP(b)
   if (pa.ityp < 7 || pa.ityp > 10) return;
   size_t LB = L - ls, LT = L + ls;
-  double* RO = b.a[FF_RO]; double* P = b.a[FF_P]; double* PD = b.a[FF_PDIFF];
-  RO[LB] = dmax(0.001 * p.frsden, 2. * RO[L] - RO[LT]);
-  P[LB] = dmax(0.001 * p.frspre, 2. * P[L] - P[LT]);
-  PD[LB] = dmax(-0.999 * p.frspre, 2. * PD[L] - PD[LT]);
-  const int sl[7] = {FF_E, FF_U, FF_V, FF_W, FF_RM, FF_RN, FF_RW};
+  const int sl[12] = {FF_RO, FF_P, FF_PDIFF, FF_E, FF_U, FF_V, FF_W, FF_RM, FF_RN, FF_RW, FF_RK, FF_REPS};
+  const double lim[3] = {0.001 * p.frsden, 0.001 * p.frspre, -0.999 * p.frspre};
+  const int nv = p.iturb >= 3 ? 12 : 10;   // turb3.f:6013-6027
+  double x[12];
 #pragma unroll
-  for (int s = 0; s < 7; s++) { double* q = b.a[sl[s]]; q[LB] = 2. * q[L] - q[LT]; }
-  if (p.iturb >= 3) {   // turb3.f:6013-6027
-    double *RK = b.a[FF_RK], *RE = b.a[FF_REPS];
-    RK[LB] = dmax(p.rklim, 2. * RK[L] - 1. * RK[LT]);
-    RE[LB] = dmax(p.epslim, 2. * RE[L] - 1. * RE[LT]);
-  }
+  for (int q = 0; q < 12; q++)
+    if (q < nv) x[q] = 2. * b.a[sl[q]][L] - b.a[sl[q]][LT];
+#pragma unroll
+  for (int q = 0; q < 12; q++)
+    if (q < nv) b.a[sl[q]][LB] = q < 3 ? dmax(lim[q], x[q]) : (q == 10 ? dmax(p.rklim, x[q]) : (q == 11 ? dmax(p.epslim, x[q]) : x[q]));
 }
 
 // INLET base3c.f:9223 (INLOUT 4) and OUTLET base3c.f:9595 (INLOUT 2, 3): the
@@ -176,65 +198,68 @@ __global__ void k_inlet_outlet(DevBlock b, ff_params p, int icycle) {
   double *P = b.a[FF_P], *PD = b.a[FF_PDIFF], *E = b.a[FF_E], *RM = b.a[FF_RM], *RN = b.a[FF_RN];
   double *RW = b.a[FF_RW], *EPS2 = b.a[FF_EPS2], *VIST = b.a[FF_VIST], *VIS = b.a[FF_VIS];
   if (inl) {
-    double dpkoe = P[II], dpdif = PD[II];
-    EPS2[IM1] = EPS2[II]; EPS2[IM2] = EPS2[II];
-    VIST[IM1] = VIST[II]; VIST[IM2] = VIST[II];
+    const double dpkoe = P[II], dpdif = PD[II], eps2 = EPS2[II], vist = VIST[II];
+    const double r1 = icycle == 1 ? pa.bounr : RO[IM1], r2 = RO[IM2];
+    EPS2[IM1] = eps2; EPS2[IM2] = eps2;
+    VIST[IM1] = vist; VIST[IM2] = vist;
     double rm = pa.bounu * pa.bounr, rn = pa.bounv * pa.bounr, rw = pa.bounw * pa.bounr;
     RM[IM1] = rm; RN[IM1] = rn; RW[IM1] = rw; RM[IM2] = rm; RN[IM2] = rn; RW[IM2] = rw;
     if (icycle == 1) RO[IM1] = pa.bounr;
     T[IM1] = pa.bount; T[IM2] = pa.bount;
     P[IM1] = dpkoe; P[IM2] = dpkoe; PD[IM1] = dpdif; PD[IM2] = dpdif;
     double e = p.rgas / (p.gamma - 1.) * pa.bount;
-    double r1 = RO[IM1], r2 = RO[IM2];
     double u1 = rm / r1, v1 = rn / r1, w1 = rw / r1, u2 = rm / r2, v2 = rn / r2, w2 = rw / r2;
     U[IM1] = u1; V[IM1] = v1; W[IM1] = w1; U[IM2] = u2; V[IM2] = v2; W[IM2] = w2;
-    E[IM1] = r1 * (e + .5 * (u1 * u1 + v1 * v1 + w1 * w1));
-    E[IM2] = r2 * (e + .5 * (u2 * u2 + v2 * v2 + w2 * w2));
+    double e1 = r1 * (e + .5 * (u1 * u1 + v1 * v1 + w1 * w1));
+    double e2 = r2 * (e + .5 * (u2 * u2 + v2 * v2 + w2 * w2));
     if (p.iturb >= 3) {   // base3c.f:9534-9541
       b.a[FF_RK][IM1] = pa.bounrk; b.a[FF_RK][IM2] = pa.bounrk;
       b.a[FF_REPS][IM1] = pa.bounep; b.a[FF_REPS][IM2] = pa.bounep;
-      E[IM1] = E[IM1] + pa.bounrk;
-      E[IM2] = E[IM2] + pa.bounrk;
+      e1 = e1 + pa.bounrk;
+      e2 = e2 + pa.bounrk;
     }
+    E[IM1] = e1; E[IM2] = e2;
     return;
   }
   // FLUCYC's local TURLIM (res3c.f:7750); FLXCYC passes the real one
   const double turlim = p.iturb >= 3 ? p.turlim : 1.e-6;
   double rk3 = pa.ibtype == 2 ? 0.7 : 1.0, rk4 = pa.ibtype == 2 ? 0.3 : 0.0;
-  const double* NX = b.a[FF_A1XA + 4 * (fg.dir - 1)];
-  const double* NY = b.a[FF_A1YA + 4 * (fg.dir - 1)];
-  const double* NZ = b.a[FF_A1ZA + 4 * (fg.dir - 1)];
-  double a11 = NX[IF1], a12 = NY[IF1], a13 = NZ[IF1], a21, a22, a23, a31, a32, a33;
+  const double a11 = b.a[FF_A1XA + 4 * (fg.dir - 1)][IF1], a12 = b.a[FF_A1YA + 4 * (fg.dir - 1)][IF1],
+               a13 = b.a[FF_A1ZA + 4 * (fg.dir - 1)][IF1];
+  const double ui = U[II], vi = V[II], wi = W[II], um = U[IM1], vm = V[IM1], wm = W[IM1], ti = T[II];
+  const double roi = RO[II], ro1 = RO[IM1], ro2 = RO[IM2], vis2 = VIS[IM2], e2i = EPS2[II], vti = VIST[II];
+  double rk = 0., re = 0., e1 = 0., e2 = 0.;
+  if (p.iturb >= 3) { rk = b.a[FF_RK][II]; re = b.a[FF_REPS][II]; e1 = E[IM1]; e2 = E[IM2]; }
+  double a21, a22, a23, a31, a32, a33;
   surfvects(a11, a12, a13, a21, a22, a23, a31, a32, a33);
-  double veloc = .5 * (a11 * (U[II] + pa.bounu) + a12 * (V[II] + pa.bounv) + a13 * (W[II] + pa.bounw));
+  double veloc = .5 * (a11 * (ui + pa.bounu) + a12 * (vi + pa.bounv) + a13 * (wi + pa.bounw));
   P[IM1] = pa.bounp; P[IM2] = pa.bounp; PD[IM1] = pa.bounpd; PD[IM2] = pa.bounpd;
-  double eps2 = dmin(EPS2[II], turlim), vist = dmin(VIST[II], turlim * VIS[IM2]);
+  double eps2 = dmin(e2i, turlim), vist = dmin(vti, turlim * vis2);
   EPS2[IM1] = eps2; EPS2[IM2] = eps2; VIST[IM1] = vist; VIST[IM2] = vist;
   if (-veloc * fg.idir > 0.) {
-    double u = RO[II] * U[II] / RO[IM1], v = V[II], w = W[II];
+    double u = roi * ui / ro1, v = vi, w = wi;
     U[IM1] = u; U[IM2] = u; V[IM1] = v; V[IM2] = v; W[IM1] = w; W[IM2] = w;
-    T[IM1] = T[II]; T[IM2] = T[II];
-    RM[IM1] = RO[IM1] * u; RM[IM2] = RO[IM2] * u;
-    RN[IM1] = RO[IM1] * v; RN[IM2] = RO[IM2] * v;
-    RW[IM1] = RO[IM1] * w; RW[IM2] = RO[IM2] * w;
+    T[IM1] = ti; T[IM2] = ti;
+    RM[IM1] = ro1 * u; RM[IM2] = ro2 * u;
+    RN[IM1] = ro1 * v; RN[IM2] = ro2 * v;
+    RW[IM1] = ro1 * w; RW[IM2] = ro2 * w;
   } else {
-    double velc1 = a11 * U[II] + a12 * V[II] + a13 * W[II];
+    double velc1 = a11 * ui + a12 * vi + a13 * wi;
     double velc2 = a21 * pa.bounu + a22 * pa.bounv + a23 * pa.bounw;
     double velc3 = a31 * pa.bounu + a32 * pa.bounv + a33 * pa.bounw;
     double uu = a11 * velc1 + a21 * velc2 + a31 * velc3;
     double vv = a12 * velc1 + a22 * velc2 + a32 * velc3;
     double ww = a13 * velc1 + a23 * velc2 + a33 * velc3;
-    double u = rk3 * U[IM1] + rk4 * uu, v = rk3 * V[IM1] + rk4 * vv, w = rk3 * W[IM1] + rk4 * ww;
+    double u = rk3 * um + rk4 * uu, v = rk3 * vm + rk4 * vv, w = rk3 * wm + rk4 * ww;
     U[IM1] = u; U[IM2] = u; V[IM1] = v; V[IM2] = v; W[IM1] = w; W[IM2] = w;
     T[IM1] = pa.bount; T[IM2] = pa.bount;
     RO[IM1] = pa.bounr; RO[IM2] = pa.bounr;
   }
   if (p.iturb >= 3 && -veloc * fg.idir > 0.) {   // base3c.f:10134-10146
-    double rk = b.a[FF_RK][II], re = b.a[FF_REPS][II];
     b.a[FF_RK][IM1] = rk; b.a[FF_RK][IM2] = rk;
     b.a[FF_REPS][IM1] = re; b.a[FF_REPS][IM2] = re;
-    E[IM1] = E[IM1] + rk;
-    E[IM2] = E[IM2] + rk;
+    E[IM1] = e1 + rk;
+    E[IM2] = e2 + rk;
   }
 }
 
@@ -253,33 +278,54 @@ __global__ void k_mir(DevBlock b) {
   double a22 = -2. * ny * ny + 1.0, a23 = -2. * ny * nz, a33 = -2. * nz * nz + 1.0;
   double *U = b.a[FF_U], *V = b.a[FF_V], *W = b.a[FF_W];
   double u1 = U[IC1], v1 = V[IC1], w1 = W[IC1], u2 = U[IC2], v2 = V[IC2], w2 = W[IC2];
+  const int sc[8] = {FF_TEMP, FF_E, FF_P, FF_PDIFF, FF_EPS2, FF_VIST, FF_RK, FF_REPS};
+  double q1[8], q2[8];
+#pragma unroll
+  for (int s = 0; s < 8; s++) { q1[s] = b.a[sc[s]][IC1]; q2[s] = b.a[sc[s]][IC2]; }
   U[IT1] = a11 * u1 + a12 * v1 + a13 * w1;
   V[IT1] = a12 * u1 + a22 * v1 + a23 * w1;
   W[IT1] = a13 * u1 + a23 * v1 + a33 * w1;
   U[IT2] = a11 * u2 + a12 * v2 + a13 * w2;
   V[IT2] = a12 * u2 + a22 * v2 + a23 * w2;
   W[IT2] = a13 * u2 + a23 * v2 + a33 * w2;
-  const int sc[8] = {FF_TEMP, FF_E, FF_P, FF_PDIFF, FF_EPS2, FF_VIST, FF_RK, FF_REPS};
 #pragma unroll
-  for (int s = 0; s < 8; s++) { double* q = b.a[sc[s]]; q[IT1] = q[IC1]; q[IT2] = q[IC2]; }
+  for (int s = 0; s < 8; s++) { b.a[sc[s]][IT1] = q1[s]; b.a[sc[s]][IT2] = q2[s]; }
 }
 
 // REFCOR turb3.f:6040: ghost cells with two or three ghost indices copy the
-// interior edge/corner cell next to them.
+// interior edge/corner cell next to them.  One thread per cell of the twelve
+// edge bars (2 x 2 ghost cells across, the corners at their ends included),
+// 16 (IMAX + JMAX + KMAX + 12) threads; a corner belongs to three bars, which
+// write it the same value.
+__host__ __device__ inline int refcor_threads(int imax, int jmax, int kmax) {
+  return 16 * (imax + jmax + kmax + 12);
+}
 __global__ void k_refcor(DevBlock b) {
-  size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= (size_t)b.ntot) return;
-  int i = (int)(n % b.is) - 1, j = (int)((n / b.is) % (b.jmax + 4)) - 1, k = (int)(n / b.il) - 1;
-  int gi = i < 1 || i > b.imax, gj = j < 1 || j > b.jmax, gk = k < 1 || k > b.kmax;
-  if (gi + gj + gk < 2) return;
-  int ic = i < 1 ? 1 : (i > b.imax ? b.imax : i);
-  int jc = j < 1 ? 1 : (j > b.jmax ? b.jmax : j);
-  int kc = k < 1 ? 1 : (k > b.kmax ? b.kmax : k);
-  size_t src = ix(b, ic, jc, kc);
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int mx[3] = {b.imax, b.jmax, b.kmax};
+  int d = 0;
+  for (; d < 3; d++) {
+    const int len = 16 * (mx[d] + 4);
+    if (t < len) break;
+    t -= len;
+  }
+  if (d == 3) return;
+  auto ghost = [&](int q, int n) { return q < 2 ? q - 1 : n + q - 1; };   // 0..3 -> -1, 0, n + 1, n + 2
+  int c[3];
+  c[d] = t / 16 - 1;
+  c[(d + 1) % 3] = ghost(t & 3, mx[(d + 1) % 3]);
+  c[(d + 2) % 3] = ghost((t >> 2) & 3, mx[(d + 2) % 3]);
+  int in[3];
+#pragma unroll
+  for (int q = 0; q < 3; q++) in[q] = max(1, min(mx[q], c[q]));
+  const size_t n = ix(b, c[0], c[1], c[2]), src = ix(b, in[0], in[1], in[2]);
   const int sl[20] = {FF_RO, FF_RM, FF_RN, FF_RW, FF_E, FF_U, FF_V, FF_W, FF_P, FF_PDIFF,
                       FF_EPS2, FF_VIST, FF_TEMP, FF_VIS, FF_CH, FF_C, FF_DRDP, FF_DRDH, FF_RK, FF_REPS};
+  double x[20];
 #pragma unroll
-  for (int s = 0; s < 20; s++) b.a[sl[s]][n] = b.a[sl[s]][src];
+  for (int s = 0; s < 20; s++) x[s] = b.a[sl[s]][src];
+#pragma unroll
+  for (int s = 0; s < 20; s++) b.a[sl[s]][n] = x[s];
 }
 
 // DERFUN turb3.f:2476 + TEMDER turb3.f:3456 (IDERI = 1), interior + first
@@ -831,20 +877,20 @@ __global__ void k_time3_copr(DevBlock b, ff_params p, double cfl, int mode = 0) 
   double denmax = 1. + dmax(0., (ro - 2. * p.frsden) * ypro) * 5.;
   double dtl = 1. / (b11 * dmax(denlow, denmax));
   if (p.timel) dtl = dtl * p.dt / (1.5 * dtl + p.dt);   // TIMEL dual time step, base3c.f:206-215
-  b.a[FF_DTL][kk] = dtl;
-  if (mode == 1) return;
+  if (mode == 1) { b.a[FF_DTL][kk] = dtl; return; }
   // LOCDT + COPR
   double dri = dtl * b.a[FF_DRO][kk], dmi = dtl * b.a[FF_DM][kk], dni = dtl * b.a[FF_DN][kk];
   double dwi = dtl * b.a[FF_DW][kk], dre = dtl * b.a[FF_DE][kk];
-  double yp = 1. / ro, drodh = b.a[FF_DRDH][kk], drodp = b.a[FF_DRDP][kk];
+  double yp = 1. / ro, drodh = b.a[FF_DRDH][kk], drodp = b.a[FF_DRDP][kk], e = b.a[FF_E][kk];
   double beta = .5 * (u * u + v * v + w * w);
   double dkin = u * dmi + v * dni + w * dwi;
+  double hi = yp * (e + P);
+  double dei = dre - (hi - 2 * beta) * dri - dkin;
+  double dpi = c * c * (dri - drodh * yp * dei);
+  b.a[FF_DTL][kk] = dtl;
   b.a[FF_DM][kk] = yp * (-u * dri + dmi);
   b.a[FF_DN][kk] = yp * (-v * dri + dni);
   b.a[FF_DW][kk] = yp * (-w * dri + dwi);
-  double hi = yp * (b.a[FF_E][kk] + P);
-  double dei = dre - (hi - 2 * beta) * dri - dkin;
-  double dpi = c * c * (dri - drodh * yp * dei);
   b.a[FF_DRO][kk] = (dri - drodp * dpi) / drodh;
   b.a[FF_DE][kk] = dpi;
 }
@@ -1156,24 +1202,33 @@ __global__ void k_fin(DevBlock b, ff_params p, unsigned long long* dromax_bits, 
     bool interior = kin && jin && i >= 2 && i < b.imax + 2;
     double T = b.a[FF_TEMP][n], U = b.a[FF_U][n], V = b.a[FF_V][n], W = b.a[FF_W][n], PD = b.a[FF_PDIFF][n];
     const bool sst = p.iturb >= 3;
+    double rk = 0., re = 0.;
+    if (sst) { rk = b.a[FF_RK][n]; re = b.a[FF_REPS][n]; }
     if (interior) {
-      double dt = b.a[FF_DRO][n];
-      if (divide_cp) { dt = dt / b.a[FF_CP][n]; b.a[FF_DRO][n] = dt; }
-      if (sst) {   // imps3.f:488-492, then FIN res3c.f:1190-1198
-        double ro = b.a[FF_RO][n], drk = b.a[FF_DRK][n], deps = b.a[FF_DEPS][n];
-        if (divide_cp) { drk = drk * ro; deps = deps * ro; b.a[FF_DRK][n] = drk; b.a[FF_DEPS][n] = deps; }
-        double rkold = b.a[FF_RKOLD][n], epold = b.a[FF_EPSOLD][n];
-        double rk = rkold + drk / (1. + fabs(drk) / (.45 * rkold));
-        double re = epold + deps / (1. + fabs(deps) / (.90 * epold));
-        b.a[FF_RK][n] = rk;
-        b.a[FF_REPS][n] = re;
+      double dt = b.a[FF_DRO][n], dm = b.a[FF_DM][n], dn = b.a[FF_DN][n], dw = b.a[FF_DW][n], de = b.a[FF_DE][n];
+      const double told = b.a[FF_TOLD][n], uold = b.a[FF_UOLD][n], vold = b.a[FF_VOLD][n], wold = b.a[FF_WOLD][n],
+                   pold = b.a[FF_POLD][n];
+      double drk = 0., deps = 0., rkold = 0., epold = 0.;
+      if (sst) { drk = b.a[FF_DRK][n]; deps = b.a[FF_DEPS][n]; rkold = b.a[FF_RKOLD][n]; epold = b.a[FF_EPSOLD][n]; }
+      if (divide_cp) {
+        const double cp = b.a[FF_CP][n], ro = sst ? b.a[FF_RO][n] : 0.;
+        dt = dt / cp;
+        b.a[FF_DRO][n] = dt;
+        if (sst) {   // imps3.f:488-492
+          drk = drk * ro; deps = deps * ro;
+          b.a[FF_DRK][n] = drk; b.a[FF_DEPS][n] = deps;
+        }
       }
-      T = b.a[FF_TOLD][n] + dt;
-      U = b.a[FF_UOLD][n] + b.a[FF_DM][n];
-      V = b.a[FF_VOLD][n] + b.a[FF_DN][n];
-      W = b.a[FF_WOLD][n] + b.a[FF_DW][n];
-      PD = b.a[FF_POLD][n] + b.a[FF_DE][n];
-      amax = fabs(b.a[FF_DE][n]);
+      if (sst) {   // FIN res3c.f:1190-1198
+        rk = rkold + drk / (1. + fabs(drk) / (.45 * rkold));
+        re = epold + deps / (1. + fabs(deps) / (.90 * epold));
+      }
+      T = told + dt;
+      U = uold + dm;
+      V = vold + dn;
+      W = wold + dw;
+      PD = pold + de;
+      amax = fabs(de);
     }
     if (kin && jin) {   // UPLIM range: interior k-planes, interior rows
       T = dmin(T, p.tuplim); U = dmin(U, 5000.); V = dmin(V, 5000.); W = dmin(W, 5000.);
@@ -1185,8 +1240,8 @@ __global__ void k_fin(DevBlock b, ff_params p, unsigned long long* dromax_bits, 
     b.a[FF_TEMP][n] = T; b.a[FF_U][n] = U; b.a[FF_V][n] = V; b.a[FF_W][n] = W;
     b.a[FF_PDIFF][n] = PD; b.a[FF_P][n] = P;
     if (sst) {   // LOLIM of RK and REPS over every cell (FIN, then CYCLES)
-      b.a[FF_RK][n] = dmax(b.a[FF_RK][n], p.rklim);
-      b.a[FF_REPS][n] = dmax(b.a[FF_REPS][n], p.epslim);
+      b.a[FF_RK][n] = dmax(rk, p.rklim);
+      b.a[FF_REPS][n] = dmax(re, p.epslim);
     }
     if (interior) {
       b.a[FF_TOLD][n] = T; b.a[FF_UOLD][n] = U; b.a[FF_VOLD][n] = V; b.a[FF_WOLD][n] = W;
@@ -1421,12 +1476,15 @@ __global__ void k_connec(const DevBlock* __restrict__ blocks, const ConnItem* __
   size_t S = face_cell(s, fs, ad, cd);
   const int vs[12] = {FF_TEMP, FF_U, FF_V, FF_W, FF_E, FF_EPS2, FF_VIST, FF_CH, FF_P, FF_PDIFF, FF_RK, FF_REPS};
   int lsd = fd.idir * fd.s, lss = fs.idir * fs.s;
+  double x[2][12];
 #pragma unroll
-  for (int g = 1; g <= 2; g++) {
-    size_t G = L - g * lsd, Q = S + (g - 1) * lss;
+  for (int g = 0; g < 2; g++)
 #pragma unroll
-    for (int v = 0; v < 12; v++) d.a[vs[v]][G] = s.a[vs[v]][Q];
-  }
+    for (int v = 0; v < 12; v++) x[g][v] = s.a[vs[v]][S + g * lss];
+#pragma unroll
+  for (int g = 0; g < 2; g++)
+#pragma unroll
+    for (int v = 0; v < 12; v++) d.a[vs[v]][L - (g + 1) * lsd] = x[g][v];
 }
 
 // Halo pack (mode 0, from the source block) / unpack (mode 1, into the

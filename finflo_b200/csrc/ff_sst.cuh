@@ -758,20 +758,19 @@ __global__ void k_locdtk_imsoko_coprke(DevBlock b, ff_params p) {
   drk = drk / drkden;
   deps = deps / domden;
   // COPRKE imps3.f:1113
-  double u = b.a[FF_U][i], v = b.a[FF_V][i], w = b.a[FF_W][i];
+  double u = b.a[FF_U][i], v = b.a[FF_V][i], w = b.a[FF_W][i], c = b.a[FF_C][i], P = b.a[FF_P][i];
   double vel2 = u * u + v * v + w * w;
   double drodh = b.a[FF_DRDH][i], drodp = b.a[FF_DRDP][i];
   double ypro = 1. / ro, rki = rk * ypro;
   double dkin = u * dmi + v * dni + w * dwi + drk;
+  double hi = ypro * (E + P);
+  double dei = dre - (hi - vel2 - rki) * dri - dkin;
+  double dpi = c * c * (dri - drodh * ypro * dei);
   b.a[FF_DM][i] = ypro * (-u * dri + dmi);
   b.a[FF_DN][i] = ypro * (-v * dri + dni);
   b.a[FF_DW][i] = ypro * (-w * dri + dwi);
   b.a[FF_DRK][i] = ypro * (-rki * dri + drk);
   b.a[FF_DEPS][i] = ypro * (-rom * ypro * dri + deps);
-  double hi = ypro * (E + b.a[FF_P][i]);
-  double dei = dre - (hi - vel2 - rki) * dri - dkin;
-  double c = b.a[FF_C][i];
-  double dpi = c * c * (dri - drodh * ypro * dei);
   b.a[FF_DRO][i] = (dri - drodp * dpi) / drodh;
   b.a[FF_DE][i] = dpi + .667 * drk;
 }
