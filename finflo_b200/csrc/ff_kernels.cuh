@@ -401,10 +401,13 @@ FF_DI FaceGeom face_geom(const DevBlock& b, size_t L, int S, int dir) {
   FaceGeom g;
   const size_t M = L - S;
   const double* D = b.a[FF_D1 + dir - 1];
-  g.w1 = 2.0 * (__ldg(D + L) / (__ldg(D + L) + __ldg(D + M)));
+  const double dl = __ldg(D + L);
+  g.w1 = 2.0 * (dl * rcp(dl + __ldg(D + M)));
   g.w2 = 2.0 - g.w1;
   double sx = LD(FF_XC, L) - LD(FF_XC, M), sy = LD(FF_YC, L) - LD(FF_YC, M), sz = LD(FF_ZC, L) - LD(FF_ZC, M);
-  g.slen = sqrt(sx * sx + sy * sy + sz * sz) + 1.e-21;
+  double rs_;
+  sqrt_rsq(dmax(sx * sx + sy * sy + sz * sz, 1.e-300), g.slen, rs_);
+  g.slen += 1.e-21;
   g.rslen = rcp(g.slen);
   g.sx = sx * g.rslen; g.sy = sy * g.rslen; g.sz = sz * g.rslen;
   const int ao = 4 * (dir - 1);

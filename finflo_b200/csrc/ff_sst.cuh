@@ -213,8 +213,9 @@ FF_DI void roe_flux_ke(const T q[7][4], T nx, T ny, T nz, T area, int intem, int
   T eim = pmi * rgm1 * yprol - e0;
   T elr = ppi * rgm1 * yprol - e0;
   T erl = pmi * rgm1 * ypror - e0;
-  T ypro1 = rcp(cr[2]), ypro2 = rcp(cl2[2]);
-  T rdh1 = rcp(cr[1]), rdh2 = rcp(cl2[1]);
+  const T rc1 = rcp(cr[1] * cr[2]), rc2 = rcp(cl2[1] * cl2[2]);   // 1 / (DRDH RO) of both cells
+  T ypro1 = rc1 * cr[1], ypro2 = rc2 * cl2[1];
+  T rdh1 = rc1 * cr[2], rdh2 = rc2 * cl2[2];
   T dedph = T(0.5) * ((-cr[0] * rdh1 - ypro1) + (-cl2[0] * rdh2 - ypro2));
   T dedrh = T(0.5) * ((rdh1 + cr[3] * (ypro1 * ypro1)) + (rdh2 + cl2[3] * (ypro2 * ypro2)));
   {
@@ -236,7 +237,8 @@ FF_DI void roe_flux_ke(const T q[7][4], T nx, T ny, T nz, T area, int intem, int
   T pr = ppi, pl = pmi, pkr = T(.6667) * rkipi, pkl = T(.6667) * rkimi;
   T epsr = reipi * ypror, epsl = reimi * yprol;
   T hr = eir + pr * ypror, hl = eil + yprol * pl;
-  T rohat = sqrt(roip * roim), yproh = rcp(rohat);
+  T rohat, yproh;
+  sqrt_rsq(roip * roim, rohat, yproh);
   T sqrl = rcp(roim + rohat), cql = roim * sqrl, cqr = T(1.) - cql;
   T uhat = cqr * ur + cql * ul;
   const T thx = cqr * txr + cql * txl, thy = cqr * tyr + cql * tyl, thz = cqr * tzr + cql * tzl;
@@ -245,18 +247,19 @@ FF_DI void roe_flux_ke(const T q[7][4], T nx, T ny, T nz, T area, int intem, int
   T phat = rohat * (hhat - ehat - T(.5) * (uhat * uhat + thx * thx + thy * thy + thz * thz) - rkhat);
   phat = dmin(dmax(pr, pl), phat);
   phat = dmax(dmin(pr, pl), phat);
-  T drdhh = rcp(dedrh - phat * (yproh * yproh));
-  T drdph = -drdhh * (dedph + yproh);
-  T xturb = T(1.) + T(.6667) * rkhat * yproh * drdph;
-  T chat2 = xturb / (drdhh * yproh + drdph);
+  // DRDHH = 1 / D, D = DEDRH - PHAT / ROHAT^2, DRDPH = -DRDHH (DEDPH + 1 / ROHAT),
+  // CHAT^2 = (1 + .6667 RKHAT / ROHAT DRDPH) / (DRDHH / ROHAT + DRDPH), whose
+  // denominator is -DRDHH DEDPH
+  T chat2 = ((phat * (yproh * yproh) - dedrh) + T(.6667) * rkhat * yproh * (dedph + yproh)) * rcp(dedph);
   T cmin = dmin(c_r, c_l), cmax = dmax(c_r, c_l);
   chat2 = dmin(cmax * cmax, chat2);
   chat2 = dmax(cmin * cmin, chat2);
-  T chat = sqrt(chat2);
+  T chat, rchat;
+  sqrt_rsq(chat2, chat, rchat);
   T pdpde = dedph;
   T dro = roip - roim, du = ur - ul, dk = rkr - rkl;
   T dp = pr - pl + T(.6667) * (rkhat * dro + rohat * dk);
-  T pchat2 = rcp(chat * chat);
+  T pchat2 = rchat * rchat;
   T alfa1 = T(.5) * (dp + rohat * chat * du) * pchat2;
   T alfa2 = T(.5) * (dp - rohat * chat * du) * pchat2;
   T alfa3 = dro - dp * pchat2;
