@@ -286,36 +286,22 @@ int st_residu_sst(Ctx* c, BlockCtx* b, int level, int m2, int icycle, int part =
   if (part == 2) goto post;
   {
   launch_scalard(c, b, level);
-  const int ncell = b->imax * b->jmax * b->kmax;
   int gg = level == 1 ? 2 : 0;
   long ng = (long)(b->imax + gg) * (b->jmax + gg) * (b->kmax + gg);
-  if (m2 >= 2 || level == 1) {   // DERFUN (+ TEMDER of T) of this level
-    k_grad<<<nblk(ng, 128), 128, 0, c->stream>>>(b->db, level);
-    c->nlaunch++;
-  }
-  if (level == 1 && m2 == 1) {
-    k_eps2ko<<<nblk(ncell, 128), 128, 0, c->stream>>>(b->db, b->prm);
-    c->nlaunch++;
-  }
-  k_crosko<<<nblk(ncell, 128), 128, 0, c->stream>>>(b->db);
-  k_rk_roundtrip<<<nblk(b->ntot, 256), 256, 0, c->stream>>>(b->db);
+  // TURBEQ's DERFUN (m2 = 1 on level 1) or RESIKE's (m2 >= 2) of this level, EPS2KO, CROSKO
   CK(cudaMemsetAsync(b->d_red, 0, sizeof(unsigned long long), c->stream));
-  k_cdmax<<<min(nblk(b->ntot, 256), 4 * c->sm_count), 256, 0, c->stream>>>(b->db, b->d_red);
-  k_fun1ko<<<nblk(ncell, 128), 128, 0, c->stream>>>(b->db, b->prm, b->d_red);
-  c->nlaunch += 4;
+  k_pre_ke<<<nblk(ng, 128), 128, 0, c->stream>>>(b->db, b->prm, level, level == 1 && m2 == 1, b->d_red);
+  c->nlaunch++;
   if (b->npatch && level == 1) {
     int maxn = 1;
     for (auto& p : b->h_patch) maxn = max(maxn, (p.r1b - p.r1a + 1) * (p.r2b - p.r2a + 1));
     k_refcen<<<dim3(nblk(maxn, 128), b->npatch), 128, 0, c->stream>>>(b->db, b->prm);
     c->nlaunch++;
   }
-  k_prodke<<<nblk((long)b->jmax * b->db.is * b->kmax, 128), 128, 0, c->stream>>>(b->db);
+  // FUN1KO, PRODKE, TEMDER of k and omega
+  k_temder_fun<<<nblk((long)b->db.is * (b->jmax + 2) * (b->kmax + 2), 128), 128, 0, c->stream>>>(
+      b->db, b->prm, level, b->prm.fullns, b->d_red);
   c->nlaunch++;
-  if (b->prm.fullns) {
-    long nt3 = (long)(b->imax + gg) * (b->jmax + gg) * ((level == 1 && b->kmax > 1) ? b->kmax + 2 : b->kmax);
-    k_temder_ke<<<nblk(nt3, 128), 128, 0, c->stream>>>(b->db, level);
-    c->nlaunch++;
-  }
   if (level == 1) launch_patch(c, b, k_inlet_outlet, icycle);
   }
   if (part == 1) return 0;
@@ -325,8 +311,10 @@ int st_residu_sst(Ctx* c, BlockCtx* b, int level, int m2, int icycle, int part =
   }
 post:
   const int ncell = b->imax * b->jmax * b->kmax;
-  k_sourko_addske<<<nblk(ncell, 128), 128, 0, c->stream>>>(b->db);
-  c->nlaunch++;
+  if (!res_fused()) {   // the fused residual adds the sources itself
+    k_sourko_addske<<<nblk(ncell, 128), 128, 0, c->stream>>>(b->db);
+    c->nlaunch++;
+  }
   if (b->prm.timel && level == 1) {   // TIMDER + TIMDKE after ADDSKE (res3c.f:5097)
     k_timder<7><<<nblk(ncell, 256), 256, 0, c->stream>>>(b->db, b->prm);
     c->nlaunch++;

@@ -328,16 +328,9 @@ __global__ void k_refcor(DevBlock b) {
   for (int s = 0; s < 20; s++) b.a[sl[s]][n] = x[s];
 }
 
-// DERFUN turb3.f:2476 + TEMDER turb3.f:3456 (IDERI = 1), interior + first
-// ghost layer on level 1.
-__global__ void k_grad(DevBlock b, int level) {
-  int lo = level == 1 ? 0 : 1, hi = level == 1 ? 1 : 0;
-  int ni = b.imax + hi - lo + 1, nj = b.jmax + hi - lo + 1, nk = b.kmax + hi - lo + 1;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ni * nj * nk) return;
-  int I = lo + t % ni, J = lo + (t / ni) % nj, K = lo + t / (ni * nj);
+// DERFUN turb3.f:2476 + TEMDER turb3.f:3456 (IDERI = 1) of one cell; returns STRAIN.
+FF_DI double grad_cell(const DevBlock& b, int level, int K, size_t L) {
   const int IS = b.is, IL = b.il;
-  size_t L = ix(b, I, J, K);
   const double *U = b.a[FF_U], *V = b.a[FF_V], *W = b.a[FF_W], *T = b.a[FF_TEMP];
   const double *A1 = b.a[FF_A1], *A2 = b.a[FF_A2], *A3 = b.a[FF_A3];
   const double *D1 = b.a[FF_D1], *D2 = b.a[FF_D2], *D3 = b.a[FF_D3];
@@ -352,13 +345,14 @@ __global__ void k_grad(DevBlock b, int level) {
 #pragma unroll
     for (int side = 0; side < 2; side++) {
       size_t nb = side == 0 ? L - st[d] : L + st[d];
-      double w1 = 2.0 * (Dd[d][L] / (Dd[d][L] + Dd[d][nb])), w2 = 2.0 - w1;
+      const double dl = Dd[d][L];
+      double w1 = 2.0 * (dl * rcp(dl + Dd[d][nb])), w2 = 2.0 - w1;
       aa[2 * d + side] = side == 0 ? Ad[d][L] : Ad[d][L + st[d]];
 #pragma unroll
       for (int v = 0; v < 4; v++) q[v][2 * d + side] = w2 * F[v][L] + w1 * F[v][nb];
     }
   }
-  double pvol = .5 / b.a[FF_VOL][L];
+  double pvol = .5 * rcp(b.a[FF_VOL][L]);
   double g[3][3];   // g[v][x] = d(u_v)/dx_x
 #pragma unroll
   for (int x = 0; x < 3; x++) {
@@ -383,7 +377,20 @@ __global__ void k_grad(DevBlock b, int level) {
   b.a[FF_S11][L] = s11; b.a[FF_S12][L] = s12; b.a[FF_S13][L] = s13;
   b.a[FF_S22][L] = s22; b.a[FF_S23][L] = s23; b.a[FF_S33][L] = s33;
   double stn = s11 * s11 + 2. * s12 * s12 + 2. * s13 * s13 + s22 * s22 + 2. * s23 * s23 + s33 * s33;
-  b.a[FF_STRAIN][L] = sqrt(2. * stn);
+  const double strain = sqrt(2. * stn);
+  b.a[FF_STRAIN][L] = strain;
+  return strain;
+}
+
+// DERFUN + TEMDER on the interior and, on level 1, the first ghost layer
+// (laminar; k_pre_ke does it for k-omega).
+__global__ void k_grad(DevBlock b, int level) {
+  int lo = level == 1 ? 0 : 1, hi = level == 1 ? 1 : 0;
+  int ni = b.imax + hi - lo + 1, nj = b.jmax + hi - lo + 1, nk = b.kmax + hi - lo + 1;
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= ni * nj * nk) return;
+  int I = lo + t % ni, J = lo + (t / ni) % nj, K = lo + t / (ni * nj);
+  grad_cell(b, level, K, ix(b, I, J, K));
 }
 
 // FLUXBL base3c.f:4085 (IDIFF = 1) for the face between M = L-S and L; the

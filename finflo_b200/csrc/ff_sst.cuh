@@ -14,15 +14,23 @@ constexpr double SST_A1KLEB = 0.31, SST_BSTAR = 0.09, SST_CKAPPA = 0.41, SST_BET
 constexpr double SST_SIGRK1 = 0.85, SST_SIGOM1 = 0.5, SST_BETA2 = 0.0828, SST_SIGRK2 = 1.0,
                  SST_SIGOM2 = 0.856;
 
-// ---- TURBEQ: EPS2KO with STRAIN (res3c.f:6338), interior cells ----------
-__global__ void k_eps2ko(DevBlock b, ff_params p) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= b.imax * b.jmax * b.kmax) return;
-  int I = t % b.imax + 1, J = (t / b.imax) % b.jmax + 1, K = t / (b.imax * b.jmax) + 1;
-  size_t L = ix(b, I, J, K);
+// ---- before the face pass -------------------------------------------------
+// The steps of TURBEQ and RESIKE before the face fluxes in two kernels (they
+// were eight): what bounds them is memory, and DERFUN, CROSKO and TEMDER of k
+// and omega each read the twelve face-metric arrays, the volume and the
+// thicknesses.  128x64x64 cells, one level-1 pass: k_grad 57.4, k_eps2ko 10.7,
+// k_crosko 27.8, k_rk_roundtrip 7.0, k_cdmax 6.7, k_fun1ko 11.2, k_prodke 11.0,
+// k_temder_ke 73.8 us before; k_pre_ke 62.9, k_temder_fun 35.9 us now.  The two are
+// apart because FUN1KO needs the largest cross diffusion of the block and
+// TEMDER the wall ghosts REFCEN fills in between.
+//
+// CROSKO divides RK and REPS by RO in place and multiplies them back, which
+// leaves them a rounding away from what they were; that step is not repeated.
+
+// EPS2KO turb3.f:7454 with STRAIN (res3c.f:6338) of one cell.
+FF_DI void eps2ko_cell(const DevBlock& b, const ff_params& p, size_t L, double st, double ro, double rk, double rom) {
   const double eps = 1.e-20, frsmut = 1.e-3 * p.frsvis;
-  double ro = b.a[FF_RO][L], rk = b.a[FF_RK][L], rom = b.a[FF_REPS][L], dw = b.a[FF_DISTW][L];
-  double vis = b.a[FF_VIS][L], st = b.a[FF_STRAIN][L];
+  double dw = b.a[FF_DISTW][L], vis = b.a[FF_VIS][L];
   double prol = 1. / ro;
   double rkl = dmax(rk * prol, 0.0);
   double oml = rom * prol;
@@ -42,71 +50,57 @@ __global__ void k_eps2ko(DevBlock b, ff_params p) {
   b.a[FF_EPS2][L] = 1.0 + rmutrb / vis;
 }
 
-// ---- CROSKO: cross diffusion into SEPS (interior).  k and omega of every
-// stencil cell are RK/RO and REPS/RO as the reference's in-place division
-// leaves them; k_rk_roundtrip then applies its RK = (RK/RO)*RO round trip.
-__global__ void k_crosko(DevBlock b) {
+// DERFUN + TEMDER of T on the level's range (grad_cell), and on the interior
+// cells EPS2KO (eps2 = 1) and CROSKO: the cross diffusion into SEPS and its
+// largest positive value (FUN1KO's CDMAX; non-negative doubles order like
+// their bit patterns) into cdmax_bits.
+__global__ void __launch_bounds__(128) k_pre_ke(DevBlock b, ff_params p, int level, int eps2,
+                                                unsigned long long* cdmax_bits) {
+  int lo = level == 1 ? 0 : 1, hi = level == 1 ? 1 : 0;
+  int ni = b.imax + hi - lo + 1, nj = b.jmax + hi - lo + 1, nk = b.kmax + hi - lo + 1;
   int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= b.imax * b.jmax * b.kmax) return;
-  int I = t % b.imax + 1, J = (t / b.imax) % b.jmax + 1, K = t / (b.imax * b.jmax) + 1;
-  const int IS = b.is, IL = b.il;
-  size_t L = ix(b, I, J, K);
-  const double *RK = b.a[FF_RK], *RE = b.a[FF_REPS], *RO = b.a[FF_RO];
-#define KV(n) (RK[n] * (1. / RO[n]))
-#define OV(n) (RE[n] * (1. / RO[n]))
-#define LD(s, n) __ldg(b.a[s] + (n))
-  double k0 = KV(L), o0 = OV(L);
-  double rk1m = LD(FF_A1, L) * (k0 + KV(L - 1)), rk1p = LD(FF_A1, L + 1) * (k0 + KV(L + 1));
-  double om1m = LD(FF_A1, L) * (o0 + OV(L - 1)), om1p = LD(FF_A1, L + 1) * (o0 + OV(L + 1));
-  double rk2m = LD(FF_A2, L) * (k0 + KV(L - IS)), rk2p = LD(FF_A2, L + IS) * (k0 + KV(L + IS));
-  double om2m = LD(FF_A2, L) * (o0 + OV(L - IS)), om2p = LD(FF_A2, L + IS) * (o0 + OV(L + IS));
-  double rk3m = LD(FF_A3, L) * (k0 + KV(L - IL)), rk3p = LD(FF_A3, L + IL) * (k0 + KV(L + IL));
-  double om3m = LD(FF_A3, L) * (o0 + OV(L - IL)), om3p = LD(FF_A3, L + IL) * (o0 + OV(L + IL));
-  double pvol = 0.5 / LD(FF_VOL, L);
-#define CSUM(c, p3, m3, p2, m2, p1, m1)                                                                   \
-  (pvol * (LD(FF_A3##c, L + IL) * p3 - LD(FF_A3##c, L) * m3 + LD(FF_A2##c, L + IS) * p2 -               \
-           LD(FF_A2##c, L) * m2 + LD(FF_A1##c, L + 1) * p1 - LD(FF_A1##c, L) * m1))
-  double dkdx = CSUM(XA, rk3p, rk3m, rk2p, rk2m, rk1p, rk1m);
-  double dkdy = CSUM(YA, rk3p, rk3m, rk2p, rk2m, rk1p, rk1m);
-  double dkdz = CSUM(ZA, rk3p, rk3m, rk2p, rk2m, rk1p, rk1m);
-  double dodx = CSUM(XA, om3p, om3m, om2p, om2m, om1p, om1m);
-  double dody = CSUM(YA, om3p, om3m, om2p, om2m, om1p, om1m);
-  double dodz = CSUM(ZA, om3p, om3m, om2p, om2m, om1p, om1m);
-#undef CSUM
-#undef LD
-#undef KV
-#undef OV
-  double divdot = dkdx * dodx + dkdy * dody + dkdz * dodz;
-  b.a[FF_SEPS][L] = 2.0 * SST_SIGOM2 * RO[L] * divdot / o0;
-}
-
-__global__ void k_rk_roundtrip(DevBlock b) {
-  size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= (size_t)b.ntot) return;
-  double ro = b.a[FF_RO][n], prol = 1. / ro;
-  b.a[FF_RK][n] = (b.a[FF_RK][n] * prol) * ro;
-  b.a[FF_REPS][n] = (b.a[FF_REPS][n] * prol) * ro;
-}
-
-// CDMAX of FUN1KO: max(0, CROSSD) over the storage range from cell (1,1,1)
-// to (IMAX,JMAX,KMAX); non-negative doubles order like their bit patterns.
-__global__ void k_cdmax(DevBlock b, unsigned long long* out) {
-  size_t lbeg = ix(b, 1, 1, 1), lend = ix(b, b.imax, b.jmax, b.kmax);
   double m = 0.;
-  for (size_t n = lbeg + (size_t)blockIdx.x * blockDim.x + threadIdx.x; n <= lend;
-       n += (size_t)gridDim.x * blockDim.x)
-    m = dmax(b.a[FF_SEPS][n], m);
+  if (t < ni * nj * nk) {
+    int I = lo + t % ni, J = lo + (t / ni) % nj, K = lo + t / (ni * nj);
+    const int IS = b.is, IL = b.il;
+    size_t L = ix(b, I, J, K);
+    const double strain = grad_cell(b, level, K, L);
+    if (I >= 1 && I <= b.imax && J >= 1 && J <= b.jmax && K >= 1 && K <= b.kmax) {
+      const double *RK = b.a[FF_RK], *RE = b.a[FF_REPS], *RO = b.a[FF_RO];
+#define LD(s, n) __ldg(b.a[s] + (n))
+      const double ro = RO[L], rk = RK[L], re = RE[L], r0 = rcp(ro), k0 = rk * r0, o0 = re * r0;
+      if (eps2) eps2ko_cell(b, p, L, strain, ro, rk, re);
+      const int st[3] = {1, IS, IL};
+      double gk[3] = {0., 0., 0.}, go[3] = {0., 0., 0.};
+#pragma unroll
+      for (int d = 2; d >= 0; d--) {
+        const size_t Lp = L + st[d], Lm = L - st[d];
+        const double rp = rcp(RO[Lp]), rm = rcp(RO[Lm]);
+        const double ap = LD(FF_A1 + 4 * d, Lp), am = LD(FF_A1 + 4 * d, L);
+        const double kp = ap * (k0 + RK[Lp] * rp), km = am * (k0 + RK[Lm] * rm);
+        const double op = ap * (o0 + RE[Lp] * rp), om = am * (o0 + RE[Lm] * rm);
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const double np = LD(FF_A1XA + 4 * d + c, Lp), nm = LD(FF_A1XA + 4 * d + c, L);
+          gk[c] += np * kp - nm * km;
+          go[c] += np * op - nm * om;
+        }
+      }
+      const double pvol = 0.5 * rcp(LD(FF_VOL, L));
+#undef LD
+      const double divdot = (gk[0] * pvol) * (go[0] * pvol) + (gk[1] * pvol) * (go[1] * pvol) + (gk[2] * pvol) * (go[2] * pvol);
+      const double cd = 2.0 * SST_SIGOM2 * ro * divdot / o0;
+      b.a[FF_SEPS][L] = cd;
+      m = dmax(cd, 0.);
+    }
+  }
   for (int o = 16; o > 0; o >>= 1) m = dmax(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m > 0.) atomicMax(out, (unsigned long long)__double_as_longlong(m));
+  if ((threadIdx.x & 31) == 0 && m > 0.) atomicMax(cdmax_bits, (unsigned long long)__double_as_longlong(m));
 }
 
-__global__ void k_fun1ko(DevBlock b, ff_params p, const unsigned long long* cdmax_bits) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= b.imax * b.jmax * b.kmax) return;
-  int I = t % b.imax + 1, J = (t / b.imax) % b.jmax + 1, K = t / (b.imax * b.jmax) + 1;
-  size_t L = ix(b, I, J, K);
+// FUN1KO turb3.f:7385 of one interior cell.
+FF_DI void fun1ko_cell(const DevBlock& b, const ff_params& p, size_t L, double cdmin) {
   const double eps = 1.e-20;
-  double cdmin = 1e-8 * __longlong_as_double((long long)*cdmax_bits);
   double ro = b.a[FF_RO][L], rk = b.a[FF_RK][L], rom = b.a[FF_REPS][L], dw = b.a[FF_DISTW][L];
   double prol = 1. / ro;
   double rkl = dmax(rk * prol, 0.0);
@@ -123,14 +117,8 @@ __global__ void k_fun1ko(DevBlock b, ff_params p, const unsigned long long* cdma
   b.a[FF_FUN1][L] = f1;
 }
 
-// MAKE_EPS + PRODKE (Kato-Launder): rows J = 1..JMAX of the interior
-// k-planes, i ghosts included, as the reference loops.
-__global__ void k_prodke(DevBlock b) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  int per = b.jmax * b.is;
-  if (t >= per * b.kmax) return;
-  int K = t / per + 1, jj = t % per;
-  size_t L = (size_t)(K + 1) * b.il + 2 * b.is + jj;
+// MAKE_EPS + PRODKE (Kato-Launder) of one cell.
+FF_DI void prodke_cell(const DevBlock& b, size_t L) {
 #define A(s) b.a[s][L]
   double s11 = A(FF_S11), s12 = A(FF_S12), s13 = A(FF_S13), s22 = A(FF_S22), s23 = A(FF_S23), s33 = A(FF_S33);
   double strain = s11 * s11 + s12 * s12 + s13 * s13 + s12 * s12 + s22 * s22 + s23 * s23 + s13 * s13 + s23 * s23 +
@@ -142,47 +130,55 @@ __global__ void k_prodke(DevBlock b) {
 #undef A
 }
 
+// FUN1KO on the interior cells, PRODKE on rows J = 1..JMAX of the interior
+// k-planes (i ghosts included, as the reference loops), and with temder = 1
 // TEMDER of k = RK/RO and omega = REPS/RO (DIVV12 + TEMDER, res3c.f:3994-4006)
-// over the TEMDER range of level 1.
-__global__ void k_temder_ke(DevBlock b, int level) {
-  const int lo = level == 1 ? 0 : 1, g = level == 1 ? 2 : 0;
-  int ni = b.imax + g, nj = b.jmax + g;
-  int klo = (level == 1 && b.kmax > 1) ? 0 : 1, nk = (level == 1 && b.kmax > 1) ? b.kmax + 2 : b.kmax;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ni * nj * nk) return;
-  int I = t % ni + lo, J = (t / ni) % nj + lo, K = t / (ni * nj) + klo;
+// over the TEMDER range of the level.  One thread per cell of the storage
+// rows (all i) of J, K = 0..MAX+1.
+__global__ void __launch_bounds__(128) k_temder_fun(DevBlock b, ff_params p, int level, int temder,
+                                                    const unsigned long long* cdmax_bits) {
   const int IS = b.is, IL = b.il;
-  size_t L = ix(b, I, J, K);
-  const double *RO = b.a[FF_RO];
-#define LD(s, n) __ldg(b.a[s] + (n))
-  const size_t nb[6] = {L - 1, L + 1, L - (size_t)IS, L + IS, L - (size_t)IL, L + IL};
-  const int dslot[6] = {FF_D1, FF_D1, FF_D2, FF_D2, FF_D3, FF_D3};
-  double w1[6], w2[6];
-#pragma unroll
-  for (int q = 0; q < 6; q++) {
-    double dl = LD(dslot[q], L);
-    w1[q] = 2.0 * (dl / (dl + LD(dslot[q], nb[q])));
-    w2[q] = 2.0 - w1[q];
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= IS * (b.jmax + 2) * (b.kmax + 2)) return;
+  const int I = t % IS - 1, J = (t / IS) % (b.jmax + 2), K = t / (IS * (b.jmax + 2));
+  const size_t L = ix(b, I, J, K);
+  const bool jk = J >= 1 && J <= b.jmax && K >= 1 && K <= b.kmax;
+  if (jk) {
+    prodke_cell(b, L);
+    if (I >= 1 && I <= b.imax) fun1ko_cell(b, p, L, 1e-8 * __longlong_as_double((long long)*cdmax_bits));
   }
-  double pvol = .5 / LD(FF_VOL, L);
+  const int lo = level == 1 ? 0 : 1, g = 1 - lo;
+  const int klo = (level == 1 && b.kmax > 1) ? 0 : 1, khi = (level == 1 && b.kmax > 1) ? b.kmax + 1 : b.kmax;
+  if (!temder || I < lo || I > b.imax + g || J < lo || J > b.jmax + g || K < klo || K > khi) return;
+  const double *RO = b.a[FF_RO], *RK = b.a[FF_RK], *RE = b.a[FF_REPS];
+#define LD(s, n) __ldg(b.a[s] + (n))
+  const int st[3] = {1, IS, IL};
+  const double r0 = rcp(RO[L]), k0 = RK[L] * r0, o0 = RE[L] * r0;
+  double gk[3] = {0., 0., 0.}, go[3] = {0., 0., 0.};
 #pragma unroll
-  for (int f = 0; f < 2; f++) {
-    const double* PH = b.a[f == 0 ? FF_RK : FF_REPS];
-    double ph0 = PH[L] / RO[L];
-    double t_[6];
+  for (int d = 2; d >= 0; d--) {
+    const double dl = LD(FF_D1 + d, L);
 #pragma unroll
-    for (int q = 0; q < 6; q++) t_[q] = w2[q] * ph0 + w1[q] * (PH[nb[q]] / RO[nb[q]]);
-    // t_: 1m, 1p, 2m, 2p, 3m, 3p
+    for (int side = 1; side >= 0; side--) {
+      const size_t nb = side ? L + st[d] : L - st[d], fc = side ? nb : L;
+      const double w1 = 2.0 * (dl * rcp(dl + LD(FF_D1 + d, nb))), w2 = 2.0 - w1, rn = rcp(RO[nb]);
+      const double ar = side ? LD(FF_A1 + 4 * d, fc) : -LD(FF_A1 + 4 * d, fc);
+      const double kf = ar * (w2 * k0 + w1 * (RK[nb] * rn)), of = ar * (w2 * o0 + w1 * (RE[nb] * rn));
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const int x1 = FF_A1XA + c, x2 = FF_A2XA + c, x3 = FF_A3XA + c;
-      double g = pvol * (LD(FF_A3, L + IL) * LD(x3, L + IL) * t_[5] - LD(FF_A3, L) * LD(x3, L) * t_[4] +
-                         LD(FF_A2, L + IS) * LD(x2, L + IS) * t_[3] - LD(FF_A2, L) * LD(x2, L) * t_[2] +
-                         LD(FF_A1, L + 1) * LD(x1, L + 1) * t_[1] - LD(FF_A1, L) * LD(x1, L) * t_[0]);
-      b.a[(f == 0 ? FF_DKDX : FF_DEDX) + c][L] = g;
+      for (int c = 0; c < 3; c++) {
+        const double nn = LD(FF_A1XA + 4 * d + c, fc);
+        gk[c] += nn * kf;
+        go[c] += nn * of;
+      }
     }
   }
+  const double pvol = .5 * rcp(LD(FF_VOL, L));
 #undef LD
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    b.a[FF_DKDX + c][L] = pvol * gk[c];
+    b.a[FF_DEDX + c][L] = pvol * go[c];
+  }
 }
 
 // ---- face fluxes of the seven equations ---------------------------------
@@ -575,6 +571,38 @@ __global__ void __launch_bounds__(NT, RES_MIN_CTAS * 128 / NT) k_residual_sst(De
   }
 }
 
+// SOURKO (KOVER=0, RANS, no rotation correction) of one interior cell: SRK and
+// SEPS, and what ADDSKE adds to the k and omega residuals.
+FF_DI void sourko_cell(const DevBlock& b, size_t L, double& srk, double& som) {
+  const double pbstar = 1.0 / SST_BSTAR, persbs = 1.0 / sqrt(SST_BSTAR), eps = 1.0E-10;
+  double f1 = b.a[FF_FUN1][L], onemf1 = dmax(0.0, 1.0 - f1);
+  double beta = f1 * SST_BETA1 + onemf1 * SST_BETA2;
+  double sigom = f1 * SST_SIGOM1 + onemf1 * SST_SIGOM2;
+  double gamkom = beta * pbstar - sigom * (SST_CKAPPA * SST_CKAPPA) * persbs;
+  double rmutrb = dmax(eps, b.a[FF_EPS2][L] - 1.0) * b.a[FF_VIS][L];
+  double ro = b.a[FF_RO][L], rom = b.a[FF_REPS][L], pt = b.a[FF_PTUR][L];
+  double prol = 1.0 / ro;
+  som = onemf1 * b.a[FF_SEPS][L];
+  srk = pt - SST_BSTAR * b.a[FF_RK][L] * rom * prol;
+  double omepro = gamkom * ro * pt / (rmutrb * rom);
+  double omedis = 1.0 * beta * prol * rom;
+  som = som + rom * (omepro - omedis);
+  b.a[FF_SRK][L] = srk;
+  b.a[FF_SEPS][L] = som;
+}
+
+// SOURKO + ADDSKE after the one-barrier-per-direction residual (FINFLO_RES_FUSED=0).
+__global__ void k_sourko_addske(DevBlock b) {
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= b.imax * b.jmax * b.kmax) return;
+  int I = t % b.imax + 1, J = (t / b.imax) % b.jmax + 1, K = t / (b.imax * b.jmax) + 1;
+  size_t L = ix(b, I, J, K);
+  double srk, som;
+  sourko_cell(b, L, srk, som);
+  b.a[FF_DRK][L] = b.a[FF_DRK][L] + srk;
+  b.a[FF_DEPS][L] = b.a[FF_DEPS][L] + som;
+}
+
 // RESIDU/RESIKE for a 32x4x4 tile with all three directions' faces in one
 // work list: the k, i and j faces (640 + 528 + 640) are computed by NT
 // threads into one shared-memory face buffer with a single barrier, then
@@ -650,12 +678,15 @@ FF_DI void residual_tile(const DevBlock& b, const ff_params& p, int level, int i
     const int fi0 = NFK + ci + (TI + 1) * (cj + TJ * ck);          // face I-1/2; I+1/2 at + 1
     const int fj0 = NFK + NFI + ci + TI * (cj + (TJ + 1) * ck);    // face J-1/2; J+1/2 at + TI
     const size_t n = ix(b, I, J, K);
-    const double rv = 1. / __ldg(b.a[FF_VOL] + n);
+    const double rv = rcp(__ldg(b.a[FF_VOL] + n));
+    double src[2] = {0., 0.};
+    if constexpr (NV == 7) sourko_cell(b, n, src[0], src[1]);   // SOURKO + ADDSKE
 #pragma unroll
     for (int v = 0; v < NV; v++) {
       double acc = 0. - (sF[v][fk0 + TI * TJ] - sF[v][fk0]);
       acc = acc - (sF[v][fi0 + 1] - sF[v][fi0]);
-      b.a[FF_DRO + v][n] = (acc - (sF[v][fj0 + TI] - sF[v][fj0])) * rv;
+      const double r = (acc - (sF[v][fj0 + TI] - sF[v][fj0])) * rv;
+      b.a[FF_DRO + v][n] = v < 5 ? r : r + src[v - 5];
     }
   }
 }
@@ -710,31 +741,6 @@ inline size_t residual_fused_smem(int nv, int ti = TI, int tj = TJ, int tk = TK,
 // j, k) and staged stencil or not (form s: shape s % 3, staged for s >= 3).
 constexpr int RES_NSHAPE = 3, RES_NFORM = 6;
 constexpr int RES_SHAPES[RES_NSHAPE][3] = {{32, 4, 4}, {16, 8, 4}, {8, 8, 8}};
-
-// SOURKO (KOVER=0, RANS, no rotation correction) + ADDSKE, interior cells.
-__global__ void k_sourko_addske(DevBlock b) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= b.imax * b.jmax * b.kmax) return;
-  int I = t % b.imax + 1, J = (t / b.imax) % b.jmax + 1, K = t / (b.imax * b.jmax) + 1;
-  size_t L = ix(b, I, J, K);
-  const double pbstar = 1.0 / SST_BSTAR, persbs = 1.0 / sqrt(SST_BSTAR), eps = 1.0E-10;
-  double f1 = b.a[FF_FUN1][L], onemf1 = dmax(0.0, 1.0 - f1);
-  double beta = f1 * SST_BETA1 + onemf1 * SST_BETA2;
-  double sigom = f1 * SST_SIGOM1 + onemf1 * SST_SIGOM2;
-  double gamkom = beta * pbstar - sigom * (SST_CKAPPA * SST_CKAPPA) * persbs;
-  double rmutrb = dmax(eps, b.a[FF_EPS2][L] - 1.0) * b.a[FF_VIS][L];
-  double ro = b.a[FF_RO][L], rom = b.a[FF_REPS][L], pt = b.a[FF_PTUR][L];
-  double prol = 1.0 / ro;
-  double som = onemf1 * b.a[FF_SEPS][L];
-  double srk = pt - SST_BSTAR * b.a[FF_RK][L] * rom * prol;
-  double omepro = gamkom * ro * pt / (rmutrb * rom);
-  double omedis = 1.0 * beta * prol * rom;
-  som = som + rom * (omepro - omedis);
-  b.a[FF_SRK][L] = srk;
-  b.a[FF_SEPS][L] = som;
-  b.a[FF_DRK][L] = b.a[FF_DRK][L] + srk;
-  b.a[FF_DEPS][L] = b.a[FF_DEPS][L] + som;
-}
 
 // LOCDTK (DTURB=1) + IMSOKO + COPRKE, after TIME3 wrote DTL (interior).
 __global__ void k_locdtk_imsoko_coprke(DevBlock b, ff_params p) {
