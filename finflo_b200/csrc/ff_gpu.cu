@@ -63,7 +63,7 @@ struct BlockCtx {
   PipeGeom pg{};
   float pipe_ms = 0.f;          // measured upper sweep of the pipelined kernel
   int tuned = 0;                // sweep kind chosen by tune_sweep
-  int res_shape = 0;            // residual tile shape (RES_SHAPES), chosen by tune_residual
+  int res_shape = 0;            // residual form (RES_FORMS), chosen by tune_residual
   int res_tuned = 0;
   float sweep_ms[2] = {0.f, 0.f};   // measured upper sweep: lines, best hyperplane
   DevBlock db{};
@@ -237,15 +237,18 @@ void launch_residual_fused_t(cudaStream_t st, dim3 g, const BlockCtx* b, int lev
   if (residual_alt(b->prm, level)) return launch_residual_fused_s<NV, NT, 32, 4, 4, false, double, true>(st, b, level);
   // a coarse level's face fluxes in FP32 (unstaged tiles; Roe with XXTRAP)
   if (level > 1 && b->prm.res_fp32) {
-    const int s3 = sh % RES_NSHAPE;
-    if (s3 == 1) return launch_residual_fused_s<NV, NT, 16, 8, 4, false, float>(st, b, level);
-    if (s3 == 2) return launch_residual_fused_s<NV, NT, 8, 8, 8, false, float>(st, b, level);
+    if (NT == 512 && sh == 6) return launch_residual_fused_s<NV, NT, 8, 4, 4, false, float>(st, b, level);
+    if (sh % 3 == 1) return launch_residual_fused_s<NV, NT, 16, 8, 4, false, float>(st, b, level);
+    if (sh % 3 == 2) return launch_residual_fused_s<NV, NT, 8, 8, 8, false, float>(st, b, level);
     return launch_residual_fused_s<NV, NT, 32, 4, 4, false, float>(st, b, level);
   }
   if constexpr (NT == 512) {
     if (sh == 3) return launch_residual_fused_s<NV, NT, 32, 4, 4, true>(st, b, level);
     if (sh == 4) return launch_residual_fused_s<NV, NT, 16, 8, 4, true>(st, b, level);
     if (sh == 5) return launch_residual_fused_s<NV, NT, 8, 8, 8, true>(st, b, level);
+    if (sh == 6) return launch_residual_fused_s<NV, NT, 8, 4, 4>(st, b, level);
+    if (sh == 7) return launch_residual_fused_s<NV, 256, 8, 8, 4>(st, b, level);
+    if (sh == 8) return launch_residual_fused_s<NV, 256, 16, 4, 4>(st, b, level);
   }
   if (sh == 1) return launch_residual_fused_s<NV, NT, 16, 8, 4>(st, b, level);
   if (sh == 2) return launch_residual_fused_s<NV, NT, 8, 8, 8>(st, b, level);
@@ -351,22 +354,58 @@ int st_residu(Ctx* c, BlockCtx* b, int level, int icycle, int m2 = 1, int part =
   return 0;
 }
 
+// The residual form without timing, by the number of 8x4x4 and 16x4x4 tiles
+// (times in us, forms 32x4x4 / 8x4x4 / 16x4x4 x2, SST): up to one 8x4x4 tile an
+// SM the single round is fastest (32x16x16 cells 40.7 / 16.5 / 32.9), from two
+// 16x4x4 tiles an SM on the two 256-thread CTAs (90x50x34 88.0 / 103 / 79.8,
+// 248x136x72 959 / 1309 / 911), between them 32x4x4 (64x32x32 37.0 / 43.2 / 41.1).
+inline int res_rule(const Ctx* c, long t844, long t1644) {
+  return t844 <= c->sm_count ? 6 : (t1644 >= 2 * c->sm_count ? 8 : 0);
+}
+inline int res_rule(const Ctx* c, const BlockCtx* b) {
+  const long jk = (long)nblk(b->jmax, 4) * nblk(b->kmax, 4);
+  return res_rule(c, nblk(b->imax, 8) * jk, nblk(b->imax, 16) * jk);
+}
+
 // The residual face pass of several level-1 blocks in one launch over their
 // tiles (k_residual_batch, RB_MAX blocks per launch); every block must have
-// the same equation count.  The tile shape is the first block's.
-template <int NV, int I_, int J_, int K_, bool ST = false>
+// the same equation count.
+template <int NV, int F>
 void launch_residual_batch_t(cudaStream_t st, const ResBatch& rb, int level) {
-  const size_t sm = residual_fused_smem(NV, I_, J_, K_, ST);
-  cudaFuncSetAttribute(k_residual_batch<NV, 512, I_, J_, K_, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sm);
-  k_residual_batch<NV, 512, I_, J_, K_, ST><<<rb.tile0[rb.nblk], 512, sm, st>>>(rb, level);
+  constexpr ResForm f = RES_FORMS[F];
+  const size_t sm = residual_fused_smem(NV, f.ti, f.tj, f.tk, f.staged);
+  auto k = k_residual_batch<NV, f.nt, f.ti, f.tj, f.tk, f.staged != 0>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k<<<rb.tile0[rb.nblk], f.nt, sm, st>>>(rb, level);
+}
+
+template <int NV>
+void launch_residual_batch_f(cudaStream_t st, const ResBatch& rb, int level, int form) {
+  switch (form) {
+    case 1: launch_residual_batch_t<NV, 1>(st, rb, level); break;
+    case 2: launch_residual_batch_t<NV, 2>(st, rb, level); break;
+    case 3: launch_residual_batch_t<NV, 3>(st, rb, level); break;
+    case 4: launch_residual_batch_t<NV, 4>(st, rb, level); break;
+    case 5: launch_residual_batch_t<NV, 5>(st, rb, level); break;
+    case 6: launch_residual_batch_t<NV, 6>(st, rb, level); break;
+    case 7: launch_residual_batch_t<NV, 7>(st, rb, level); break;
+    case 8: launch_residual_batch_t<NV, 8>(st, rb, level); break;
+    default: launch_residual_batch_t<NV, 0>(st, rb, level);
+  }
 }
 
 int launch_residual_batch(Ctx* c, const std::vector<BlockCtx*>& blks, int level) {
-  const int shape = blks[0]->res_shape;
+  // the rule of res_rule on the tiles of all blocks together
+  long t844 = 0, t1644 = 0;
+  for (const BlockCtx* b : blks) {
+    const long jk = (long)nblk(b->jmax, 4) * nblk(b->kmax, 4);
+    t844 += nblk(b->imax, 8) * jk;
+    t1644 += nblk(b->imax, 16) * jk;
+  }
+  static const int env = [] { const char* e = getenv("FINFLO_RES_SHAPE"); return e ? atoi(e) : -1; }();
+  const int shape = env >= 0 && env < RES_NFORM ? env : res_rule(c, t844, t1644);
   const bool sst = blks[0]->prm.iturb >= 3;
-  const int ti = RES_SHAPES[shape % RES_NSHAPE][0], tj = RES_SHAPES[shape % RES_NSHAPE][1],
-            tk = RES_SHAPES[shape % RES_NSHAPE][2];
+  const int ti = RES_FORMS[shape].ti, tj = RES_FORMS[shape].tj, tk = RES_FORMS[shape].tk;
   for (size_t s0 = 0; s0 < blks.size(); s0 += RB_MAX) {
     static ResBatch rb;   // ~19 KB: kept off the host stack
     rb = ResBatch{};
@@ -381,20 +420,8 @@ int launch_residual_batch(Ctx* c, const std::vector<BlockCtx*>& blks, int level)
       rb.b[n] = b->db;
       rb.p[n] = b->prm;
     }
-    switch (shape) {
-      case 1: sst ? launch_residual_batch_t<7, 16, 8, 4>(c->stream, rb, level)
-                  : launch_residual_batch_t<5, 16, 8, 4>(c->stream, rb, level); break;
-      case 2: sst ? launch_residual_batch_t<7, 8, 8, 8>(c->stream, rb, level)
-                  : launch_residual_batch_t<5, 8, 8, 8>(c->stream, rb, level); break;
-      case 3: sst ? launch_residual_batch_t<7, 32, 4, 4, true>(c->stream, rb, level)
-                  : launch_residual_batch_t<5, 32, 4, 4, true>(c->stream, rb, level); break;
-      case 4: sst ? launch_residual_batch_t<7, 16, 8, 4, true>(c->stream, rb, level)
-                  : launch_residual_batch_t<5, 16, 8, 4, true>(c->stream, rb, level); break;
-      case 5: sst ? launch_residual_batch_t<7, 8, 8, 8, true>(c->stream, rb, level)
-                  : launch_residual_batch_t<5, 8, 8, 8, true>(c->stream, rb, level); break;
-      default: sst ? launch_residual_batch_t<7, 32, 4, 4>(c->stream, rb, level)
-                   : launch_residual_batch_t<5, 32, 4, 4>(c->stream, rb, level);
-    }
+    if (sst) launch_residual_batch_f<7>(c->stream, rb, level, shape);
+    else launch_residual_batch_f<5>(c->stream, rb, level, shape);
     c->nlaunch++;
   }
   CK(cudaGetLastError());
@@ -826,10 +853,11 @@ int tune_ddadi(Ctx* c, BlockCtx* b, const TuneKey& key) {
   return 0;
 }
 
-// Residual form of a block: each tile shape of RES_SHAPES, with and without
-// the staged stencil, timed on the block's own level (CUDA events, after
-// one untimed launch), the fastest kept; cached per device, block shape and
-// equation count.  FINFLO_RES_SHAPE (0..5) fixes it.
+// Residual form of a block: each unstaged one of RES_FORMS (the staged ones
+// were slower on every shape tried; FINFLO_RES_SHAPE still selects them) timed
+// on the block's own level (CUDA events, after one untimed launch), the
+// fastest kept; cached per device, block shape and equation count.
+// FINFLO_RES_SHAPE (0..8) fixes it.
 std::map<TuneKey, int> g_res_cache;
 
 int tune_residual(Ctx* c, BlockCtx* b) {
@@ -848,6 +876,7 @@ int tune_residual(Ctx* c, BlockCtx* b) {
   float best = 1e30f;
   int pick = 0;
   for (int s = 0; s < RES_NFORM; s++) {
+    if (RES_FORMS[s].staged) continue;
     b->res_shape = s;
     launch_residual(c->stream, b, b->level);
     CK(cudaEventRecord(c->ev0, c->stream));
@@ -1697,6 +1726,7 @@ static int block_add(Ctx* c, int imax, int jmax, int kmax, int npatch, const ff_
   b->db.is = imax + 4; b->db.il = (imax + 4) * (jmax + 4); b->db.ntot = b->ntot;
   b->db.npatch = npatch; b->db.patch = b->d_patch;
   for (int s = 0; s < FF_NSLOTS; s++) b->db.a[s] = b->base + (size_t)s * b->slot_stride;
+  b->res_shape = res_rule(c, b);
   {
     int rc = pick_sweep(c, b);
     if (rc || (rc = alloc_sweep(c, b))) return rc;

@@ -719,7 +719,7 @@ struct ResBatch {
   ff_params p[RB_MAX];
 };
 
-template <int NV, int NT, int TI_, int TJ_, int TK_, bool STAGE = false>
+template <int NV, int NT, int TI_, int TJ_, int TK_, bool STAGE>
 __global__ void __launch_bounds__(NT, RES_MIN_CTAS * 128 / NT)
     k_residual_batch(const __grid_constant__ ResBatch rb, int level) {
   extern __shared__ double res_smem[];
@@ -737,10 +737,20 @@ inline size_t residual_fused_smem(int nv, int ti = TI, int tj = TJ, int tk = TK,
   return (faces + box) * sizeof(double);
 }
 
-// The residual forms the autotuner chooses from: tile shape (cells in i,
-// j, k) and staged stencil or not (form s: shape s % 3, staged for s >= 3).
-constexpr int RES_NSHAPE = 3, RES_NFORM = 6;
-constexpr int RES_SHAPES[RES_NSHAPE][3] = {{32, 4, 4}, {16, 8, 4}, {8, 8, 8}};
+// The residual forms the autotuner chooses from: tile shape (cells in i, j,
+// k), threads of a CTA, staged stencil or not.  The face work of a tile is
+// dealt out in rounds of one face a thread, and with one 512-thread CTA an SM
+// every warp waits at the tile's barrier for the last, part-filled round;
+// two 256-thread CTAs (their face buffers together as large) fill each other's
+// waits.  8x4x4 at 512 threads is a single round: the shortest time for blocks
+// of few tiles.
+struct ResForm {
+  int ti, tj, tk, nt, staged;
+};
+constexpr int RES_NFORM = 9;
+constexpr ResForm RES_FORMS[RES_NFORM] = {{32, 4, 4, 512, 0}, {16, 8, 4, 512, 0}, {8, 8, 8, 512, 0},
+                                          {32, 4, 4, 512, 1}, {16, 8, 4, 512, 1}, {8, 8, 8, 512, 1},
+                                          {8, 4, 4, 512, 0},  {8, 8, 4, 256, 0},  {16, 4, 4, 256, 0}};
 
 // LOCDTK (DTURB=1) + IMSOKO + COPRKE, after TIME3 wrote DTL (interior).
 __global__ void k_locdtk_imsoko_coprke(DevBlock b, ff_params p) {

@@ -348,7 +348,7 @@ class GpuSolver:
 
     def residual_shape(self, bid=0) -> str:
         return ("32x4x4", "16x8x4", "8x8x8", "32x4x4 staged", "16x8x4 staged",
-                "8x8x8 staged")[self.L.ff_residual_shape(self.ctx, bid)]
+                "8x8x8 staged", "8x4x4", "8x8x4 x2", "16x4x4 x2")[self.L.ff_residual_shape(self.ctx, bid)]
 
     def lusgs_kind(self, bid=0) -> int:
         return self.L.ff_lusgs_kind(self.ctx, bid)
