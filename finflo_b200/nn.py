@@ -19,7 +19,7 @@ NVCC_FLAGS = ["-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "-Xcompiler", "-fPIC", "-shared", "-std=c++17"]
 
 SYMBOLS = ["ffnn_gemm", "ffnn_silu_bwd", "ffnn_colsum", "ffnn_transpose", "ffnn_to_bf16", "ffnn_mse",
-           "ffnn_adam", "ffnn_error"]
+           "ffnn_adam", "ffnn_error", "ffnn_wgrad", "ffnn_silu_bwd_bias", "ffnn_mse_bias"]
 
 
 class NNError(RuntimeError):
@@ -51,6 +51,9 @@ def lib():
         L.ffnn_mse.argtypes = [vp, ci, vp, ci, ci, vp, vp, vp, vp]
         L.ffnn_adam.argtypes = [vp, vp, vp, vp, cl, cf, cf, cf, cf, ci, cf, vp, vp, ci, vp]
         L.ffnn_error.argtypes = [ci]
+        L.ffnn_wgrad.argtypes = [vp, ci, vp, ci, ci, ci, ci, vp, ci, vp]
+        L.ffnn_silu_bwd_bias.argtypes = [vp, vp, ci, ci, vp, vp, vp, vp]
+        L.ffnn_mse_bias.argtypes = [vp, ci, vp, ci, ci, vp, vp, vp, vp, vp]
         _LIB = L
     return _LIB
 
@@ -99,6 +102,36 @@ def gemm(A, B, *, bias=None, act=0, zf=None, yb=None, atomic=False, ksplit=0):
 def silu_bwd(dy, z, dzb=None, dzf=None):
     _check(lib().ffnn_silu_bwd(dy.data_ptr(), z.data_ptr(), z.numel(), _ptr(dzb), _ptr(dzf), _stream()),
            "ffnn_silu_bwd")
+
+
+def wgrad(x, y, g):
+    """g[N,K] += x[rows,N]^T y[rows,K], BF16 operands, FP32 sums over the rows."""
+    import torch
+    if x.dtype != torch.bfloat16 or y.dtype != torch.bfloat16 or g.dtype != torch.float32:
+        raise NNError("wgrad: bfloat16 operands, float32 result")
+    rows, N = x.shape
+    K = y.shape[1]
+    if y.shape[0] != rows or g.shape[0] < N or g.shape[1] < K:
+        raise NNError(f"wgrad: shapes {tuple(x.shape)}, {tuple(y.shape)}, {tuple(g.shape)}")
+    _check(lib().ffnn_wgrad(x.data_ptr(), _rowmajor(x, "x"), y.data_ptr(), _rowmajor(y, "y"), rows, N, K, g.data_ptr(),
+                            _rowmajor(g, "g"), _stream()), "ffnn_wgrad")
+
+
+def silu_bwd_bias(dy, z, dzb, gbias, dzf=None):
+    """silu_bwd on [rows, cols] and gbias += the column sums of dz."""
+    rows, cols = dzb.shape
+    for t, n in ((dy, "dy"), (z, "z"), (dzb, "dzb")):
+        if not t.is_contiguous() or t.numel() != rows * cols:
+            raise NNError(f"silu_bwd_bias: {n} must be a contiguous [rows, cols]")
+    _check(lib().ffnn_silu_bwd_bias(dy.data_ptr(), z.data_ptr(), rows, cols, dzb.data_ptr(), _ptr(dzf), gbias.data_ptr(),
+                                    _stream()), "ffnn_silu_bwd_bias")
+
+
+def mse_bias(pred, tgt, grad, loss, gbias, gradf=None):
+    """mse and gbias += the column sums of the gradient."""
+    rows, ld = pred.shape
+    _check(lib().ffnn_mse_bias(pred.data_ptr(), ld, tgt.data_ptr(), rows, tgt.shape[1], grad.data_ptr(), _ptr(gradf),
+                               loss.data_ptr(), gbias.data_ptr(), _stream()), "ffnn_mse_bias")
 
 
 def colsum(x, out):

@@ -167,10 +167,6 @@ def normalise_params(*cols, spec=BUMP):
     return x
 
 
-def _r16(n):
-    return (n + 15) // 16 * 16
-
-
 @dataclass
 class Layer:
     name: str
@@ -289,8 +285,6 @@ class WarmStartNet:
         self.dA = torch.empty(big, dtype=f32, device=d)
         self.dB = torch.empty(big, dtype=f32, device=d)
         self.dzb = torch.empty(big, dtype=b16, device=d)
-        self.tA = torch.empty(max(big, self.spec.enc[-1] * _r16(B)), dtype=b16, device=d)
-        self.tB = torch.empty(max(big, self.spec.enc[-1] * _r16(B)), dtype=b16, device=d)
         self.loss = torch.zeros(1, dtype=f32, device=d)
 
     # -- forward ------------------------------------------------------------------
@@ -313,20 +307,6 @@ class WarmStartNet:
         return self.pred
 
     # -- backward + update ----------------------------------------------------------
-    def _wgrad(self, l, dzb, x, rows):
-        """gW(l) += dz^T x over `rows` rows: both operands transposed so that
-        the reduction (the rows) is the GEMM's contiguous K, split over CTAs."""
-        nn = self.nn
-        rp = _r16(rows)
-        a = self.tA[:l.n * rp].view(l.n, rp)
-        b = self.tB[:l.k * rp].view(l.k, rp)
-        nn.transpose(dzb, a, rows_pad=rp)
-        nn.transpose(x, b, rows_pad=rp)
-        tiles = ((l.n + 127) // 128) * ((l.k + 255) // 256)
-        splits = max(1, min(rp // 64, 296 // tiles))
-        ks = max(64, (rp + splits - 1) // splits + 63) // 64 * 64
-        nn.gemm(a, b, zf=self.gW(l), atomic=True, ksplit=ks)
-
     def backward(self, tgt, capture=None):
         """Gradients of the mean-squared error of self.pred against tgt
         [B * ncell, nvar] (normalised targets, octree order) into self.g.
@@ -338,7 +318,8 @@ class WarmStartNet:
         self.g.zero_()
         self.loss.zero_()
         V = self.nvox
-        nn.mse(self.pred, tgt, self.dpred, self.loss, gradf=self.dpredf)
+        keep = capture is not None   # the FP32 pre-activation gradients are only needed by the checks
+        nn.mse_bias(self.pred, tgt, self.dpred, self.loss, self.gb(self.L[-1]), gradf=self.dpredf if keep else None)
         bufA, bufB = self.dA, self.dB
         dy = None
         for l in reversed(self.L):
@@ -351,12 +332,12 @@ class WarmStartNet:
                 dzb = self.dzb[:rows * l.n].view(rows, l.n)
                 dzf = bufB[:rows * l.n].view(rows, l.n)
                 if l.act:
-                    nn.silu_bwd(dy, self.z[l.name], dzb=dzb, dzf=dzf)
+                    nn.silu_bwd_bias(dy, self.z[l.name], dzb, self.gb(l), dzf=dzf if keep else None)
                 else:
                     nn.to_bf16(dy, dzb)
+                    nn.colsum(dy, self.gb(l))
                     dzf = dy
-            self._wgrad(l, dzb, x, rows)
-            nn.colsum(dzf, self.gb(l))
+            nn.wgrad(dzb, x.reshape(rows, l.k), self.gW(l))
             if capture is not None:
                 capture[l.name] = {"dzb": dzb.clone(), "dzf": dzf.clone(), "x": x.reshape(rows, l.k).clone()}
             if l.name == "enc1":

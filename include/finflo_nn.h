@@ -37,6 +37,22 @@ int ffnn_gemm(const void *A, int lda, const void *B, int ldb, int M, int N, int 
 /* dz = dy * SiLU'(z) element-wise over n values; dzb (BF16) and/or dzf (FP32). */
 int ffnn_silu_bwd(const float *dy, const float *z, long n, void *dzb, float *dzf, void *stream);
 
+/* G[N,K] += X[rows,N]^T * Y[rows,K], the sum over the rows, BF16 operands, FP32
+ * sums (weight gradients straight from the layer's row-major gradient and
+ * input).  N, K, ldx, ldy multiples of 8, K <= 256, X and Y 16-byte aligned. */
+int ffnn_wgrad(const void *X, int ldx, const void *Y, int ldy, int rows, int N, int K, float *G, int ldg, void *stream);
+
+/* ffnn_silu_bwd of a contiguous [rows, cols] with gbias[c] += the column sums
+ * of dz; dzf may be NULL.  cols a multiple of 4 with cols / 4 a power of two up
+ * to 64; 16-byte aligned arrays. */
+int ffnn_silu_bwd_bias(const float *dy, const float *z, int rows, int cols, void *dzb, float *dzf, float *gbias,
+                       void *stream);
+
+/* ffnn_mse with gbias[c] += the column sums of the gradient, c < ld (ld as
+ * cols above). */
+int ffnn_mse_bias(const float *pred, int ld, const float *tgt, int rows, int cols, void *grad, float *gradf, float *loss,
+                  float *gbias, void *stream);
+
 /* out[c] += sum_r x[r*ld + c] for c < cols (bias gradients). */
 int ffnn_colsum(const float *x, int rows, int cols, int ld, float *out, void *stream);
 
