@@ -138,28 +138,45 @@ __global__ void k_flow_static(DevBlock b, FlowGeom g, CT* __restrict__ up, CT* _
     }
 }
 
-// The state-dependent rows of both sweeps' records and the right-hand side of
-// the upper sweep's (PREDGS imps4.f:388-470, DIAGGS 604-660, CORRGS 120-200):
-// one pass over the state for both sweeps, whose diagonal factor needs the
-// low and the high faces anyway.  Also rewinds the tile counters.
-// A thread block is eight consecutive steps of one tile: each of its lines is
-// read in runs of eight cells, each row of a record written as one run of 32.
-// drop: the upper sweep leaves out the i+1 coupling of row JMAX (PREDGS,
-// imps4.f:1460-1466).
+// TIME3, LOCDT and COPR (LOCDTK, IMSOKO, COPRKE), the state-dependent rows of
+// both sweeps' records and the right-hand side of the upper sweep's (PREDGS
+// imps4.f:388-470, DIAGGS 604-660, CORRGS 120-200): one pass over the state
+// for both sweeps, whose diagonal factor needs the low and the high faces
+// anyway.  Also rewinds the tile counters.
+//
+// A warp is 8 consecutive cells of 4 lines that are neighbours in j: a load is
+// four runs of 64 bytes, and of a record's row, which holds the lines' cells
+// of one diagonal, the four lanes of a diagonal of the warp write one sector.
+// With one thread a slot, in record order, stores were whole lines but each
+// load touched 32 sectors; turning the values in shared memory instead cost
+// the occupancy that the chains of divisions need (128x64x64 cells, seven
+// equations: 142 us in three passes with the time step and the conversion on
+// their own, 165 us through shared memory, 104 us now).  Reciprocals are
+// rcp's where the divisor cannot be zero or infinite.
 template <typename CT, int NV>
-__global__ void __launch_bounds__(256) k_flow_coef(DevBlock b, ff_params p, FlowGeom g, CT* __restrict__ up,
+__global__ void __launch_bounds__(256, 4) k_flow_coef(DevBlock b, ff_params p, ff::TimeConst tc, FlowGeom g, CT* __restrict__ up,
                                                    CT* __restrict__ lo, unsigned* ticket) {
   using R = FlowRec<NV>;
-  const size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n < 2) ticket[n] = 0u;
-  int I, J, K;
-  if (n >= (size_t)g.ntiles * g.ns * 32 || !flow_cell(b, g, n, I, J, K)) return;
-  const size_t N = ix(b, I, J, K), o = (n >> 5) * (R::N * 32) + (n & 31);
+  if (blockIdx.x == 0 && threadIdx.x < 2) ticket[threadIdx.x] = 0u;
+  const int nch = (b.imax + 7) / 8;
+  const int tile = blockIdx.x / nch, i0 = (blockIdx.x - tile * nch) * 8;
+  const int tk = tile / g.ntj, tj = tile - tk * g.ntj;
+  const int line = threadIdx.x / 8, lj = line % FTJ, lk = line / FTJ, I = i0 + threadIdx.x % 8 + 1;
+  const int J = tj * FTJ + lj + 1, K = tk * FTK + lk + 1;
+  if (I > b.imax || J > b.jmax || K > b.kmax) return;
+  const size_t N = ix(b, I, J, K), rec = ((size_t)tile * g.ns + I - 1 + lj + lk) * (R::N * 32) + line;
+  CT *o = up + rec, *ol = lo + rec;
 #define LD(s, m) __ldg(b.a[s] + (m))
+  const double dtl = ff::time3_cell(b, p, tc, I, J, K, N), dt1 = p.theta * dtl;
+  double x[NV];
+  if constexpr (NV == 7) ff::coprke_cell(b, p, dtl, N, x);
+  else ff::copr_cell(b, dtl, N, x);
+#pragma unroll
+  for (int q = 0; q < NV; q++) o[q * 32] = (CT)x[q];
   const double u = LD(FF_U, N), v = LD(FF_V, N), w = LD(FF_W, N), c = LD(FF_C, N), ro = LD(FF_RO, N);
-  const double vol = LD(FF_VOL, N), mu = LD(FF_VIST, N) + LD(FF_VIS, N), dt1 = p.theta * LD(FF_DTL, N);
+  const double vol = LD(FF_VOL, N), mu = LD(FF_VIST, N) + LD(FF_VIS, N);
   const int st[3] = {1, b.is, b.il}, idi[3] = {p.idi1, p.idi2, p.idi3}, idx[3] = {I, J, K};
-  double alo[3], ahi[3], mup[3], mlo[3], su = 0., sl = 0., pu = 0., pl = 0., sd = 0.;
+  double alo[3], ahi[3], su = 0., sl = 0., pu = 0., pl = 0., sd = 0.;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     const int ao = 4 * d;
@@ -170,42 +187,37 @@ __global__ void __launch_bounds__(256) k_flow_coef(DevBlock b, ff_params p, Flow
     const double rhi = LD(FF_A1XA + ao, hi) * u + LD(FF_A1YA + ao, hi) * v + LD(FF_A1ZA + ao, hi) * w;
     double tu = 0., tl = 0.;
     if (idx[d] <= idi[d]) {
-      tu = (idx[d] == 1 ? 8. : 4.) * alo[d] / ((vol + LD(FF_VOL, lw)) * (ro + LD(FF_RO, lw))) *
+      tu = (idx[d] == 1 ? 8. : 4.) * alo[d] * rcp((vol + LD(FF_VOL, lw)) * (ro + LD(FF_RO, lw))) *
            (mu + LD(FF_VIST, lw) + LD(FF_VIS, lw));
-      tl = 4. * alo[d] / ((vol + LD(FF_VOL, hi)) * (ro + LD(FF_RO, hi))) * (mu + LD(FF_VIST, hi) + LD(FF_VIS, hi));
+      tl = 4. * alo[d] * rcp((vol + LD(FF_VOL, hi)) * (ro + LD(FF_RO, hi))) * (mu + LD(FF_VIST, hi) + LD(FF_VIS, hi));
     }
     const double rmu = fabs(rlo) + c, rml = fabs(rhi) + c;
-    mup[d] = dmin(rlo, 0.) - tu - .5 * c;
-    mlo[d] = dmax(rhi, 0.) + tl + .5 * c;
+    o[(R::L + d) * 32] = (CT)(dmin(rlo, 0.) - tu - .5 * c);
+    ol[(R::L + d) * 32] = (CT)(dmax(rhi, 0.) + tl + .5 * c);
     su += (rmu + tu) * alo[d];
     sl += (rml + tl) * ahi[d];
     pu += rmu * alo[d];
     pl += rml * alo[d];
     sd += alo[d] * rmu + ahi[d] * rml;
   }
-  const double scu = 1. / (vol + dt1 * su), scl = 1. / (vol + dt1 * sl);
-  const double fd = 1. + dt1 / vol * (.5 * sd);
-  up[o + R::AL * 32] = (CT)(vol * scu);
-  lo[o + R::AL * 32] = (CT)(vol * fd * scl);
+  const double du = vol + dt1 * su, dl = vol + dt1 * sl, scu = rcp(du), scl = rcp(dl);
+  const double fd = 1. + dt1 * rcp(vol) * (.5 * sd);
+  o[R::AL * 32] = (CT)(vol * scu);
+  ol[R::AL * 32] = (CT)(vol * fd * scl);
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    up[o + (R::B + d) * 32] = (CT)(-(dt1 * ahi[d]) * scu);
-    lo[o + (R::B + d) * 32] = (CT)((dt1 * alo[d]) * scl);
-    up[o + (R::L + d) * 32] = (CT)mup[d];
-    lo[o + (R::L + d) * 32] = (CT)mlo[d];
+    o[(R::B + d) * 32] = (CT)(-(dt1 * ahi[d]) * scu);
+    ol[(R::B + d) * 32] = (CT)((dt1 * alo[d]) * scl);
   }
-  up[o + R::SP * 32] = (CT)((vol + dt1 * su) / (vol + dt1 * pu));
-  lo[o + R::SP * 32] = (CT)((vol + dt1 * sl) / (vol + dt1 * pl));
-  auto both = [&](int row, double val) {
-    up[o + row * 32] = (CT)val;
-    lo[o + row * 32] = (CT)val;
-  };
-  const double k0 = .5 * (c * c), ypro = 1. / ro;
+  o[R::SP * 32] = (CT)(du * rcp(vol + dt1 * pu));
+  ol[R::SP * 32] = (CT)(dl * rcp(vol + dt1 * pl));
+  auto both = [&](int row, double val) { o[row * 32] = ol[row * 32] = (CT)val; };
+  const double k0 = .5 * (c * c), ypro = rcp(ro);
   both(R::K0, k0);
   both(R::HR, .5 * ypro);
   if constexpr (NV == 7) {
     const double rk = LD(FF_RK, N);
-    const double ydrp = 1. / (1. + .667 * rk * ypro * LD(FF_DRDP, N));
+    const double ydrp = rcp(1. + .667 * rk * ypro * LD(FF_DRDP, N));
     const double h2 = ydrp * (.667 * rk * (ypro * ypro) * LD(FF_DRDH, N)) * ro;
     both(R::K4, ydrp * (ro * k0) - h2 * k0);
     both(R::Y, ydrp);
@@ -215,20 +227,39 @@ __global__ void __launch_bounds__(256) k_flow_coef(DevBlock b, ff_params p, Flow
     both(R::K4, ro * k0);
   }
 #undef LD
-#pragma unroll
-  for (int q = 0; q < NV; q++) up[o + q * 32] = (CT)b.a[FF_DRO + q][N];
+  b.a[FF_DTL][N] = dtl;
 }
 
-// The lower sweep's results from its records into DRO..DE(,DRK,DEPS).
+// The lower sweep's results from its records into DRO..DE(,DRK,DEPS): 32 cells
+// of a tile's 32 lines a thread block, record rows in, runs along the lines out
+// (128x64x64 cells, seven equations: 35 us with one thread a slot, 19 us).
+constexpr int FOP = 36;   // shared-memory pitch of a line: a record row's lanes fall on different banks
 template <typename CT, int NV>
 __global__ void __launch_bounds__(256) k_flow_out(DevBlock b, FlowGeom g, const CT* __restrict__ lo) {
   using R = FlowRec<NV>;
-  const size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int I, J, K;
-  if (n >= (size_t)g.ntiles * g.ns * 32 || !flow_cell(b, g, n, I, J, K)) return;
-  const size_t N = ix(b, I, J, K), o = (n >> 5) * (R::N * 32) + (n & 31);
+  extern __shared__ __align__(128) unsigned char flow_smem[];
+  CT* sv = reinterpret_cast<CT*>(flow_smem);   // [NV][32 lines][FOP]
+  const int nch = (b.imax + 31) / 32;
+  const int tile = blockIdx.x / nch, i0 = (blockIdx.x - tile * nch) * 32;
+  const int tk = tile / g.ntj, tj = tile - tk * g.ntj;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int NR = 32 + FTJ + FTK - 2;
+  for (int r = warp; r < NR; r += 8) {
+    const int i = r - lane % FTJ - lane / FTJ;
+    if (i < 0 || i >= 32 || i0 + i >= b.imax) continue;
+    const CT* row = lo + ((size_t)tile * g.ns + i0 + r) * (R::N * 32) + lane;
 #pragma unroll
-  for (int q = 0; q < NV; q++) b.a[FF_DRO + q][N] = (double)lo[o + q * 32];
+    for (int v = 0; v < NV; v++) sv[(v * 32 + lane) * FOP + i] = row[v * 32];
+  }
+  __syncthreads();
+  if (i0 + lane >= b.imax) return;
+  for (int l = warp; l < 32; l += 8) {
+    const int J = tj * FTJ + l % FTJ + 1, K = tk * FTK + l / FTJ + 1;
+    if (J > b.jmax || K > b.kmax) continue;
+    const size_t N = ix(b, i0 + lane + 1, J, K);
+#pragma unroll
+    for (int v = 0; v < NV; v++) b.a[FF_DRO + v][N] = (double)sv[(v * 32 + l) * FOP + lane];
+  }
 }
 
 // ---- edge words -------------------------------------------------------------

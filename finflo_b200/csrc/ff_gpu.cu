@@ -566,22 +566,39 @@ int flow_sweep(Ctx* c, BlockCtx* b, int upper) {
   return f32 ? flow_sweep_t<float, 5>(c, b, upper) : flow_sweep_t<double, 5>(c, b, upper);
 }
 
-template <typename CT, int NV>
-void flow_fill_t(Ctx* c, BlockCtx* b, int what) {
-  const int nb = nblk((long)b->fg.ntiles * b->fg.ns * 32, 256);
-  CT *up = (CT*)b->fup, *lo = (CT*)b->flo;
-  if (what == 0) k_flow_static<CT, NV><<<nb, 256, 0, c->stream>>>(b->db, b->fg, up, lo);
-  else if (what == 1) k_flow_coef<CT, NV><<<nb, 256, 0, c->stream>>>(b->db, b->prm, b->fg, up, lo, b->fticket);
-  else k_flow_out<CT, NV><<<nb, 256, 0, c->stream>>>(b->db, b->fg, lo);
-  c->nlaunch++;
+TimeConst time_const(const BlockCtx* b) {
+  const ff_params& p = b->prm;
+  return {1. / (b->level == 1 ? p.cfl : p.cfll), 1. / p.cdiff, p.pr / p.prt};
 }
 
-// what: 0 the records' face normals, 1 their coefficients and right-hand
-// side, 2 the results back into DRO..DE(,DRK,DEPS).
-void flow_fill(Ctx* c, BlockCtx* b, int what) {
+template <typename CT, int NV>
+int flow_fill_t(Ctx* c, BlockCtx* b, int what) {
+  CT *up = (CT*)b->fup, *lo = (CT*)b->flo;
+  constexpr int so = NV * 32 * FOP * (int)sizeof(CT);
+  static bool set[kMaxDev];
+  if (c->device < 0 || c->device >= kMaxDev) return fail(c, FF_ERR_ARG, "device id");
+  if (!set[c->device]) {
+    CK(cudaFuncSetAttribute(k_flow_out<CT, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, so));
+    set[c->device] = true;
+  }
+  if (what == 0)
+    k_flow_static<CT, NV><<<nblk((long)b->fg.ntiles * b->fg.ns * 32, 256), 256, 0, c->stream>>>(b->db, b->fg, up, lo);
+  else if (what == 1)
+    k_flow_coef<CT, NV><<<b->fg.ntiles * nblk(b->imax, 8), 256, 0, c->stream>>>(b->db, b->prm, time_const(b), b->fg, up,
+                                                                             lo, b->fticket);
+  else
+    k_flow_out<CT, NV><<<b->fg.ntiles * nblk(b->imax, 32), 256, so, c->stream>>>(b->db, b->fg, lo);
+  c->nlaunch++;
+  return 0;
+}
+
+// what: 0 the records' face normals, 1 the time step, the records'
+// coefficients and the right-hand side, 2 the results back into
+// DRO..DE(,DRK,DEPS).
+int flow_fill(Ctx* c, BlockCtx* b, int what) {
   const bool f32 = b->prm.lusgs_fp32 != 0;
-  if (b->prm.iturb >= 3) f32 ? flow_fill_t<float, 7>(c, b, what) : flow_fill_t<double, 7>(c, b, what);
-  else f32 ? flow_fill_t<float, 5>(c, b, what) : flow_fill_t<double, 5>(c, b, what);
+  if (b->prm.iturb >= 3) return f32 ? flow_fill_t<float, 7>(c, b, what) : flow_fill_t<double, 7>(c, b, what);
+  return f32 ? flow_fill_t<float, 5>(c, b, what) : flow_fill_t<double, 5>(c, b, what);
 }
 
 // ---- pipelined tile wavefront (k_lusgs_pipe) ------------------------------
@@ -1008,21 +1025,21 @@ int ddadi_sweeps(Ctx* c, BlockCtx* b, int only_dir) {
 // IMPS (imps3.f:6) in three parts: the time step and COPR before the
 // sweeps, the sweeps, and the increments out of the sweep layout (plus
 // DRO/CP for a standalone IMPS) after them.
-void st_imps_pre(Ctx* c, BlockCtx* b, int level) {
+void st_imps_pre(Ctx* c, BlockCtx* b) {
   int ncell = b->imax * b->jmax * b->kmax;
-  double cfl = level == 1 ? b->prm.cfl : b->prm.cfll;
+  const TimeConst tc = time_const(b);
   if (b->prm.iturb >= 3) {   // TIME3, then LOCDTK + IMSOKO + COPRKE
-    k_time3_copr<<<nblk(ncell, 128), 128, 0, c->stream>>>(b->db, b->prm, cfl, 1);
+    k_time3_copr<<<nblk(ncell, 128), 128, 0, c->stream>>>(b->db, b->prm, tc, 1);
     k_locdtk_imsoko_coprke<<<nblk(ncell, 128), 128, 0, c->stream>>>(b->db, b->prm);
     c->nlaunch += 2;
   } else {
-    k_time3_copr<<<nblk(ncell, 128), 128, 0, c->stream>>>(b->db, b->prm, cfl);
+    k_time3_copr<<<nblk(ncell, 128), 128, 0, c->stream>>>(b->db, b->prm, tc);
     c->nlaunch++;
   }
 }
 
 void st_sweep_out(Ctx* c, BlockCtx* b) {
-  if (b->use_lines) return flow_fill(c, b, 2);
+  if (b->use_lines) { flow_fill(c, b, 2); return; }
   int ncell = b->imax * b->jmax * b->kmax;
   if (b->prm.lusgs_fp32)
     k_sweep_out<float><<<nblk(ncell, 128), 128, 0, c->stream>>>(b->db, b->dwp32, b->prm.iturb >= 3 ? 7 : 5);
@@ -1041,7 +1058,8 @@ void st_imps_post(Ctx* c, BlockCtx* b, bool divide_cp) {
 }
 
 int st_imps(Ctx* c, BlockCtx* b, int level, bool divide_cp) {
-  st_imps_pre(c, b, level);
+  // the warp wavefront takes the time step and the conversion in k_flow_coef
+  if (b->prm.ddadi || !b->use_lines) st_imps_pre(c, b);
   bool fp32 = b->prm.lusgs_fp32 != 0;
   int rc;
   if (b->prm.ddadi) {

@@ -850,14 +850,14 @@ __global__ void k_resl2(DevBlock b, double* out) {
   }
 }
 
-// TIME3 base3c.f:79 + LOCDT imps3.f:784 + COPR imps3.f:891 (interior cells).
-// mode 1: TIME3 only (the two-equation path converts in k_locdtk_imsoko_coprke).
-__global__ void k_time3_copr(DevBlock b, ff_params p, double cfl, int mode = 0) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= b.imax * b.jmax * b.kmax) return;
-  int I = t % b.imax + 1, J = (t / b.imax) % b.jmax + 1, K = t / (b.imax * b.jmax) + 1;
+// What TIME3 divides by that is the same for all cells, inverted once.
+struct TimeConst {
+  double rcfl, rdiff, prt;   // 1 / CFL of the level, 1 / CDIFF, PR / PRT
+};
+
+// TIME3 base3c.f:79 (interior cell I, J, K at kk): the local time step.
+FF_DI double time3_cell(const DevBlock& b, const ff_params& p, const TimeConst& tc, int I, int J, int K, size_t kk) {
   const int IS = b.is, IL = b.il;
-  size_t kk = ix(b, I, J, K);
 #define LD(s, n) __ldg(b.a[s] + (n))
   double a1 = LD(FF_A1, kk), a1p = LD(FF_A1, kk + 1), a2 = LD(FF_A2, kk), a2p = LD(FF_A2, kk + IS);
   double a3 = LD(FF_A3, kk), a3p = LD(FF_A3, kk + IL);
@@ -867,7 +867,7 @@ __global__ void k_time3_copr(DevBlock b, ff_params p, double cfl, int mode = 0) 
   if (p.idi3 != 0 && K <= min(p.idi3, b.kmax)) zz = dmax(.5 * (a3 + a3p), zz);
   double ro = b.a[FF_RO][kk], u = b.a[FF_U][kk], v = b.a[FF_V][kk], w = b.a[FF_W][kk];
   double c = b.a[FF_C][kk], P = b.a[FF_P][kk];
-  double pvol = 1. / LD(FF_VOL, kk), ypro = 1. / (ro + 1.e-10);
+  double pvol = rcp(LD(FF_VOL, kk)), ypro = rcp(ro + 1.e-10);
   double a1k = .5 * (a1 + a1p), a2k = .5 * (a2 + a2p), a3k = .5 * (a3 + a3p);
   double ucii = .5 * (LD(FF_A1XA, kk) * a1 + LD(FF_A1XA, kk + 1) * a1p) * u
               + .5 * (LD(FF_A1YA, kk) * a1 + LD(FF_A1YA, kk + 1) * a1p) * v
@@ -879,30 +879,53 @@ __global__ void k_time3_copr(DevBlock b, ff_params p, double cfl, int mode = 0) 
               + .5 * (LD(FF_A3YA, kk) * a3 + LD(FF_A3YA, kk + IL) * a3p) * v
               + .5 * (LD(FF_A3ZA, kk) * a3 + LD(FF_A3ZA, kk + IL) * a3p) * w;
 #undef LD
-  double b1 = pvol * (fabs(ucii) + fabs(vcii) + fabs(wcii) + c * sqrt(a1k * a1k + a2k * a2k + a3k * a3k)) / cfl;
+  double ar, rar;
+  sqrt_rsq(dmax(a1k * a1k + a2k * a2k + a3k * a3k, 1.e-300), ar, rar);
+  double b1 = pvol * (fabs(ucii) + fabs(vcii) + fabs(wcii) + c * ar) * tc.rcfl;
   double rnum = zz * zz * (pvol * pvol) * ypro;
-  double tt = rnum * (b.a[FF_VIS][kk] + p.pr / p.prt * b.a[FF_VIST][kk]) / p.cdiff;
+  double tt = rnum * (b.a[FF_VIS][kk] + tc.prt * b.a[FF_VIST][kk]) * tc.rdiff;
   double b11 = dmax(b1, 2. * tt * p.pvisc);
-  double denlow = 1. + dmax(0., (p.frspre - 2. * P) / P);
+  double denlow = 1. + dmax(0., (p.frspre - 2. * P) * rcp(P));
   double denmax = 1. + dmax(0., (ro - 2. * p.frsden) * ypro) * 5.;
-  double dtl = 1. / (b11 * dmax(denlow, denmax));
+  double dtl = rcp(b11 * dmax(denlow, denmax));
   if (p.timel) dtl = dtl * p.dt / (1.5 * dtl + p.dt);   // TIMEL dual time step, base3c.f:206-215
-  if (mode == 1) { b.a[FF_DTL][kk] = dtl; return; }
-  // LOCDT + COPR
+  return dtl;
+}
+
+// LOCDT imps3.f:784 + COPR imps3.f:891: the residual of cell kk times the time
+// step in primitive increments.
+FF_DI void copr_cell(const DevBlock& b, double dtl, size_t kk, double x[5]) {
   double dri = dtl * b.a[FF_DRO][kk], dmi = dtl * b.a[FF_DM][kk], dni = dtl * b.a[FF_DN][kk];
   double dwi = dtl * b.a[FF_DW][kk], dre = dtl * b.a[FF_DE][kk];
-  double yp = 1. / ro, drodh = b.a[FF_DRDH][kk], drodp = b.a[FF_DRDP][kk], e = b.a[FF_E][kk];
+  double ro = b.a[FF_RO][kk], u = b.a[FF_U][kk], v = b.a[FF_V][kk], w = b.a[FF_W][kk], c = b.a[FF_C][kk];
+  double yp = rcp(ro), drodh = b.a[FF_DRDH][kk], drodp = b.a[FF_DRDP][kk];
   double beta = .5 * (u * u + v * v + w * w);
   double dkin = u * dmi + v * dni + w * dwi;
-  double hi = yp * (e + P);
+  double hi = yp * (b.a[FF_E][kk] + b.a[FF_P][kk]);
   double dei = dre - (hi - 2 * beta) * dri - dkin;
   double dpi = c * c * (dri - drodh * yp * dei);
+  x[0] = (dri - drodp * dpi) * rcp(drodh);
+  x[1] = yp * (-u * dri + dmi);
+  x[2] = yp * (-v * dri + dni);
+  x[3] = yp * (-w * dri + dwi);
+  x[4] = dpi;
+}
+
+// TIME3 + LOCDT + COPR in place (the sweeps that work on DRO..DE; the warp
+// wavefront takes them in k_flow_coef).  mode 1: TIME3 only (the two-equation
+// path converts in k_locdtk_imsoko_coprke).
+__global__ void k_time3_copr(DevBlock b, ff_params p, TimeConst tc, int mode = 0) {
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= b.imax * b.jmax * b.kmax) return;
+  int I = t % b.imax + 1, J = (t / b.imax) % b.jmax + 1, K = t / (b.imax * b.jmax) + 1;
+  const size_t kk = ix(b, I, J, K);
+  const double dtl = time3_cell(b, p, tc, I, J, K, kk);
+  if (mode == 1) { b.a[FF_DTL][kk] = dtl; return; }
+  double x[5];
+  copr_cell(b, dtl, kk, x);
   b.a[FF_DTL][kk] = dtl;
-  b.a[FF_DM][kk] = yp * (-u * dri + dmi);
-  b.a[FF_DN][kk] = yp * (-v * dri + dni);
-  b.a[FF_DW][kk] = yp * (-w * dri + dwi);
-  b.a[FF_DRO][kk] = (dri - drodp * dpi) / drodh;
-  b.a[FF_DE][kk] = dpi;
+#pragma unroll
+  for (int v = 0; v < 5; v++) b.a[FF_DRO + v][kk] = x[v];
 }
 
 // LU-SGS coefficients of one interior cell (PREDGS imps4.f:388-470 for

@@ -135,7 +135,7 @@ extern "C" int ff_imps_noalloc(int imax, int jmax, int kmax, const ff_params* pr
   int ncell = imax * jmax * kmax;
   ff_params p = *prm;
   double cfl = level == 1 ? p.cfl : p.cfll;
-  k_time3_copr<<<(ncell + 127) / 128, 128, 0, st>>>(db, p, cfl);
+  k_time3_copr<<<(ncell + 127) / 128, 128, 0, st>>>(db, p, {1. / cfl, 1. / p.cdiff, p.pr / p.prt});
   if (p.ddadi) {   // DDADI (LUSGS=0): k, i, j line sweeps, no scratch
     const int dirs[3] = {3, 1, 2};
     for (int d : dirs) {

@@ -752,13 +752,8 @@ constexpr ResForm RES_FORMS[RES_NFORM] = {{32, 4, 4, 512, 0}, {16, 8, 4, 512, 0}
                                           {32, 4, 4, 512, 1}, {16, 8, 4, 512, 1}, {8, 8, 8, 512, 1},
                                           {8, 4, 4, 512, 0},  {8, 8, 4, 256, 0},  {16, 4, 4, 256, 0}};
 
-// LOCDTK (DTURB=1) + IMSOKO + COPRKE, after TIME3 wrote DTL (interior).
-__global__ void k_locdtk_imsoko_coprke(DevBlock b, ff_params p) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= b.imax * b.jmax * b.kmax) return;
-  int I = t % b.imax + 1, J = (t / b.imax) % b.jmax + 1, K = t / (b.imax * b.jmax) + 1;
-  size_t i = ix(b, I, J, K);
-  double dtl = b.a[FF_DTL][i];
+// LOCDTK (DTURB=1) + IMSOKO + COPRKE of one cell with the time step of TIME3.
+FF_DI void coprke_cell(const DevBlock& b, const ff_params& p, double dtl, size_t i, double x[7]) {
   double dri = dtl * b.a[FF_DRO][i], dmi = dtl * b.a[FF_DM][i], dni = dtl * b.a[FF_DN][i];
   double dwi = dtl * b.a[FF_DW][i], dre = dtl * b.a[FF_DE][i];
   double drk = 1. * dtl * b.a[FF_DRK][i], deps = 1. * dtl * b.a[FF_DEPS][i];
@@ -769,29 +764,41 @@ __global__ void k_locdtk_imsoko_coprke(DevBlock b, ff_params p) {
   double emeanf = E - rk;
   double drkmax = dmax(ckmax * dmin(rk, fabs(0.1 * emeanf - 0.9 * rk)), eps);
   double dommax = ckmax * rom;
-  double prol = 1. / ro;
+  double prol = rcp(ro);
   double atprod = fabs(b.a[FF_PTUR][i]);
   double rnutrb = dmax(b.a[FF_EPS2][i] - 1.0, eps) * b.a[FF_VIS][i] * prol;
   double drkden = 1.0 + dtl * (atprod / drkmax + prol * SST_BSTAR * rom);
   double domden = 1.0 + dtl * (gamkom * atprod / (rnutrb * dommax) + 2. * SST_BETA1 * rom);
-  drk = drk / drkden;
-  deps = deps / domden;
+  drk = drk * rcp(drkden);
+  deps = deps * rcp(domden);
   // COPRKE imps3.f:1113
   double u = b.a[FF_U][i], v = b.a[FF_V][i], w = b.a[FF_W][i], c = b.a[FF_C][i], P = b.a[FF_P][i];
   double vel2 = u * u + v * v + w * w;
   double drodh = b.a[FF_DRDH][i], drodp = b.a[FF_DRDP][i];
-  double ypro = 1. / ro, rki = rk * ypro;
+  const double ypro = prol, rki = rk * ypro;
   double dkin = u * dmi + v * dni + w * dwi + drk;
   double hi = ypro * (E + P);
   double dei = dre - (hi - vel2 - rki) * dri - dkin;
   double dpi = c * c * (dri - drodh * ypro * dei);
-  b.a[FF_DM][i] = ypro * (-u * dri + dmi);
-  b.a[FF_DN][i] = ypro * (-v * dri + dni);
-  b.a[FF_DW][i] = ypro * (-w * dri + dwi);
-  b.a[FF_DRK][i] = ypro * (-rki * dri + drk);
-  b.a[FF_DEPS][i] = ypro * (-rom * ypro * dri + deps);
-  b.a[FF_DRO][i] = (dri - drodp * dpi) / drodh;
-  b.a[FF_DE][i] = dpi + .667 * drk;
+  x[0] = (dri - drodp * dpi) * rcp(drodh);
+  x[1] = ypro * (-u * dri + dmi);
+  x[2] = ypro * (-v * dri + dni);
+  x[3] = ypro * (-w * dri + dwi);
+  x[4] = dpi + .667 * drk;
+  x[5] = ypro * (-rki * dri + drk);
+  x[6] = ypro * (-rom * ypro * dri + deps);
+}
+
+// The same in place, after TIME3 wrote DTL (the sweeps that work on DRO..DEPS).
+__global__ void k_locdtk_imsoko_coprke(DevBlock b, ff_params p) {
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= b.imax * b.jmax * b.kmax) return;
+  int I = t % b.imax + 1, J = (t / b.imax) % b.jmax + 1, K = t / (b.imax * b.jmax) + 1;
+  const size_t i = ix(b, I, J, K);
+  double x[7];
+  coprke_cell(b, p, b.a[FF_DTL][i], i, x);
+#pragma unroll
+  for (int v = 0; v < 7; v++) b.a[FF_DRO + v][i] = x[v];
 }
 
 // SUBIN for SST: the k cap (RKMAX = FRSDEN*FRSVEL^2) and RKOLD/EPSOLD over
