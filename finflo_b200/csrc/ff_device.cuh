@@ -39,6 +39,13 @@ FF_DI double rcp(double x) {
   return fma(r, fma(e, e, e), r);
 }
 FF_DI float rcp(float x) { return __frcp_rn(x); }
+// a / b from r = rcp(b): the quotient corrected by its remainder (Markstein
+// 1990), as exact as a division where an ulp of the operand is amplified, as in
+// differences of neighbouring values.
+FF_DI double quot(double a, double b, double r) {
+  const double q = a * r;
+  return fma(fma(-q, b, a), r, q);
+}
 // sqrt(x) and 1/sqrt(x) for normal x > 0: one third-order (Householder) step
 // on the hardware's reciprocal root, then one correction of the root.
 // Largest errors 0.50 and 1.00 ulp.

@@ -346,7 +346,7 @@ FF_DI double grad_cell(const DevBlock& b, int level, int K, size_t L) {
     for (int side = 0; side < 2; side++) {
       size_t nb = side == 0 ? L - st[d] : L + st[d];
       const double dl = Dd[d][L];
-      double w1 = 2.0 * (dl * rcp(dl + Dd[d][nb])), w2 = 2.0 - w1;
+      const double dd = dl + Dd[d][nb], w1 = 2.0 * quot(dl, dd, rcp(dd)), w2 = 2.0 - w1;
       aa[2 * d + side] = side == 0 ? Ad[d][L] : Ad[d][L + st[d]];
 #pragma unroll
       for (int v = 0; v < 4; v++) q[v][2 * d + side] = w2 * F[v][L] + w1 * F[v][nb];

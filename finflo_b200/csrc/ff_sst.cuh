@@ -15,8 +15,8 @@ constexpr double SST_SIGRK1 = 0.85, SST_SIGOM1 = 0.5, SST_BETA2 = 0.0828, SST_SI
                  SST_SIGOM2 = 0.856;
 
 // ---- before the face pass -------------------------------------------------
-// The steps of TURBEQ and RESIKE before the face fluxes in two kernels (they
-// were eight): what bounds them is memory, and DERFUN, CROSKO and TEMDER of k
+// The steps of TURBEQ and RESIKE before the face fluxes in two kernels and one
+// of two arrays (they were eight): what bounds them is memory, and DERFUN, CROSKO and TEMDER of k
 // and omega each read the twelve face-metric arrays, the volume and the
 // thicknesses.  128x64x64 cells, one level-1 pass: k_grad 57.4, k_eps2ko 10.7,
 // k_crosko 27.8, k_rk_roundtrip 7.0, k_cdmax 6.7, k_fun1ko 11.2, k_prodke 11.0,
@@ -25,7 +25,11 @@ constexpr double SST_SIGRK1 = 0.85, SST_SIGOM1 = 0.5, SST_BETA2 = 0.0828, SST_SI
 // TEMDER the wall ghosts REFCEN fills in between.
 //
 // CROSKO divides RK and REPS by RO in place and multiplies them back, which
-// leaves them a rounding away from what they were; that step is not repeated.
+// leaves them a rounding away from what they were.  In cells of 2e-6 the
+// differences of neighbouring k amplify that rounding to 1e-12 of the k
+// residual, so it is kept (k_rk_roundtrip: the two passes read neighbours and
+// cannot do it in place).  For the same reason the weights and quotients of
+// the gradients are quot's.
 
 // EPS2KO turb3.f:7454 with STRAIN (res3c.f:6338) of one cell.
 FF_DI void eps2ko_cell(const DevBlock& b, const ff_params& p, size_t L, double st, double ro, double rk, double rom) {
@@ -98,6 +102,15 @@ __global__ void __launch_bounds__(128) k_pre_ke(DevBlock b, ff_params p, int lev
   if ((threadIdx.x & 31) == 0 && m > 0.) atomicMax(cdmax_bits, (unsigned long long)__double_as_longlong(m));
 }
 
+// CROSKO's RK = (RK / RO) RO over every cell, after its reads.
+__global__ void k_rk_roundtrip(DevBlock b) {
+  size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= (size_t)b.ntot) return;
+  const double ro = b.a[FF_RO][n], rk = b.a[FF_RK][n], re = b.a[FF_REPS][n], prol = 1. / ro;
+  b.a[FF_RK][n] = (rk * prol) * ro;
+  b.a[FF_REPS][n] = (re * prol) * ro;
+}
+
 // FUN1KO turb3.f:7385 of one interior cell.
 FF_DI void fun1ko_cell(const DevBlock& b, const ff_params& p, size_t L, double cdmin) {
   const double eps = 1.e-20;
@@ -153,7 +166,7 @@ __global__ void __launch_bounds__(128) k_temder_fun(DevBlock b, ff_params p, int
   const double *RO = b.a[FF_RO], *RK = b.a[FF_RK], *RE = b.a[FF_REPS];
 #define LD(s, n) __ldg(b.a[s] + (n))
   const int st[3] = {1, IS, IL};
-  const double r0 = rcp(RO[L]), k0 = RK[L] * r0, o0 = RE[L] * r0;
+  const double ro = RO[L], r0 = rcp(ro), k0 = quot(RK[L], ro, r0), o0 = quot(RE[L], ro, r0);
   double gk[3] = {0., 0., 0.}, go[3] = {0., 0., 0.};
 #pragma unroll
   for (int d = 2; d >= 0; d--) {
@@ -161,9 +174,10 @@ __global__ void __launch_bounds__(128) k_temder_fun(DevBlock b, ff_params p, int
 #pragma unroll
     for (int side = 1; side >= 0; side--) {
       const size_t nb = side ? L + st[d] : L - st[d], fc = side ? nb : L;
-      const double w1 = 2.0 * (dl * rcp(dl + LD(FF_D1 + d, nb))), w2 = 2.0 - w1, rn = rcp(RO[nb]);
+      const double dd = dl + LD(FF_D1 + d, nb), w1 = 2.0 * quot(dl, dd, rcp(dd)), w2 = 2.0 - w1;
+      const double rb = RO[nb], rn = rcp(rb);
       const double ar = side ? LD(FF_A1 + 4 * d, fc) : -LD(FF_A1 + 4 * d, fc);
-      const double kf = ar * (w2 * k0 + w1 * (RK[nb] * rn)), of = ar * (w2 * o0 + w1 * (RE[nb] * rn));
+      const double kf = ar * (w2 * k0 + w1 * quot(RK[nb], rb, rn)), of = ar * (w2 * o0 + w1 * quot(RE[nb], rb, rn));
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         const double nn = LD(FF_A1XA + 4 * d + c, fc);
