@@ -1076,10 +1076,22 @@ int st_imps(Ctx* c, BlockCtx* b, int level, bool divide_cp) {
   return 0;
 }
 
-int st_fin(Ctx* c, BlockCtx* b, int divide_cp) {
-  k_fin<<<nblk(b->ntot, 256), 256, 0, c->stream>>>(b->db, b->prm, c->d_dromax, divide_cp);
+int st_fin(Ctx* c, BlockCtx* b, int divide_cp, int state = 0) {
+  k_fin<<<nblk(b->ntot, 256), 256, 0, c->stream>>>(b->db, b->prm, c->d_dromax, divide_cp, state);
   c->nlaunch++;
   return 0;
+}
+
+// Transfer of the solution and the residual to the next coarser level;
+// forced: after adding the finer level's own forcing terms to its residual.
+void launch_transf(Ctx* c, BlockCtx* f, BlockCtx* cc, int forced) {
+  k_transf<<<nblk(cc->ntot, 128), 128, 0, c->stream>>>(f->db, cc->db, f->prm.iturb >= 3, forced);
+  c->nlaunch++;
+}
+
+void launch_prolong(Ctx* c, BlockCtx* cc, BlockCtx* f) {
+  k_prolong<<<nblk(f->ntot, 256), 256, 0, c->stream>>>(cc->db, f->db, f->prm);
+  c->nlaunch++;
 }
 
 int one_cycle(Ctx* c, BlockCtx* b, int icycle) {
@@ -1127,12 +1139,13 @@ int mg_body(Ctx* c, BlockCtx* b, int icycle, bool own, int part = 0) {
   if ((rc = st_residu(c, b, 1, icycle, 1, part))) return rc;
   if (part == 1) return 0;
   if ((rc = st_imps(c, b, 1, false))) return rc;
-  if ((rc = st_fin(c, b, 1))) return rc;
+  // the equation of state of a level's update comes with the update where a coarser level follows
+  if ((rc = st_fin(c, b, 1, b->coarse != nullptr))) return rc;
   std::vector<BlockCtx*> lv;
   for (BlockCtx* x = b; x; x = x->coarse) lv.push_back(x);
   for (size_t m = 1; m < lv.size(); m++) {
     BlockCtx *f = lv[m - 1], *cc = lv[m];
-    st_statim(c, f, 1);
+    launch_patch(c, f, k_reflec, 0);
     if ((rc = st_residu(c, f, (int)m, icycle, (int)m + 1))) return rc;
     if (m == 1) {   // RESL2 of the level-1 residual after the fine update
       if (own) {
@@ -1142,36 +1155,18 @@ int mg_body(Ctx* c, BlockCtx* b, int icycle, bool own, int part = 0) {
       int ncell = f->imax * f->jmax * f->kmax;
       k_resl2<<<min(nblk(ncell, 256), 4 * c->sm_count), 256, 0, c->stream>>>(f->db, c->d_resi);
       c->nlaunch++;
-    } else {
-      k_forcing<<<nblk(f->ntot, 256), 256, 0, c->stream>>>(f->db, 1, sst);
-      c->nlaunch++;
     }
-    long nc = (long)(cc->imax + 2) * (cc->jmax + 2) * (cc->kmax + 2);
-    k_transf<<<nblk(nc, 128), 128, 0, c->stream>>>(f->db, cc->db, sst);
-    c->nlaunch++;
-    k_transf_ring<<<nblk(cc->ntot, 256), 256, 0, c->stream>>>(cc->db, sst);
-    c->nlaunch++;
+    launch_transf(c, f, cc, m > 1);
     st_statim(c, cc, 1);
     if ((rc = st_residu(c, cc, (int)m + 1, icycle, (int)m + 1))) return rc;
-    k_forcing<<<nblk(cc->ntot, 256), 256, 0, c->stream>>>(cc->db, 0, sst);
+    k_forcing<<<nblk(cc->ntot, 256), 256, 0, c->stream>>>(cc->db, 2, sst);
     c->nlaunch++;
-    k_forcing<<<nblk(cc->ntot, 256), 256, 0, c->stream>>>(cc->db, 1, sst);
-    c->nlaunch++;
-    if ((rc = st_imps(c, cc, (int)m + 1, true))) return rc;
-    k_fin_coarse<<<nblk(cc->ntot, 256), 256, 0, c->stream>>>(cc->db, cc->prm, 1);
+    if ((rc = st_imps(c, cc, (int)m + 1, false))) return rc;
+    k_fin_coarse<<<nblk(cc->ntot, 256), 256, 0, c->stream>>>(cc->db, cc->prm, 2, cc->coarse != nullptr);
     c->nlaunch++;
   }
   for (size_t m = lv.size() - 1; m >= 1; m--) {
-    BlockCtx *f = lv[m - 1], *cc = lv[m];
-    int nf = f->imax * f->jmax * f->kmax;
-    k_interp<<<nblk(nf, 256), 256, 0, c->stream>>>(cc->db, f->db);
-    c->nlaunch++;
-    if (sst) {
-      k_intert<<<nblk(nf, 256), 256, 0, c->stream>>>(cc->db, f->db, f->prm);
-      c->nlaunch++;
-    }
-    k_fin_coarse<<<nblk(f->ntot, 256), 256, 0, c->stream>>>(f->db, f->prm, 0);
-    c->nlaunch++;
+    launch_prolong(c, lv[m], lv[m - 1]);
   }
   launch_patch(c, b, k_reflec, 0);
   return 0;
@@ -1346,7 +1341,7 @@ int mb_mg_body_ls(Ctx* c, int icycle) {
   if (rbatch && (rc = launch_residual_batch(c, tops, 1))) return rc;
   if (rbatch && (rc = fork_n(c, nb, [&](int n) { return st_residu(c, tops[n], 1, icycle, 1, 2); }))) return rc;
   if ((rc = ls_imps(c, tops, 1, false))) return rc;
-  if ((rc = fork_n(c, nb, [&](int n) { return st_fin(c, tops[n], 1); }))) return rc;
+  if ((rc = fork_n(c, nb, [&](int n) { return st_fin(c, tops[n], 1, tops[n]->coarse != nullptr); }))) return rc;
   std::vector<std::vector<BlockCtx*>> chain(nb);
   size_t nlev = 0;
   for (int n = 0; n < nb; n++) {
@@ -1361,30 +1356,23 @@ int mb_mg_body_ls(Ctx* c, int icycle) {
       BlockCtx *f = fs[n], *cc = cs[n];
       const int sst = f->prm.iturb >= 3;
       int r;
-      st_statim(c, f, 1);
+      launch_patch(c, f, k_reflec, 0);
       if ((r = st_residu(c, f, (int)m, icycle, (int)m + 1))) return r;
       if (m == 1) {   // RESL2 of the level-1 residual after the fine update
         int ncell = f->imax * f->jmax * f->kmax;
         k_resl2<<<min(nblk(ncell, 256), 4 * c->sm_count), 256, 0, c->stream>>>(f->db, c->d_resi);
         c->nlaunch++;
-      } else {
-        k_forcing<<<nblk(f->ntot, 256), 256, 0, c->stream>>>(f->db, 1, sst);
-        c->nlaunch++;
       }
-      long nc = (long)(cc->imax + 2) * (cc->jmax + 2) * (cc->kmax + 2);
-      k_transf<<<nblk(nc, 128), 128, 0, c->stream>>>(f->db, cc->db, sst);
-      k_transf_ring<<<nblk(cc->ntot, 256), 256, 0, c->stream>>>(cc->db, sst);
-      c->nlaunch += 2;
+      launch_transf(c, f, cc, m > 1);
       st_statim(c, cc, 1);
       if ((r = st_residu(c, cc, (int)m + 1, icycle, (int)m + 1))) return r;
-      k_forcing<<<nblk(cc->ntot, 256), 256, 0, c->stream>>>(cc->db, 0, sst);
-      k_forcing<<<nblk(cc->ntot, 256), 256, 0, c->stream>>>(cc->db, 1, sst);
-      c->nlaunch += 2;
+      k_forcing<<<nblk(cc->ntot, 256), 256, 0, c->stream>>>(cc->db, 2, sst);
+      c->nlaunch++;
       return 0;
     });
-    if (rc || (rc = ls_imps(c, cs, (int)m + 1, true))) return rc;
+    if (rc || (rc = ls_imps(c, cs, (int)m + 1, false))) return rc;
     rc = fork_n(c, (int)cs.size(), [&](int n) {
-      k_fin_coarse<<<nblk(cs[n]->ntot, 256), 256, 0, c->stream>>>(cs[n]->db, cs[n]->prm, 1);
+      k_fin_coarse<<<nblk(cs[n]->ntot, 256), 256, 0, c->stream>>>(cs[n]->db, cs[n]->prm, 2, cs[n]->coarse != nullptr);
       c->nlaunch++;
       return 0;
     });
@@ -1393,16 +1381,7 @@ int mb_mg_body_ls(Ctx* c, int icycle) {
   return fork_n(c, nb, [&](int n) {
     auto& lv = chain[n];
     for (size_t m = lv.size() - 1; m >= 1; m--) {
-      BlockCtx *f = lv[m - 1], *cc = lv[m];
-      int nf = f->imax * f->jmax * f->kmax;
-      k_interp<<<nblk(nf, 256), 256, 0, c->stream>>>(cc->db, f->db);
-      c->nlaunch++;
-      if (f->prm.iturb >= 3) {
-        k_intert<<<nblk(nf, 256), 256, 0, c->stream>>>(cc->db, f->db, f->prm);
-        c->nlaunch++;
-      }
-      k_fin_coarse<<<nblk(f->ntot, 256), 256, 0, c->stream>>>(f->db, f->prm, 0);
-      c->nlaunch++;
+      launch_prolong(c, lv[m], lv[m - 1]);
     }
     launch_patch(c, tops[n], k_reflec, 0);
     return 0;
@@ -1896,11 +1875,7 @@ int ff_transf(void* ctx, int fine, int coarse) {
   Ctx* c = (Ctx*)ctx;
   BlockCtx *f = getb(c, fine), *cc = getb(c, coarse);
   if (!f || !cc || f->coarse != cc) return fail(c, FF_ERR_ARG, "ff_transf: blocks are not linked levels");
-  const int sst = f->prm.iturb >= 3;
-  long nc = (long)(cc->imax + 2) * (cc->jmax + 2) * (cc->kmax + 2);
-  k_transf<<<nblk(nc, 128), 128, 0, c->stream>>>(f->db, cc->db, sst);
-  k_transf_ring<<<nblk(cc->ntot, 256), 256, 0, c->stream>>>(cc->db, sst);
-  c->nlaunch += 2;
+  launch_transf(c, f, cc, 0);
   CK(cudaGetLastError());
   return 0;
 }
@@ -1929,15 +1904,7 @@ int ff_interp(void* ctx, int coarse, int fine) {
   Ctx* c = (Ctx*)ctx;
   BlockCtx *f = getb(c, fine), *cc = getb(c, coarse);
   if (!f || !cc || f->coarse != cc) return fail(c, FF_ERR_ARG, "ff_interp: blocks are not linked levels");
-  int nf = f->imax * f->jmax * f->kmax;
-  k_interp<<<nblk(nf, 256), 256, 0, c->stream>>>(cc->db, f->db);
-  c->nlaunch++;
-  if (f->prm.iturb >= 3) {
-    k_intert<<<nblk(nf, 256), 256, 0, c->stream>>>(cc->db, f->db, f->prm);
-    c->nlaunch++;
-  }
-  k_fin_coarse<<<nblk(f->ntot, 256), 256, 0, c->stream>>>(f->db, f->prm, 0);
-  c->nlaunch++;
+  launch_prolong(c, cc, f);
   CK(cudaGetLastError());
   return 0;
 }
@@ -2112,7 +2079,7 @@ int ff_fin(void* ctx, int blk, double* dromax) {
   k_reset_acc<<<1, 32, 0, c->stream>>>(c->d_resi, c->d_dromax);
   c->nlaunch++;
   if (b->level > 1) {   // coarse level: FIN with the coarse limits (ns3c.f:1935-1990)
-    k_fin_coarse<<<nblk(b->ntot, 256), 256, 0, c->stream>>>(b->db, b->prm, 1);
+    k_fin_coarse<<<nblk(b->ntot, 256), 256, 0, c->stream>>>(b->db, b->prm, 1, 0);
     c->nlaunch++;
     if (dromax) *dromax = 0.0;
     CK(cudaGetLastError());

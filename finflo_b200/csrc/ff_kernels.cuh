@@ -73,17 +73,20 @@ FF_DI void state_store(const DevBlock& b, size_t n, const StateV& s) {
   b.a[FF_RN][n] = s.ro * s.v;
   b.a[FF_RW][n] = s.ro * s.w;
 }
+// one cell of the equation of state
+FF_DI void state_cell(const DevBlock& b, const ff_params& p, size_t n, bool interior) {
+  state_store(b, n, state_eval(b, p, n));
+  if (p.iturb < 3 && interior) {   // with two equations TURBEQ, not ADJUIN, sets EPS2 and VIST
+    b.a[FF_EPS2][n] = 1.0;
+    b.a[FF_VIST][n] = 0.0;
+  }
+}
 
 __global__ void k_state(DevBlock b, ff_params p) {
   size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= (size_t)b.ntot) return;
-  state_store(b, n, state_eval(b, p, n));
-  if (p.iturb >= 3) return;   // TURBEQ, not ADJUIN, sets EPS2 and VIST
   int i = (int)(n % b.is), j = (int)((n / b.is) % (b.jmax + 4)), k = (int)(n / b.il);
-  if (i >= 2 && i < b.imax + 2 && j >= 2 && j < b.jmax + 2 && k >= 2 && k < b.kmax + 2) {
-    b.a[FF_EPS2][n] = 1.0;
-    b.a[FF_VIST][n] = 0.0;
-  }
+  state_cell(b, p, n, i >= 2 && i < b.imax + 2 && j >= 2 && j < b.jmax + 2 && k >= 2 && k < b.kmax + 2);
 }
 
 // Face description of a patch: direction, sign, normal stride, interior layer.
@@ -1226,7 +1229,8 @@ __global__ void k_lusgs_sweep(DevBlock b, const CT* __restrict__ sw, CT* dwp, in
 // DRO/CP (imps3.f:483), FIN res3c.f:1077, the limits of CYCLES
 // (ns3c.f:1553-1596: UPLIM/LOLIM res3c.f:3314-3401, PDTOP, LOLIMP), the
 // interior *OLD copies of SUBIN and the max|dp| monitor (DROMXX, IDRXX=6).
-__global__ void k_fin(DevBlock b, ff_params p, unsigned long long* dromax_bits, int divide_cp) {
+// state: the equation of state of the new values in the same pass (where it comes next).
+__global__ void k_fin(DevBlock b, ff_params p, unsigned long long* dromax_bits, int divide_cp, int state) {
   size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   double amax = 0.;
   if (n < (size_t)b.ntot) {
@@ -1280,6 +1284,7 @@ __global__ void k_fin(DevBlock b, ff_params p, unsigned long long* dromax_bits, 
       b.a[FF_TOLD][n] = T; b.a[FF_UOLD][n] = U; b.a[FF_VOLD][n] = V; b.a[FF_WOLD][n] = W;
       b.a[FF_POLD][n] = PD;
     }
+    if (state) state_cell(b, p, n, interior);
   }
   for (int o = 16; o > 0; o >>= 1) amax = dmax(amax, __shfl_down_sync(0xffffffffu, amax, o));
   if ((threadIdx.x & 31) == 0 && amax > 0.) atomicMax(dromax_bits, (unsigned long long)__double_as_longlong(amax));
@@ -1306,12 +1311,25 @@ __global__ void k_fin_divide(DevBlock b, int sst) {
 // TRANSF multi.f:156: volume-weighted restriction of TEMP,U,V,W,PDIFF,EPS2,
 // VIST and of the residuals (into P2H) for coarse cells 0..MAX+1, and the
 // interior *OLD copies.
-__global__ void k_transf(DevBlock f, DevBlock c, int sst) {
-  int ni = c.imax + 2, nj = c.jmax + 2, nk = c.kmax + 2;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ni * nj * nk) return;
-  int I = t % ni, J = (t / ni) % nj, K = t / (ni * nj);
-  size_t N = ix(c, I, J, K);
+// One thread a coarse cell, ghosts included, the outer ring in the same pass:
+// a face ghost of the second layer takes what the first layer gets along the
+// face normal (computed again), other second-layer cells are not used on
+// coarse levels and left alone; the forcing terms of all ghosts are zero.
+// forced: ADDRES of the finer level (its DRO += P2H) first, as k_forcing does;
+// only the interior, whose 8 children are this thread's.
+__global__ void k_transf(DevBlock f, DevBlock c, int sst, int forced) {
+  size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= (size_t)c.ntot) return;
+  int I = (int)(n % c.is) - 1, J = (int)((n / c.is) % (c.jmax + 4)) - 1, K = (int)(n / c.il) - 1;
+  const bool interior = I >= 1 && I <= c.imax && J >= 1 && J <= c.jmax && K >= 1 && K <= c.kmax;
+  if (!interior) {
+#pragma unroll
+    for (int v = 0; v < 5; v++) c.a[FF_ROP2H + v][n] = 0.;
+    if (sst) { c.a[FF_RKP2H][n] = 0.; c.a[FF_EPP2H][n] = 0.; }
+    const int second = (I == -1 || I == c.imax + 2) + (J == -1 || J == c.jmax + 2) + (K == -1 || K == c.kmax + 2);
+    if (second > 1) return;
+    I = max(0, min(c.imax + 1, I)); J = max(0, min(c.jmax + 1, J)); K = max(0, min(c.kmax + 1, K));
+  }
   size_t ijk = ix(f, 2 * I - 1, 2 * J - 1, 2 * K - 1);
   size_t o[8] = {ijk + f.is + 1, ijk, ijk + 1, ijk + f.is,
                  ijk + f.is + 1 + f.il, ijk + f.il, ijk + 1 + f.il, ijk + f.is + f.il};
@@ -1319,62 +1337,48 @@ __global__ void k_transf(DevBlock f, DevBlock c, int sst) {
   double vv[8];
 #pragma unroll
   for (int q = 0; q < 8; q++) vv[q] = VOL[o[q]];
-  double pvol = 1. / c.a[FF_VOL][N];
-  const int vs[12] = {FF_TEMP, FF_U, FF_V, FF_W, FF_PDIFF, FF_EPS2, FF_VIST, FF_DRO, FF_DM, FF_DN, FF_DW, FF_DE};
-  const int ds[12] = {FF_TEMP, FF_U, FF_V, FF_W, FF_PDIFF, FF_EPS2, FF_VIST, FF_ROP2H, FF_RMP2H, FF_RNP2H, FF_RWP2H, FF_EP2H};
-#pragma unroll
-  for (int v = 0; v < 12; v++) {
-    const double* X = f.a[vs[v]];
+  double pvol = 1. / c.a[FF_VOL][ix(c, I, J, K)];
+  auto mean = [&](int slot) {
+    const double* X = f.a[slot];
     double s = 0.;
 #pragma unroll
     for (int q = 0; q < 8; q++) s += vv[q] * X[o[q]];
-    c.a[ds[v]][N] = s * pvol;
-  }
-  if (sst) {   // TRANKE multi.f:434: RK, REPS and DRK, DEPS into RKP2H, EPP2H
-    const int vk[4] = {FF_RK, FF_REPS, FF_DRK, FF_DEPS}, dk[4] = {FF_RK, FF_REPS, FF_RKP2H, FF_EPP2H};
+    return s * pvol;
+  };
+  const int vs[7] = {FF_TEMP, FF_U, FF_V, FF_W, FF_PDIFF, FF_EPS2, FF_VIST};
+  double x[9];
 #pragma unroll
-    for (int v = 0; v < 4; v++) {
-      const double* X = f.a[vk[v]];
-      double s = 0.;
+  for (int v = 0; v < 7; v++) x[v] = mean(vs[v]);
+  if (sst) { x[7] = mean(FF_RK); x[8] = mean(FF_REPS); }   // TRANKE multi.f:434
 #pragma unroll
-      for (int q = 0; q < 8; q++) s += vv[q] * X[o[q]];
-      c.a[dk[v]][N] = s * pvol;
+  for (int v = 0; v < 7; v++) c.a[vs[v]][n] = x[v];
+  if (sst) { c.a[FF_RK][n] = x[7]; c.a[FF_REPS][n] = x[8]; }
+  if (!interior) return;
+  c.a[FF_TOLD][n] = x[0];
+  c.a[FF_UOLD][n] = x[1];
+  c.a[FF_VOLD][n] = x[2];
+  c.a[FF_WOLD][n] = x[3];
+  c.a[FF_POLD][n] = x[4];
+  if (sst) { c.a[FF_RKOLD][n] = x[7]; c.a[FF_EPSOLD][n] = x[8]; }
+  const int rs[7] = {FF_DRO, FF_DM, FF_DN, FF_DW, FF_DE, FF_DRK, FF_DEPS};
+  const int ps[7] = {FF_ROP2H, FF_RMP2H, FF_RNP2H, FF_RWP2H, FF_EP2H, FF_RKP2H, FF_EPP2H};
+#pragma unroll
+  for (int v = 0; v < 7; v++) {
+    if (v >= 5 && !sst) break;
+    double r[8], s = 0.;
+#pragma unroll
+    for (int q = 0; q < 8; q++) r[q] = f.a[rs[v]][o[q]];
+    if (forced) {
+      double* P2 = f.a[ps[v]];
+#pragma unroll
+      for (int q = 0; q < 8; q++) r[q] = P2[o[q]] + r[q];
+#pragma unroll
+      for (int q = 0; q < 8; q++) f.a[rs[v]][o[q]] = r[q];
     }
-  }
-  if (I >= 1 && I <= c.imax && J >= 1 && J <= c.jmax && K >= 1 && K <= c.kmax) {
-    c.a[FF_TOLD][N] = c.a[FF_TEMP][N];
-    c.a[FF_UOLD][N] = c.a[FF_U][N];
-    c.a[FF_VOLD][N] = c.a[FF_V][N];
-    c.a[FF_WOLD][N] = c.a[FF_W][N];
-    c.a[FF_POLD][N] = c.a[FF_PDIFF][N];
-    if (sst) { c.a[FF_RKOLD][N] = c.a[FF_RK][N]; c.a[FF_EPSOLD][N] = c.a[FF_REPS][N]; }
-  }
-}
-
-// Coarse ghost rings of TRANSF (multi.f:250-432): P2H = 0 in both ghost
-// layers; the second ghost layer of each face copies the first one.
-__global__ void k_transf_ring(DevBlock c, int sst) {
-  size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= (size_t)c.ntot) return;
-  int i = (int)(n % c.is) - 1, j = (int)((n / c.is) % (c.jmax + 4)) - 1, k = (int)(n / c.il) - 1;
-  bool gi = i < 1 || i > c.imax, gj = j < 1 || j > c.jmax, gk = k < 1 || k > c.kmax;
-  if (!(gi || gj || gk)) return;
 #pragma unroll
-  for (int v = 0; v < 5; v++) c.a[FF_ROP2H + v][n] = 0.;
-  if (sst) { c.a[FF_RKP2H][n] = 0.; c.a[FF_EPP2H][n] = 0.; }
-  // second-layer face ghosts copy the first layer along the face normal
-  // (cells in the second layer of two directions are not used on coarse
-  // levels and are left alone)
-  int second = (i == -1 || i == c.imax + 2) + (j == -1 || j == c.jmax + 2) + (k == -1 || k == c.kmax + 2);
-  if (second != 1) return;
-  int src_off = 0;
-  if (i == -1) src_off = 1; else if (i == c.imax + 2) src_off = -1;
-  else if (j == -1) src_off = c.is; else if (j == c.jmax + 2) src_off = -c.is;
-  else if (k == -1) src_off = c.il; else if (k == c.kmax + 2) src_off = -c.il;
-  if (src_off == 0) return;
-  const int vs[9] = {FF_TEMP, FF_U, FF_V, FF_W, FF_PDIFF, FF_EPS2, FF_VIST, FF_RK, FF_REPS};
-  const int nv = sst ? 9 : 7;
-  for (int v = 0; v < nv; v++) c.a[vs[v]][n] = c.a[vs[v]][n + src_off];
+    for (int q = 0; q < 8; q++) s += vv[q] * r[q];
+    c.a[ps[v]][n] = s * pvol;
+  }
 }
 
 // FORCFU multi.f:1609 (mode 0: P2H -= R) and ADDRES multi.f:1686 (mode 1:
@@ -1384,21 +1388,21 @@ __global__ void k_forcing(DevBlock b, int mode, int sst) {
   if (n >= (size_t)b.ntot) return;
   const int ps[7] = {FF_ROP2H, FF_RMP2H, FF_RNP2H, FF_RWP2H, FF_EP2H, FF_RKP2H, FF_EPP2H};
   const int nv = sst ? 7 : 5;
-  for (int v = 0; v < nv; v++) {
+#pragma unroll
+  for (int v = 0; v < 7; v++) {
+    if (v >= nv) break;
     double* P2 = b.a[ps[v]];
     double* R = b.a[FF_DRO + v];
-    if (mode == 0) P2[n] = P2[n] - R[n];
-    else R[n] = P2[n] + R[n];
+    const double r = R[n];
+    double q = P2[n];
+    if (mode != 1) P2[n] = q = q - r;
+    if (mode != 0) R[n] = q + r;
   }
 }
 
 // INTERT multi.f:2051 -> INTERO 2007: damped injection of the coarse k and
 // omega corrections (CMGK, CMGEPS) into the fine interior.
-__global__ void k_intert(DevBlock c, DevBlock f, ff_params p) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= f.imax * f.jmax * f.kmax) return;
-  int I = t % f.imax + 1, J = (t / f.imax) % f.jmax + 1, K = t / (f.imax * f.jmax) + 1;
-  size_t N = ix(c, (I + 1) / 2, (J + 1) / 2, (K + 1) / 2), F = ix(f, I, J, K);
+FF_DI void intert_cell(const DevBlock& c, const DevBlock& f, const ff_params& p, size_t N, size_t F) {
 #pragma unroll
   for (int q = 0; q < 2; q++) {
     const double cc1 = q == 0 ? p.cmgk : p.cmgeps, cc2 = cc1 + 1.E-7;
@@ -1410,39 +1414,44 @@ __global__ void k_intert(DevBlock c, DevBlock f, ff_params p) {
 }
 
 // INTERP multi.f:1763: inject the coarse correction into the 8 children.
-__global__ void k_interp(DevBlock c, DevBlock f) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= f.imax * f.jmax * f.kmax) return;
-  int I = t % f.imax + 1, J = (t / f.imax) % f.jmax + 1, K = t / (f.imax * f.jmax) + 1;
-  size_t N = ix(c, (I + 1) / 2, (J + 1) / 2, (K + 1) / 2), F = ix(f, I, J, K);
-  double dp = c.a[FF_PDIFF][N] - c.a[FF_POLD][N];
-  f.a[FF_TEMP][F] = f.a[FF_TEMP][F] + (c.a[FF_TEMP][N] - c.a[FF_TOLD][N]);
-  f.a[FF_U][F] = f.a[FF_U][F] + (c.a[FF_U][N] - c.a[FF_UOLD][N]);
-  f.a[FF_V][F] = f.a[FF_V][F] + (c.a[FF_V][N] - c.a[FF_VOLD][N]);
-  f.a[FF_W][F] = f.a[FF_W][F] + (c.a[FF_W][N] - c.a[FF_WOLD][N]);
-  f.a[FF_P][F] = f.a[FF_P][F] + dp;
-  f.a[FF_PDIFF][F] = f.a[FF_PDIFF][F] + dp;
+FF_DI void interp_cell(const DevBlock& c, const DevBlock& f, size_t N, size_t F) {
+  const double dp = c.a[FF_PDIFF][N] - c.a[FF_POLD][N], dt = c.a[FF_TEMP][N] - c.a[FF_TOLD][N];
+  const double du = c.a[FF_U][N] - c.a[FF_UOLD][N], dv = c.a[FF_V][N] - c.a[FF_VOLD][N];
+  const double dw = c.a[FF_W][N] - c.a[FF_WOLD][N];
+  const double t = f.a[FF_TEMP][F], u = f.a[FF_U][F], v = f.a[FF_V][F], w = f.a[FF_W][F], P = f.a[FF_P][F],
+               pd = f.a[FF_PDIFF][F];
+  f.a[FF_TEMP][F] = t + dt;
+  f.a[FF_U][F] = u + du;
+  f.a[FF_V][F] = v + dv;
+  f.a[FF_W][F] = w + dw;
+  f.a[FF_P][F] = P + dp;
+  f.a[FF_PDIFF][F] = pd + dp;
 }
 
 // FIN on a coarse level (update = 1: UPLIM/LOLIM TEMP, LOLIMP, no PDTOP,
 // ns3c.f:1935-1990) and the limits after INTERP (update = 0, ns3c.f:2059-2125:
 // LOLIMP; the two-equation branch also limits TEMP, RK and REPS).
-__global__ void k_fin_coarse(DevBlock b, ff_params p, int update) {
-  size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= (size_t)b.ntot) return;
-  int i = (int)(n % b.is), j = (int)((n / b.is) % (b.jmax + 4)), k = (int)(n / b.il);
-  bool kin = k >= 2 && k < b.kmax + 2, jin = j >= 2 && j < b.jmax + 2;
-  bool interior = kin && jin && i >= 2 && i < b.imax + 2;
+// update 2: the division by CP (and RO) of k_fin_divide in the same pass.
+// state: see k_fin.
+FF_DI void fin_coarse_cell(const DevBlock& b, const ff_params& p, size_t n, bool kin, bool jin, bool interior, int update,
+                           int state) {
   const bool sst = p.iturb >= 3;
   double T = b.a[FF_TEMP][n];
   if (update && interior) {
-    T = b.a[FF_TOLD][n] + b.a[FF_DRO][n];
+    double dt = b.a[FF_DRO][n];
+    if (update == 2) b.a[FF_DRO][n] = dt = dt / b.a[FF_CP][n];
+    T = b.a[FF_TOLD][n] + dt;
     b.a[FF_U][n] = b.a[FF_UOLD][n] + b.a[FF_DM][n];
     b.a[FF_V][n] = b.a[FF_VOLD][n] + b.a[FF_DN][n];
     b.a[FF_W][n] = b.a[FF_WOLD][n] + b.a[FF_DW][n];
     b.a[FF_PDIFF][n] = b.a[FF_POLD][n] + b.a[FF_DE][n];
     if (sst) {   // FIN res3c.f:1190-1198
       double drk = b.a[FF_DRK][n], deps = b.a[FF_DEPS][n];
+      if (update == 2) {   // imps3.f:488-492
+        const double ro = b.a[FF_RO][n];
+        b.a[FF_DRK][n] = drk = drk * ro;
+        b.a[FF_DEPS][n] = deps = deps * ro;
+      }
       double rkold = b.a[FF_RKOLD][n], epold = b.a[FF_EPSOLD][n];
       b.a[FF_RK][n] = rkold + drk / (1. + fabs(drk) / (.45 * rkold));
       b.a[FF_REPS][n] = epold + deps / (1. + fabs(deps) / (.90 * epold));
@@ -1462,6 +1471,31 @@ __global__ void k_fin_coarse(DevBlock b, ff_params p, int update) {
   double prelim = dmin(0., P - 0.01 * p.frspre);
   b.a[FF_P][n] = P - prelim;
   b.a[FF_PDIFF][n] = b.a[FF_PDIFF][n] - prelim;
+  if (state) state_cell(b, p, n, interior);
+}
+
+__global__ void k_fin_coarse(DevBlock b, ff_params p, int update, int state) {
+  size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= (size_t)b.ntot) return;
+  int i = (int)(n % b.is), j = (int)((n / b.is) % (b.jmax + 4)), k = (int)(n / b.il);
+  bool kin = k >= 2 && k < b.kmax + 2, jin = j >= 2 && j < b.jmax + 2;
+  fin_coarse_cell(b, p, n, kin, jin, kin && jin && i >= 2 && i < b.imax + 2, update, state);
+}
+
+// INTERP, INTERT and the limits of k_fin_coarse over the finer level in one
+// pass: each cell depends on itself and its parent only.
+__global__ void k_prolong(DevBlock c, DevBlock f, ff_params p) {
+  size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= (size_t)f.ntot) return;
+  int I = (int)(n % f.is) - 1, J = (int)((n / f.is) % (f.jmax + 4)) - 1, K = (int)(n / f.il) - 1;
+  const bool kin = K >= 1 && K <= f.kmax, jin = J >= 1 && J <= f.jmax;
+  const bool interior = kin && jin && I >= 1 && I <= f.imax;
+  if (interior) {
+    const size_t N = ix(c, (I + 1) / 2, (J + 1) / 2, (K + 1) / 2);
+    interp_cell(c, f, N, n);
+    if (p.iturb >= 3) intert_cell(c, f, p, N, n);
+  }
+  fin_coarse_cell(f, p, n, kin, jin, interior, 0, 0);
 }
 
 // CONNEC ns3c.f:8605 (EXPTOT/IMPVO2 gluebm.f:6819/6964) for aligned 1:1
