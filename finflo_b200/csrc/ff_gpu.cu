@@ -27,6 +27,7 @@ struct BlockCtx {
   size_t slot_stride = 0;
   ff_patch* d_patch = nullptr;
   std::vector<ff_patch> h_patch;
+  bool patch_own = false;       // no cell is a ghost, or the source of one, of two patches (patches_own)
   ff_params prm{};
   // LU-SGS, warp wavefront (the default sweep): the records of the upper and
   // the lower sweep, the edge words between tiles and the tile counters, in
@@ -162,20 +163,52 @@ int launch_patch(Ctx* c, BlockCtx* b, void (*kern)(DevBlock, ff_params, int), in
 int st_statim(Ctx* c, BlockCtx* b, int npass = 2) {
   k_state<<<nblk(b->ntot, 256), 256, 0, c->stream>>>(b->db, b->prm);
   c->nlaunch++;
-  launch_patch(c, b, k_reflec, 0);
-  if (npass > 1) launch_patch(c, b, k_reflec, 1);
+  launch_patch(c, b, k_reflec, npass > 1 && b->patch_own ? 2 : 0);
+  if (npass > 1 && !b->patch_own) launch_patch(c, b, k_reflec, 1);
   return 0;
 }
 
-int st_boundi(Ctx* c, BlockCtx* b) {
-  k_refcor<<<nblk(refcor_threads(b->imax, b->jmax, b->kmax), 128), 128, 0, c->stream>>>(b->db);
+// Whether the ghost cells of a block's patches are each written by one thread
+// from cells that no patch writes: ranges inside the faces, no two patches of
+// a face overlapping, at least two cells between opposite faces.  REFLEC's two
+// passes and REFCOR with MIR then need no launch between them (ten cycles of
+// 16x8x8 cells 832 -> 812 us; elsewhere the passes keep their order).
+bool patches_own(const BlockCtx* b) {
+  const int mx[3] = {b->imax, b->jmax, b->kmax};
+  if (b->kmax < 2 || b->imax < 2 || b->jmax < 2) return false;
+  for (size_t n = 0; n < b->h_patch.size(); n++) {
+    const ff_patch& p = b->h_patch[n];
+    if (p.iface < 1 || p.iface > 6) return false;
+    const int d = (p.iface - 1) % 3, m1 = d == 0 ? mx[1] : mx[0], m2 = d == 2 ? mx[1] : mx[2];
+    if (p.r1a < 1 || p.r1b > m1 || p.r2a < 1 || p.r2b > m2) return false;
+    for (size_t q = 0; q < n; q++) {
+      const ff_patch& o = b->h_patch[q];
+      if (o.iface == p.iface && o.r1a <= p.r1b && p.r1a <= o.r1b && o.r2a <= p.r2b && p.r2a <= o.r2b) return false;
+    }
+  }
+  return true;
+}
+
+// REFCOR and MIR.
+void launch_refcor_mir(Ctx* c, BlockCtx* b) {
+  const int nr = nblk(refcor_threads(b->imax, b->jmax, b->kmax), 128);
+  int maxn = 1;
+  for (auto& p : b->h_patch) maxn = max(maxn, (p.r1b - p.r1a + 1) * (p.r2b - p.r2a + 1));
+  if (b->patch_own) {
+    k_refcor_mir<<<dim3(max(nr, nblk(maxn, 128)), b->npatch + 1), 128, 0, c->stream>>>(b->db, b->npatch);
+    c->nlaunch++;
+    return;
+  }
+  k_refcor<<<nr, 128, 0, c->stream>>>(b->db);
   c->nlaunch++;
   if (b->npatch) {
-    int maxn = 1;
-    for (auto& p : b->h_patch) maxn = max(maxn, (p.r1b - p.r1a + 1) * (p.r2b - p.r2a + 1));
     k_mir<<<dim3(nblk(maxn, 128), b->npatch), 128, 0, c->stream>>>(b->db);
     c->nlaunch++;
   }
+}
+
+int st_boundi(Ctx* c, BlockCtx* b) {
+  launch_refcor_mir(c, b);
   return st_statim(c, b);
 }
 
@@ -1394,14 +1427,7 @@ int mb_boundi(Ctx* c) {
   int nb = (int)c->tops.size(), rc;
   rc = fork_join(c, nb, [&](int n) {
     BlockCtx* b = c->tops[n];
-    k_refcor<<<nblk(refcor_threads(b->imax, b->jmax, b->kmax), 128), 128, 0, c->stream>>>(b->db);
-    c->nlaunch++;
-    if (b->npatch) {
-      int maxn = 1;
-      for (auto& p : b->h_patch) maxn = max(maxn, (p.r1b - p.r1a + 1) * (p.r2b - p.r2a + 1));
-      k_mir<<<dim3(nblk(maxn, 128), b->npatch), 128, 0, c->stream>>>(b->db);
-      c->nlaunch++;
-    }
+    launch_refcor_mir(c, b);
     return st_statim(c, b, 1);
   });
   if (rc) return rc;
@@ -1549,14 +1575,7 @@ int mb_phase(Ctx* c, int phase, int icycle) {
   if (phase == FF_PHASE_CYCLE_A || phase == FF_PHASE_BOUNDI_A) {
     rc = fork_join(c, nb, [&](int n) {
       BlockCtx* b = c->tops[n];
-      k_refcor<<<nblk(refcor_threads(b->imax, b->jmax, b->kmax), 128), 128, 0, c->stream>>>(b->db);
-      c->nlaunch++;
-      if (b->npatch) {
-        int maxn = 1;
-        for (auto& p : b->h_patch) maxn = max(maxn, (p.r1b - p.r1a + 1) * (p.r2b - p.r2a + 1));
-        k_mir<<<dim3(nblk(maxn, 128), b->npatch), 128, 0, c->stream>>>(b->db);
-        c->nlaunch++;
-      }
+      launch_refcor_mir(c, b);
       return st_statim(c, b, 1);
     });
     if (rc) return rc;
@@ -1711,6 +1730,7 @@ static int block_add(Ctx* c, int imax, int jmax, int kmax, int npatch, const ff_
       return fail(c, FF_ERR_ARG, "ff_block_add: bad patch range");
     }
   }
+  b->patch_own = patches_own(b);
   CK(cudaMalloc(&b->base, sizeof(double) * b->slot_stride * FF_NSLOTS));
   CK(cudaMemsetAsync(b->base, 0, sizeof(double) * b->slot_stride * FF_NSLOTS, c->stream));
   if (npatch) {

@@ -127,8 +127,7 @@ FF_DI size_t face_cell(const DevBlock& b, const FaceG& f, int a, int c) {
 // REFLEC turb3.f:5294: solid walls (viscous, wall at rest) and the inlet
 // pressure extrapolation.  mode 0: REFLEC; mode 1: re-evaluate the equation of
 // state in the two ghost cells first (the second STATIM pass).
-__global__ void k_reflec(DevBlock b, ff_params p, int mode) {
-  FF_PATCH_LOOP(b)
+FF_DI void reflec_cell(const DevBlock& b, const ff_params& p, const ff_patch& pa, size_t L, int ls, int mode) {
   size_t LB = L - ls, LT = L + ls, LC = L - 2 * ls;
   bool wall = pa.ityp >= 7 && pa.ityp <= 10;
   if (!wall && pa.ityp != FF_BC_INL) return;
@@ -169,6 +168,14 @@ __global__ void k_reflec(DevBlock b, ff_params p, int mode) {
     b.a[FF_RK][LB] = -rk;
     b.a[FF_REPS][LB] = dmax(0., 2. * re - ret);
   }
+}
+
+// mode 2: both passes, for blocks whose patches touch no cell of one another
+// (BlockCtx::patch_own): a cell's two ghosts are then this thread's alone.
+__global__ void k_reflec(DevBlock b, ff_params p, int mode) {
+  FF_PATCH_LOOP(b)
+  if (mode != 1) reflec_cell(b, p, pa, L, ls, 0);
+  if (mode != 0) reflec_cell(b, p, pa, L, ls, 1);
 }
 
 // REFCEN turb3.f:5881: linear extrapolation into the first wall ghost.
@@ -267,7 +274,7 @@ __global__ void k_inlet_outlet(DevBlock b, ff_params p, int icycle) {
 }
 
 // MIR ns3c.f:9003 -> MIRROR gluebm.f:3911 for symmetry patches.
-__global__ void k_mir(DevBlock b) {
+FF_DI void mir_cells(const DevBlock& b) {
   FF_PATCH_LOOP(b)
   if (pa.ityp != FF_BC_MIR) return;
   (void)ls;
@@ -303,7 +310,7 @@ __global__ void k_mir(DevBlock b) {
 __host__ __device__ inline int refcor_threads(int imax, int jmax, int kmax) {
   return 16 * (imax + jmax + kmax + 12);
 }
-__global__ void k_refcor(DevBlock b) {
+FF_DI void refcor_cells(const DevBlock& b) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int mx[3] = {b.imax, b.jmax, b.kmax};
   int d = 0;
@@ -329,6 +336,16 @@ __global__ void k_refcor(DevBlock b) {
   for (int s = 0; s < 20; s++) x[s] = b.a[sl[s]][src];
 #pragma unroll
   for (int s = 0; s < 20; s++) b.a[sl[s]][n] = x[s];
+}
+
+__global__ void k_mir(DevBlock b) { mir_cells(b); }
+__global__ void k_refcor(DevBlock b) { refcor_cells(b); }
+// Both in one launch, for blocks whose patches touch no cell of one another:
+// MIR writes face ghosts and REFCOR edge and corner ghosts, both from interior
+// cells.  blockIdx.y past the patches: REFCOR.
+__global__ void k_refcor_mir(DevBlock b, int npatch) {
+  if ((int)blockIdx.y < npatch) mir_cells(b);
+  else refcor_cells(b);
 }
 
 // DERFUN turb3.f:2476 + TEMDER turb3.f:3456 (IDERI = 1) of one cell; returns STRAIN.
