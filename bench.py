@@ -51,12 +51,12 @@ WORKLOADS = {
 # ncu capture of the same workload (profiles/k_residual_fused_sstmg128x64x64_full.md:
 # 244.6 MB read + 25.4 MB written, 16x8x4-cell tiles).
 TRAFFIC = {"sst-mg": 270.0e6}
-# DRAM bytes (read + write) per cell of one FP64 line-wavefront LU-SGS sweep
-# (k_lusgs_lines<double,7,0>) in the multi-block cycle, from an ncu capture of
+# DRAM bytes (read + write) per cell of one FP64 LU-SGS sweep
+# (k_flow_sweep<double,7>) in the multi-block cycle, from an ncu capture of
 # the same eight-block case at 256x128x64 cells (profiles/
-# k_lusgs_lines_large8blk_256x128x64_dram.md); a launch's traffic scales with
-# its block's cells
-SWEEP_TRAFFIC_PER_CELL = 376.1
+# k_flow_sweep_8blk_256x128x64_dram.md); a launch's traffic scales with its
+# block's cells
+SWEEP_TRAFFIC_PER_CELL = 281.0
 
 
 def build_case(wl, nodes=None):
@@ -642,8 +642,8 @@ def run_large(args):
                    "parallelism": f"8 blocks per GPU, replicas x{ws}",
                    "l2": "state resident in HBM (~30 GB), per-cycle working set far above L2"},
         "gpu_launches": per_cycle * args.steps,
-        # the dominant kernel of the cycle (profiles/launches_large8blk_512x256x128.md):
-        # the LU-SGS line-wavefront sweep; one lower sweep of the largest block, timed alone
+        # one upper LU-SGS sweep of the largest block, timed alone (the residual, beside it, has the
+        # larger share of the cycle since the sweep became a wavefront of warps)
         "roofline": {"bound": "hbm", "kernel": "k_flow_sweep<double,7> (upper sweep, largest block)",
                      "achieved": achieved_sweep, "peak": peak, "peak_kind": pkind, "unit": "GB/s",
                      "frac": achieved_sweep / peak,

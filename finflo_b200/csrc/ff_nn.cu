@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(GTHREADS) k_gemm_rows(GemmArgs g) {
 // tensor core reads -- no transposed copies (two launches and 4 bytes of
 // traffic an element before the GEMM even began).  blockIdx.y takes 128 of the
 // N columns; each CTA a share of the rows, added with FP32 atomics.
-// 1,048,576 rows, N = K = 32: 375 us (two transposes, a split GEMM) -> 95 us.
+// 1,048,576 rows, N = K = 32: 375 us (two transposes, a split GEMM) -> 90 us.
 struct WgradArgs {
   const __nv_bfloat16 *X, *Y;
   int ldx, ldy, rows, N, K, per, kst, nst;   // per: rows of a CTA, a multiple of kst; kst: rows of a stage; nst: stages
