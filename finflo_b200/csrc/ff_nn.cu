@@ -679,8 +679,21 @@ __global__ void k_adam(float* w, const float* __restrict__ g, float* m, float* v
   }
 }
 
-int g_smem_set[64];   // dynamic shared memory granted to k_gemm_bf16, per device
-int g_rows_set[64], g_wgrad_set[64];   // and to k_gemm_rows, k_wgrad
+int g_smem_set[64], g_rows_set[64], g_wgrad_set[64];   // the kernels' shared memory is granted, per device
+
+// What a GEMM kernel with tiles of nt columns is launched with: its
+// tensor-memory columns, and its shared memory, at least `need` and so much
+// that the CTAs resident on one SM never ask for more than its 512 columns.
+struct GemmPlan {
+  int nt, ncol;
+  size_t smem;
+};
+GemmPlan gemm_plan(int nt, size_t need) {
+  int ncol = 32;
+  while (ncol < nt) ncol <<= 1;
+  const size_t least = ncol >= 256 ? 80 * 1024 : (ncol >= 128 ? 48 * 1024 : (ncol >= 64 ? 28 * 1024 : 0));
+  return {nt, ncol, need < least ? least : need};
+}
 
 inline int blocks_for(long n, int t) { return (int)min((n + t - 1) / t, (long)148 * 16); }
 
@@ -704,44 +717,39 @@ int ffnn_gemm(const void* A, int lda, const void* B, int ldb, int M, int N, int 
   GemmArgs g;
   g.A = (const __nv_bfloat16*)A; g.B = (const __nv_bfloat16*)B;
   g.lda = lda; g.ldb = ldb; g.M = M; g.N = N; g.K = K;
-  // columns of a CTA tile: as many as fit, but 32 where the tiles would leave SMs idle (a few rows: the K loop's
-  // loads are the whole time, 16 x 256 x 512 took 106 us in one CTA)
-  g.nt = N <= 256 ? (N + 15) / 16 * 16 : 256;
-  if ((long)((M + GM - 1) / GM) * ((N + g.nt - 1) / g.nt) < 74 && g.nt > 32) g.nt = 32;
   g.ksplit = ksplit;
   g.bias = bias; g.act = act; g.zf = zf; g.ldz = ldz; g.atomic = atomic;
   g.yb = (__nv_bfloat16*)yb; g.ldy = ldy;
-  // tensor-memory columns of a CTA; shared memory sized so that the CTAs
-  // resident on one SM never ask for more than its 512 columns
-  int ncol = 32;
-  while (ncol < g.nt) ncol <<= 1;
-  size_t smem = 2 * (size_t)(GM + g.nt) * GKT * 2 + 64;
-  const size_t floor_ = ncol >= 256 ? 80 * 1024 : (ncol >= 128 ? 48 * 1024 : (ncol >= 64 ? 28 * 1024 : 0));
-  if (smem < floor_) smem = floor_;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FFNN_ERR_CUDA;
+  const int wide = N <= 256 ? (N + 15) / 16 * 16 : 256;
   if (rows_ok) {
-    g.nt = (N + 15) / 16 * 16;
-    size_t sm = gemm_rows_smem(N, K);
-    if (sm < floor_) sm = floor_;
-    if (sm <= 200 * 1024) {
+    const GemmPlan p = gemm_plan(wide, gemm_rows_smem(N, K));
+    if (p.smem <= 200 * 1024) {   // 210 KB at N, K = 256: the kernel below
       if (!g_rows_set[dev]) {
         if (cudaFuncSetAttribute(k_gemm_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
           return FFNN_ERR_CUDA;
         g_rows_set[dev] = 1;
       }
-      const int per_sm = min(ncol >= 256 ? 2 : (ncol >= 128 ? 4 : 8), max(1, (int)(220 * 1024 / sm)));
-      k_gemm_rows<<<min((M + GM - 1) / GM, 148 * per_sm), GTHREADS, sm, (cudaStream_t)stream>>>(g);
+      g.nt = p.nt;
+      const int per_sm = min(p.ncol >= 256 ? 2 : (p.ncol >= 128 ? 4 : 8), max(1, (int)(220 * 1024 / p.smem)));
+      k_gemm_rows<<<min((M + GM - 1) / GM, 148 * per_sm), GTHREADS, p.smem, (cudaStream_t)stream>>>(g);
       return cudaGetLastError() == cudaSuccess ? 0 : FFNN_ERR_CUDA;
     }
   }
-  if (g_smem_set[dev] < (int)smem) {
+  // columns of a CTA tile: as many as fit, but 32 where the tiles would leave SMs idle (a few rows: the K loop's
+  // loads are the whole time, 16 x 256 x 512 took 106 us in one CTA)
+  const bool few = (long)((M + GM - 1) / GM) * ((N + wide - 1) / wide) < 74;
+  const int nt = few ? min(wide, 32) : wide;
+  const GemmPlan p = gemm_plan(nt, 2 * (size_t)(GM + nt) * GKT * 2 + 64);
+  if (!g_smem_set[dev]) {
     if (cudaFuncSetAttribute(k_gemm_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)
       return FFNN_ERR_CUDA;
-    g_smem_set[dev] = 100 * 1024;
+    g_smem_set[dev] = 1;
   }
+  g.nt = p.nt;
   dim3 grid((M + GM - 1) / GM, (N + g.nt - 1) / g.nt, (K + ksplit - 1) / ksplit);
-  k_gemm_bf16<<<grid, GTHREADS, smem, (cudaStream_t)stream>>>(g);
+  k_gemm_bf16<<<grid, GTHREADS, p.smem, (cudaStream_t)stream>>>(g);
   return cudaGetLastError() == cudaSuccess ? 0 : FFNN_ERR_CUDA;
 }
 
@@ -752,15 +760,11 @@ int ffnn_wgrad(const void* X, int ldx, const void* Y, int ldy, int rows, int N, 
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FFNN_ERR_CUDA;
   const int kt = (K + 15) / 16 * 16, mt = (N + GM - 1) / GM;
-  int ncol = 32;
-  while (ncol < kt) ncol <<= 1;
   WgradArgs g;
   g.X = (const __nv_bfloat16*)X; g.Y = (const __nv_bfloat16*)Y;
   g.ldx = ldx; g.ldy = ldy; g.rows = rows; g.N = N; g.K = K; g.G = G; g.ldg = ldg;
   wgrad_stage(g);
-  size_t sm = g.nst * (size_t)wgrad_stage_bytes(g.kst, kt) + 64;
-  const size_t floor_ = ncol >= 256 ? 80 * 1024 : (ncol >= 128 ? 48 * 1024 : (ncol >= 64 ? 28 * 1024 : 0));
-  if (sm < floor_) sm = floor_;
+  const size_t sm = gemm_plan(kt, g.nst * (size_t)wgrad_stage_bytes(g.kst, kt) + 64).smem;
   if (!g_wgrad_set[dev]) {
     if (cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, 120 * 1024) != cudaSuccess)
       return FFNN_ERR_CUDA;

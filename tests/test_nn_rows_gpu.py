@@ -43,6 +43,19 @@ def test_row_gemm(nn, M, N, K, act):
     nn.error()
 
 
+@pytest.mark.parametrize("M,N,K", [(4096, 256, 256), (4100, 228, 256), (4096, 224, 256), (9344, 256, 256), (9345, 256, 256)])
+def test_row_gemm_past_the_shared_memory_of_the_row_kernel(nn, M, N, K):
+    """B and one A tile of 256 x 256 take 210 KB, more than the row kernel is
+    given: the tile kernel runs, in 32 columns a CTA up to 73 row tiles (9344
+    rows), in 256 from there on.  224 columns are the row kernel's last."""
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    a, b = _bf(gen, M, K), _bf(gen, N, K)
+    z = torch.full((M, N), -7.0, device="cuda")
+    nn.gemm(a, b, zf=z)
+    _close(z, a.double() @ b.double().T, 1e-5)
+    nn.error()
+
+
 @pytest.mark.parametrize("rows,N,K", [(1, 8, 8), (16, 512, 256), (63, 32, 32), (64, 16, 32), (65, 256, 32), (1000, 136, 40),
                                       (100003, 32, 32)])
 def test_weight_gradient(nn, rows, N, K):
