@@ -39,8 +39,9 @@
 // CTA tiles are taken from a counter in the order of their anti-diagonals, so
 // a CTA only ever waits for tiles that other CTAs already hold: no
 // co-residency is needed and any number of blocks' sweeps may run side by
-// side.  Every wait is bounded; on time-out the error word is set and the
-// tile finishes without waiting.
+// side.  Every wait is bounded; on time-out the error word is set, the tile
+// finishes without waiting or starting copies, and waits once more, again
+// with a bound, for the copies it has in flight.
 //
 // The cells' data is stored in the order of use: per tile and step one
 // contiguous record of FlowRec<NV>::N rows of 32 values (a value of the 32
@@ -58,6 +59,8 @@ constexpr int FIO = 64;             // threads that fetch, and that publish, the
 constexpr int FTHREADS = FW * 32 + 2 * FIO;
 constexpr int FD = 6;               // ring slots: up to FD - 1 steps of record copies in flight
 constexpr int FPF = 2;              // steps between an edge request and its use
+constexpr int kFlowSpins = 1 << 22; // reads of a missing edge word before its wait gives up (seconds); records: 4 times
+constexpr long kFlowDrain = 1L << 24;   // tries of the last wait for a CTA's copies after a time-out
 constexpr int FHS = FW * 32 + (FBJ > FBK ? FBJ : FBK);   // products of one value: the CTA's lines + the incoming edge
 
 // Rows of a record.  Solve: x = AL * rhs + B1 * yi + B2 * yj + B3 * yk, the
@@ -304,7 +307,13 @@ FF_DI void flow_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar
 // fetch the incoming edge words and wait for the records, one step ahead; the
 // last FIO publish the outgoing edge words of the step before and start the
 // record copies.
-template <typename CT, int NV, bool UP>
+//
+// HASTE: the same kernel with no patience (ff_sweep_haste): the CTAs that take
+// an even ticket give up on their first record, every CTA on the first edge
+// word that is not there yet.  A template parameter, because the limit as an
+// argument cost the poll a register and the sweep 1 % (248x136x72 cells, seven
+// equations: 254 -> 257 us).
+template <typename CT, int NV, bool UP, bool HASTE>
 __global__ void __launch_bounds__(FTHREADS) k_flow_sweep(const CT* rec, CT* res, CT* edge, FlowGeom g, int imax,
                                                          int jmax, int kmax, int drop, unsigned* ticket, int* err) {
   using R = FlowRec<NV>;
@@ -316,11 +325,13 @@ __global__ void __launch_bounds__(FTHREADS) k_flow_sweep(const CT* rec, CT* res,
   CT* pk = pj + 2 * PB;                          // and for the k neighbours
   uint64_t* bars = reinterpret_cast<uint64_t*>(pk + 2 * PB);
   __shared__ int s_tile;
+  __shared__ volatile int s_stop;   // 1 + the step whose record did not come: no record is waited for or copied any more
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t bar0 = pipe_smem_u32(bars), ring0 = pipe_smem_u32(ring);
   // the next CTA tile, in the order of the anti-diagonals (the counter wraps to 0 after the last one)
   if (threadIdx.x == 0) {
     s_tile = (int)atomicInc(ticket, (unsigned)g.nb - 1u);
+    s_stop = 0;
     for (int q = 0; q < FD; q++) pipe_mbar_init(bar0 + 8 * q, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -449,7 +460,7 @@ __global__ void __launch_bounds__(FTHREADS) k_flow_sweep(const CT* rec, CT* res,
 #pragma unroll
       for (int q = 0; q < NQ; q++) miss = miss || (want(q, T) && flow_mark(x[q]));
       if (__any_sync(0xffffffffu, miss)) {
-        for (long it = 0; !dead; it++) {
+        for (int it = 0; !dead; it++) {
           miss = false;
 #pragma unroll
           for (int q = 0; q < NQ; q++)
@@ -458,8 +469,8 @@ __global__ void __launch_bounds__(FTHREADS) k_flow_sweep(const CT* rec, CT* res,
               miss = miss || flow_mark(x[q]);
             }
           if (!__any_sync(0xffffffffu, miss)) break;
-          if ((it & 255) == 255) {
-            int stop = it > (1L << 22);
+          if (HASTE || (it & 255) == 255) {
+            int stop = HASTE || it >= kFlowSpins;
             if (stop && lane == 0) atomicExch(err, 3);
             stop = stop || *((volatile int*)err) != 0;
             dead = __any_sync(0xffffffffu, stop);
@@ -479,10 +490,13 @@ __global__ void __launch_bounds__(FTHREADS) k_flow_sweep(const CT* rec, CT* res,
       for (int q = 0; q < NQ; q++)
         if (want(q, T)) x[q] = flow_ld(ep[q] + at);
     };
+    bool gone = io >= 32;   // one warp waits for the records, each lane up to its first time-out
     auto record = [&](int T) {
-      if (io >= 32 || T >= nbs) return;
-      for (long it = 0; !pipe_try_wait(bar0 + 8 * (T % FD), (uint32_t)((T / FD) & 1)); it++)
-        if (it > (1L << 24)) { atomicExch(err, 4); break; }
+      if (gone || T >= nbs) return;
+      for (long it = 0;; it++) {
+        if (it >= (HASTE && (s_tile & 1) == 0 ? 0 : 4L * kFlowSpins)) { atomicExch(err, 4); s_stop = T + 1; gone = true; break; }
+        if (pipe_try_wait(bar0 + 8 * (T % FD), (uint32_t)((T / FD) & 1))) break;
+      }
     };
     CT ew[FPF][NQ];
 #pragma unroll
@@ -511,20 +525,21 @@ __global__ void __launch_bounds__(FTHREADS) k_flow_sweep(const CT* rec, CT* res,
 
   // ---- outgoing edge words, record copies ----
   const int po = io - FIO;
-  auto copy = [&](int T) {   // the records of CTA step T, one lane a warp tile
+  int last = -1;             // the last step whose copies were started
+  auto copy = [&](int T, int stop) {   // the records of CTA step T, one lane a warp tile
     if (po >= 32 || T >= nbs) return;
     int off = 0;
     const int wt = po < FW ? wtile(po, off) : -1;
-    const bool act = wt >= 0 && (unsigned)(T - off) < (unsigned)ns;
+    const bool act = !stop && wt >= 0 && (unsigned)(T - off) < (unsigned)ns;
     const unsigned n = __popc(__ballot_sync(0xffffffffu, act));
     const uint32_t bar = bar0 + 8 * (T % FD);
-    if (po == 0) flow_expect(bar, n * RB);
+    if (po == 0 && (n || !stop)) { flow_expect(bar, n * RB); last = T; }
     __syncwarp();
     if (act)
       flow_bulk(ring0 + ((T % FD) * FW + po) * RB, rec + ((size_t)wt * ns + (UP ? ns - 1 - (T - off) : T - off)) * ROW, RB,
                 bar);
   };
-  for (int T = 0; T < FD; T++) copy(T);
+  for (int T = 0; T < FD; T++) copy(T, 0);
   CT* ep[NQ];          // the word of step 0
   int eoff[NQ];        // there while 0 <= T - eoff < imax (NEVER: no downstream tile, no line)
   const CT* es[NQ];    // its place in buffer 0
@@ -552,10 +567,14 @@ __global__ void __launch_bounds__(FTHREADS) k_flow_sweep(const CT* rec, CT* res,
   __syncthreads();
   for (int T = 0; T < nbs; T++) {
     if (T > 0) {
+      const int stop = s_stop;
       publish(T - 1);
-      copy(T - 1 + FD);
+      copy(T - 1 + FD, stop);
     }
     __syncthreads();
   }
   publish(nbs - 1);
+  if (po == 0 && s_stop)   // copies that nobody waited for must land before the CTA leaves
+    for (int T = s_stop - 1; T <= last; T++)
+      for (long it = 0; it < kFlowDrain && !pipe_try_wait(bar0 + 8 * (T % FD), (uint32_t)((T / FD) & 1)); it++) {}
 }

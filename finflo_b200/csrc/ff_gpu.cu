@@ -110,6 +110,7 @@ struct Ctx {
   bool halo_pack = false, halo_unpack = false;
   double *halo_send = nullptr, *halo_recv = nullptr;
   cudaGraphExec_t phase_graph[2] = {nullptr, nullptr};
+  bool haste = false;                   // the warp wavefront gives up at once (ff_sweep_haste)
   // scratch of the set-up calls (synchronous, so one buffer serves them all)
   void* setup = nullptr;
   size_t setup_bytes = 0;
@@ -571,33 +572,39 @@ constexpr int kMaxDev = 64;
 
 // ---- warp wavefront (k_flow_sweep) ------------------------------------------
 // One sweep: one CTA per tile of 8 x 8 lines.
-template <typename CT, int NV>
+template <typename CT, int NV, bool HASTE>
 int flow_sweep_t(Ctx* c, BlockCtx* b, int upper) {
   constexpr int sm = (int)flow_smem_bytes(NV, sizeof(CT));
   static bool set[kMaxDev];
   if (c->device < 0 || c->device >= kMaxDev) return fail(c, FF_ERR_ARG, "device id");
+  auto ku = k_flow_sweep<CT, NV, true, HASTE>, kl = k_flow_sweep<CT, NV, false, HASTE>;
   if (!set[c->device]) {
-    CK(cudaFuncSetAttribute(k_flow_sweep<CT, NV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-    CK(cudaFuncSetAttribute(k_flow_sweep<CT, NV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    CK(cudaFuncSetAttribute(ku, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    CK(cudaFuncSetAttribute(kl, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
     set[c->device] = true;
   }
   CT *up = (CT*)b->fup, *lo = (CT*)b->flo, *ed = (CT*)b->fedge;
   // PREDGS drops the i+1 coupling of row JMAX unless predgs_full asks for
   // it; PRKEGS does not drop it
   if (upper)
-    k_flow_sweep<CT, NV, true><<<b->fg.nb, FTHREADS, sm, c->stream>>>(up, lo, ed, b->fg, b->imax, b->jmax, b->kmax,
-                                                                    !b->prm.predgs_full, b->fticket, c->d_err);
+    ku<<<b->fg.nb, FTHREADS, sm, c->stream>>>(up, lo, ed, b->fg, b->imax, b->jmax, b->kmax, !b->prm.predgs_full,
+                                             b->fticket, c->d_err);
   else
-    k_flow_sweep<CT, NV, false><<<b->fg.nb, FTHREADS, sm, c->stream>>>(lo, lo, ed, b->fg, b->imax, b->jmax, b->kmax, 0,
-                                                                     b->fticket + 1, c->d_err);
+    kl<<<b->fg.nb, FTHREADS, sm, c->stream>>>(lo, lo, ed, b->fg, b->imax, b->jmax, b->kmax, 0, b->fticket + 1, c->d_err);
   c->nlaunch++;
   return 0;
 }
 
-int flow_sweep(Ctx* c, BlockCtx* b, int upper) {
+template <bool HASTE>
+int flow_sweep_h(Ctx* c, BlockCtx* b, int upper) {
   const bool f32 = b->prm.lusgs_fp32 != 0;
-  if (b->prm.iturb >= 3) return f32 ? flow_sweep_t<float, 7>(c, b, upper) : flow_sweep_t<double, 7>(c, b, upper);
-  return f32 ? flow_sweep_t<float, 5>(c, b, upper) : flow_sweep_t<double, 5>(c, b, upper);
+  if (b->prm.iturb >= 3)
+    return f32 ? flow_sweep_t<float, 7, HASTE>(c, b, upper) : flow_sweep_t<double, 7, HASTE>(c, b, upper);
+  return f32 ? flow_sweep_t<float, 5, HASTE>(c, b, upper) : flow_sweep_t<double, 5, HASTE>(c, b, upper);
+}
+
+int flow_sweep(Ctx* c, BlockCtx* b, int upper) {
+  return c->haste ? flow_sweep_h<true>(c, b, upper) : flow_sweep_h<false>(c, b, upper);
 }
 
 TimeConst time_const(const BlockCtx* b) {
@@ -795,16 +802,22 @@ void fill_static(Ctx* c) {
     if (!b->prm.ddadi) sweep_static(c, b, b->prm.lusgs_fp32 != 0);
 }
 
+// Every captured cycle and phase of the context.
+void drop_graphs(Ctx* c) {
+  auto drop1 = [](cudaGraphExec_t& g) {
+    if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+  };
+  for (auto* x : c->blocks) drop1(x->graph);
+  for (auto& g : c->phase_graph) drop1(g);
+  drop1(c->mb_graph);
+}
+
 // The metrics of a block changed: its sweep layouts' static part is stale,
 // and so is every captured graph that skipped refilling it.
 void metrics_changed(Ctx* c, BlockCtx* b) {
   b->sw_static = 0;
   b->flow_static = 0;
-  for (auto* x : c->blocks)
-    if (x->graph) { cudaGraphExecDestroy(x->graph); x->graph = nullptr; }
-  for (auto& g : c->phase_graph)
-    if (g) { cudaGraphExecDestroy(g); g = nullptr; }
-  if (c->mb_graph) { cudaGraphExecDestroy(c->mb_graph); c->mb_graph = nullptr; }
+  drop_graphs(c);
 }
 
 // Sweep data of one sweep in the sweep layout (and, for upper = 1, the
@@ -1852,6 +1865,14 @@ int ff_synchronize(void* ctx) {
       }
     return fail(c, FF_ERR_TIMEOUT, "LU-SGS sweep: a bounded wait timed out");
   }
+  return 0;
+}
+
+int ff_sweep_haste(void* ctx, int on) {
+  Ctx* c = (Ctx*)ctx;
+  if (!c) return FF_ERR_ARG;
+  c->haste = on != 0;
+  drop_graphs(c);   // captured cycles hold the other kernel
   return 0;
 }
 

@@ -77,6 +77,7 @@ def lib():
         L.ff_stream.restype = vp
         L.ff_stream.argtypes = [vp]
         L.ff_synchronize.argtypes = [vp]
+        L.ff_sweep_haste.argtypes = [vp, ci]
         for n in ("ff_statim", "ff_boundi"):
             getattr(L, n).argtypes = [vp, ci]
         L.ff_residu.argtypes = [vp, ci, ci, ci]
@@ -199,6 +200,10 @@ class GpuSolver:
 
     def sync(self):
         self._check(self.L.ff_synchronize(self.ctx))
+
+    def sweep_haste(self, on: bool):
+        """Whether the line wavefront's waits give up at once (a time-out on purpose)."""
+        self._check(self.L.ff_sweep_haste(self.ctx, int(on)))
 
     # ---- stages (reference routine names) -------------------------------
     def statim(self, bid=0):

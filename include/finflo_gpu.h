@@ -67,7 +67,14 @@ int ff_host_register(void *ctx, void *host, size_t bytes);
 int ff_host_unregister(void *ctx, void *host);
 void *ff_device_ptr(void *ctx, int blk, int slot);
 void *ff_stream(void *ctx);
+/* Waits for the context's work; FF_ERR_TIMEOUT if a bounded wait of a sweep
+ * gave up since the last call: the increments of that sweep and what followed
+ * from them are then undefined, and the context is ready for a new state. */
 int ff_synchronize(void *ctx);
+/* on = 1: the waits of the line wavefront (LU-SGS) give up at once instead of
+ * after seconds, so that a sweep runs into the time-out that ff_synchronize
+ * reports; on = 0 (the default): as usual.  For tests of a host's handling. */
+int ff_sweep_haste(void *ctx, int on);
 
 /* Stages (drop-in replacements of the reference routines listed above). */
 int ff_statim(void *ctx, int blk);
