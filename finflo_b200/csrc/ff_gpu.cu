@@ -1645,13 +1645,13 @@ int ff_create(void** out, int device) {
   CK(cudaSetDevice(device));
   CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   CK(cudaMalloc(&c->d_bar, 2 * sizeof(unsigned)));
-  CK(cudaMemset(c->d_bar, 0, 2 * sizeof(unsigned)));
+  CK(cudaMemsetAsync(c->d_bar, 0, 2 * sizeof(unsigned), c->stream));
   CK(cudaMalloc(&c->d_err, sizeof(int)));
-  CK(cudaMemset(c->d_err, 0, sizeof(int)));
+  CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
   CK(cudaMalloc(&c->d_resi, 16 * sizeof(double)));
   CK(cudaMalloc(&c->d_dromax, sizeof(unsigned long long)));
   CK(cudaMalloc(&c->d_hist_pos, sizeof(int)));
-  CK(cudaMemset(c->d_hist_pos, 0, sizeof(int)));
+  CK(cudaMemsetAsync(c->d_hist_pos, 0, sizeof(int), c->stream));
   CK(cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device));
   CK(cudaDeviceGetAttribute(&c->smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   {   // co-resident CTAs of the cooperative sweep per SM, per instantiation and CTA size
@@ -1855,14 +1855,17 @@ int ff_synchronize(void* ctx) {
   int err = 0;
   CK(cudaMemcpy(&err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (err) {
-    cudaMemset(c->d_err, 0, sizeof(int));
-    cudaMemset(c->d_bar, 0, 2 * sizeof(unsigned));
+    // on the context's stream and waited for: cudaMemset fills on the legacy
+    // stream, which the context's streams do not wait for
+    CK(cudaMemsetAsync(c->d_bar, 0, 2 * sizeof(unsigned), c->stream));
     for (auto* b : c->blocks)   // edge words of an unfinished warp wavefront
       if (b->fedge) {
         const size_t el = b->prm.lusgs_fp32 ? sizeof(float) : sizeof(double);
-        cudaMemset(b->fedge, 0xff, flow_edge_len(b->fg, b->prm.iturb >= 3 ? 7 : 5) * el);
-        cudaMemset(b->fticket, 0, 2 * sizeof(unsigned));
+        CK(cudaMemsetAsync(b->fedge, 0xff, flow_edge_len(b->fg, b->prm.iturb >= 3 ? 7 : 5) * el, c->stream));
+        CK(cudaMemsetAsync(b->fticket, 0, 2 * sizeof(unsigned), c->stream));
       }
+    CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
+    CK(cudaStreamSynchronize(c->stream));
     return fail(c, FF_ERR_TIMEOUT, "LU-SGS sweep: a bounded wait timed out");
   }
   return 0;

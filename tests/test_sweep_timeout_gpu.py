@@ -62,3 +62,33 @@ def test_a_captured_cycle_takes_the_switch(gpu_lib):
     g.start(bid)
     assert np.isfinite(g.cycles(2, bid, icycle0=2)).all()
     g.close()
+
+
+def test_sweeps_queued_right_after_a_time_out(gpu_lib):
+    """The edge words (5.8 MB here) hold their marks again before anything that
+    is queued after the call which reported the time-out: many sweeps, each
+    started as soon as that call returns, all give the increments of the first."""
+    bg, _, prm, _ = make_pair(101, 81, 61)
+    names = ["DRO", "DM", "DN", "DW", "DE"]
+    g = GpuSolver(0)
+    bid = g.add_block(bg, prm)
+    g.upload(bid)
+    g.start(bid)
+    g.statim(bid)
+    for _ in range(2):   # the second call finds the ghost cells as every later one does
+        g.residu(bid, 1, 1)
+    g.imps(bid, 1)
+    want = g.download(bid, names)
+    for _ in range(10):
+        g.residu(bid, 1, 1)
+        g.sweep_haste(True)
+        g.imps(bid, 1)
+        g.sweep_haste(False)
+        g.residu(bid, 1, 1)   # queued behind the sweep that times out
+        with pytest.raises(FinfloGpuError, match="timed out"):
+            g.sync()
+        g.imps(bid, 1)
+        got = g.download(bid, names)
+        for n in names:
+            np.testing.assert_array_equal(got[n], want[n])
+    g.close()
