@@ -25,13 +25,13 @@ FF_DI size_t ix(const DevBlock& b, int I, int J, int K) {
 }
 
 template <typename T> FF_DI T dmax(T a, T b) { return a > b ? a : b; }
-// 1/x for normal x away from the ends of the range: the hardware's
-// approximation and one step of the third-order Newton iteration (r (1 + e +
-// e^2), e = 1 - x r), without the general routine's range checks.  Largest
-// error over the exponents the fluxes meet, against 80-bit arithmetic: 0.506
-// ulp (__drcp_rn 0.50).  A face takes about twenty of these; with
-// __drcp_rn and the general square root the SST residual of a 128x64x64
-// block took 0.278 ms, now 0.218.
+// 1/x for normal x away from the ends of the range (1/0 and 1/inf are NaN; see
+// rcp_any): the hardware's approximation and one step of the third-order
+// Newton iteration (r (1 + e + e^2), e = 1 - x r), without the general
+// routine's range checks.  Largest error over the exponents the fluxes meet,
+// against 80-bit arithmetic: 0.506 ulp (__drcp_rn 0.50).  A face takes about
+// twenty of these; with __drcp_rn and the general square root the SST residual
+// of a 128x64x64 block took 0.278 ms, now 0.218.
 FF_DI double rcp(double x) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
@@ -39,6 +39,15 @@ FF_DI double rcp(double x) {
   return fma(r, fma(e, e, e), r);
 }
 FF_DI float rcp(float x) { return __frcp_rn(x); }
+// The same where x may be zero or infinite and the result is still wanted:
+// there the step's error e is not a number, and the approximation stands
+// (1/0 = inf, 1/inf = 0).
+FF_DI double rcp_any(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.);
+  return fabs(e) < 1. ? fma(r, fma(e, e, e), r) : r;
+}
 // a / b from r = rcp(b): the quotient corrected by its remainder (Markstein
 // 1990), as exact as a division where an ulp of the operand is amplified, as in
 // differences of neighbouring values.
@@ -210,7 +219,7 @@ FF_DI void roe_flux(const T q[5][4], T nx, T ny, T nz, T area, int intem, const 
   // CHAT^2 = 1 / (DRDHH / ROHAT + DRDPH) = -1 / (DRDHH DEDPH)
   T chat2 = (phat * (yproh * yproh) - dedrh) * rcp(dedph);
   T cmin = dmin(c_r, c_l), cmax = dmax(c_r, c_l);
-  chat2 = dmin(cmax * cmax, chat2);
+  chat2 = dmin(chat2, cmax * cmax);   // NaN where DEDPH is 0: the cells' bound
   chat2 = dmax(cmin * cmin, chat2);
   T chat, rchat;
   sqrt_rsq(chat2, chat, rchat);

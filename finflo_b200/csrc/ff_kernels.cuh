@@ -905,9 +905,9 @@ FF_DI double time3_cell(const DevBlock& b, const ff_params& p, const TimeConst& 
   double rnum = zz * zz * (pvol * pvol) * ypro;
   double tt = rnum * (b.a[FF_VIS][kk] + tc.prt * b.a[FF_VIST][kk]) * tc.rdiff;
   double b11 = dmax(b1, 2. * tt * p.pvisc);
-  double denlow = 1. + dmax(0., (p.frspre - 2. * P) * rcp(P));
+  double denlow = 1. + dmax(0., (p.frspre - 2. * P) * rcp_any(P));   // infinite for P = 0
   double denmax = 1. + dmax(0., (ro - 2. * p.frsden) * ypro) * 5.;
-  double dtl = rcp(b11 * dmax(denlow, denmax));
+  double dtl = rcp_any(b11 * dmax(denlow, denmax));
   if (p.timel) dtl = dtl * p.dt / (1.5 * dtl + p.dt);   // TIMEL dual time step, base3c.f:206-215
   return dtl;
 }

@@ -262,7 +262,7 @@ FF_DI void roe_flux_ke(const T q[7][4], T nx, T ny, T nz, T area, int intem, int
   // denominator is -DRDHH DEDPH
   T chat2 = ((phat * (yproh * yproh) - dedrh) + T(.6667) * rkhat * yproh * (dedph + yproh)) * rcp(dedph);
   T cmin = dmin(c_r, c_l), cmax = dmax(c_r, c_l);
-  chat2 = dmin(cmax * cmax, chat2);
+  chat2 = dmin(chat2, cmax * cmax);   // NaN where DEDPH is 0: the cells' bound
   chat2 = dmax(cmin * cmin, chat2);
   T chat, rchat;
   sqrt_rsq(chat2, chat, rchat);
@@ -783,8 +783,8 @@ FF_DI void coprke_cell(const DevBlock& b, const ff_params& p, double dtl, size_t
   double rnutrb = dmax(b.a[FF_EPS2][i] - 1.0, eps) * b.a[FF_VIS][i] * prol;
   double drkden = 1.0 + dtl * (atprod / drkmax + prol * SST_BSTAR * rom);
   double domden = 1.0 + dtl * (gamkom * atprod / (rnutrb * dommax) + 2. * SST_BETA1 * rom);
-  drk = drk * rcp(drkden);
-  deps = deps * rcp(domden);
+  drk = drk * rcp_any(drkden);   // infinite for a cell without k or omega
+  deps = deps * rcp_any(domden);
   // COPRKE imps3.f:1113
   double u = b.a[FF_U][i], v = b.a[FF_V][i], w = b.a[FF_W][i], c = b.a[FF_C][i], P = b.a[FF_P][i];
   double vel2 = u * u + v * v + w * w;
