@@ -252,51 +252,51 @@ bool res_fused() {
 }
 
 template <int NV, int NT, int I_, int J_, int K_, bool ST = false, typename FT = double, bool ALT = false>
-void launch_residual_fused_s(cudaStream_t st, const BlockCtx* b, int level) {
+void launch_residual_fused_s(cudaStream_t st, const BlockCtx* b, int level, int keep) {
   dim3 g(nblk(b->imax, I_), nblk(b->jmax, J_), nblk(b->kmax, K_));
   const size_t sm = residual_fused_smem(NV, I_, J_, K_, ST);
   cudaFuncSetAttribute(k_residual_fused<NV, NT, I_, J_, K_, ST, FT, ALT>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_residual_fused<NV, NT, I_, J_, K_, ST, FT, ALT><<<g, NT, sm, st>>>(b->db, b->prm, level);
+  k_residual_fused<NV, NT, I_, J_, K_, ST, FT, ALT><<<g, NT, sm, st>>>(b->db, b->prm, level, keep);
 }
 
 template <int NV, int NT>
-void launch_residual_fused_t(cudaStream_t st, dim3 g, const BlockCtx* b, int level) {
-  (void)g;
+void launch_residual_fused_t(cudaStream_t st, const BlockCtx* b, int level, int keep) {
   // the form the autotuner chose for this block (512 threads only): tile
   // shape, and the stencil staged in shared memory or not
   const int sh = NT == 512 ? b->res_shape : 0;
   // another IFLUX scheme, XXTRAA or JAMESON: the kernel with those variants
   // compiled in, in the default 32x4x4 unstaged form
-  if (residual_alt(b->prm, level)) return launch_residual_fused_s<NV, NT, 32, 4, 4, false, double, true>(st, b, level);
+  if (residual_alt(b->prm, level)) return launch_residual_fused_s<NV, NT, 32, 4, 4, false, double, true>(st, b, level, keep);
   // a coarse level's face fluxes in FP32 (unstaged tiles; Roe with XXTRAP)
   if (level > 1 && b->prm.res_fp32) {
-    if (NT == 512 && sh == 6) return launch_residual_fused_s<NV, NT, 8, 4, 4, false, float>(st, b, level);
-    if (sh % 3 == 1) return launch_residual_fused_s<NV, NT, 16, 8, 4, false, float>(st, b, level);
-    if (sh % 3 == 2) return launch_residual_fused_s<NV, NT, 8, 8, 8, false, float>(st, b, level);
-    return launch_residual_fused_s<NV, NT, 32, 4, 4, false, float>(st, b, level);
+    if (NT == 512 && sh == 6) return launch_residual_fused_s<NV, NT, 8, 4, 4, false, float>(st, b, level, keep);
+    if (sh % 3 == 1) return launch_residual_fused_s<NV, NT, 16, 8, 4, false, float>(st, b, level, keep);
+    if (sh % 3 == 2) return launch_residual_fused_s<NV, NT, 8, 8, 8, false, float>(st, b, level, keep);
+    return launch_residual_fused_s<NV, NT, 32, 4, 4, false, float>(st, b, level, keep);
   }
   if constexpr (NT == 512) {
-    if (sh == 3) return launch_residual_fused_s<NV, NT, 32, 4, 4, true>(st, b, level);
-    if (sh == 4) return launch_residual_fused_s<NV, NT, 16, 8, 4, true>(st, b, level);
-    if (sh == 5) return launch_residual_fused_s<NV, NT, 8, 8, 8, true>(st, b, level);
-    if (sh == 6) return launch_residual_fused_s<NV, NT, 8, 4, 4>(st, b, level);
-    if (sh == 7) return launch_residual_fused_s<NV, 256, 8, 8, 4>(st, b, level);
-    if (sh == 8) return launch_residual_fused_s<NV, 256, 16, 4, 4>(st, b, level);
+    if (sh == 3) return launch_residual_fused_s<NV, NT, 32, 4, 4, true>(st, b, level, keep);
+    if (sh == 4) return launch_residual_fused_s<NV, NT, 16, 8, 4, true>(st, b, level, keep);
+    if (sh == 5) return launch_residual_fused_s<NV, NT, 8, 8, 8, true>(st, b, level, keep);
+    if (sh == 6) return launch_residual_fused_s<NV, NT, 8, 4, 4>(st, b, level, keep);
+    if (sh == 7) return launch_residual_fused_s<NV, 256, 8, 8, 4>(st, b, level, keep);
+    if (sh == 8) return launch_residual_fused_s<NV, 256, 16, 4, 4>(st, b, level, keep);
   }
-  if (sh == 1) return launch_residual_fused_s<NV, NT, 16, 8, 4>(st, b, level);
-  if (sh == 2) return launch_residual_fused_s<NV, NT, 8, 8, 8>(st, b, level);
-  launch_residual_fused_s<NV, NT, 32, 4, 4>(st, b, level);
+  if (sh == 1) return launch_residual_fused_s<NV, NT, 16, 8, 4>(st, b, level, keep);
+  if (sh == 2) return launch_residual_fused_s<NV, NT, 8, 8, 8>(st, b, level, keep);
+  launch_residual_fused_s<NV, NT, 32, 4, 4>(st, b, level, keep);
 }
 
-void launch_residual(cudaStream_t st, const BlockCtx* b, int level) {
+// keep: the k and omega sources' arrays are not written (repeated launches on one state).
+void launch_residual(cudaStream_t st, const BlockCtx* b, int level, int keep = 0) {
   dim3 g(nblk(b->imax, TI), nblk(b->jmax, TJ), nblk(b->kmax, TK));
   const bool sst = b->prm.iturb >= 3;
   if (res_fused()) {
     switch (res_threads(sst)) {
-      case 128: sst ? launch_residual_fused_t<7, 128>(st, g, b, level) : launch_residual_fused_t<5, 128>(st, g, b, level); break;
-      case 512: sst ? launch_residual_fused_t<7, 512>(st, g, b, level) : launch_residual_fused_t<5, 512>(st, g, b, level); break;
-      default: sst ? launch_residual_fused_t<7, 256>(st, g, b, level) : launch_residual_fused_t<5, 256>(st, g, b, level);
+      case 128: sst ? launch_residual_fused_t<7, 128>(st, b, level, keep) : launch_residual_fused_t<5, 128>(st, b, level, keep); break;
+      case 512: sst ? launch_residual_fused_t<7, 512>(st, b, level, keep) : launch_residual_fused_t<5, 512>(st, b, level, keep); break;
+      default: sst ? launch_residual_fused_t<7, 256>(st, b, level, keep) : launch_residual_fused_t<5, 256>(st, b, level, keep);
     }
     return;
   }
@@ -942,9 +942,9 @@ int tune_residual(Ctx* c, BlockCtx* b) {
   for (int s = 0; s < RES_NFORM; s++) {
     if (RES_FORMS[s].staged) continue;
     b->res_shape = s;
-    launch_residual(c->stream, b, b->level);
+    launch_residual(c->stream, b, b->level, 1);
     CK(cudaEventRecord(c->ev0, c->stream));
-    for (int r = 0; r < 3; r++) launch_residual(c->stream, b, b->level);
+    for (int r = 0; r < 3; r++) launch_residual(c->stream, b, b->level, 1);
     CK(cudaEventRecord(c->ev1, c->stream));
     CK(cudaEventSynchronize(c->ev1));
     float ms = 0.f;
@@ -2400,7 +2400,7 @@ int ff_time_stage(void* ctx, int blk, int stage, int reps, float* ms) {
   CK(cudaEventRecord(c->ev0, c->stream));
   for (int r = 0; r < reps; r++) {
     if (stage == FF_STAGE_RESIDUAL) {
-      launch_residual(c->stream, b, 1);
+      launch_residual(c->stream, b, 1, 1);
       c->nlaunch++;
     } else if (stage == FF_STAGE_SWEEP) {   // LU-SGS: the lower sweep; DDADI: all three directions
       int rc = b->prm.ddadi ? ddadi_sweeps(c, b) : sweep(c, b, 1, b->prm.lusgs_fp32 != 0);

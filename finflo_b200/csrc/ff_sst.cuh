@@ -586,8 +586,10 @@ __global__ void __launch_bounds__(NT, RES_MIN_CTAS * 128 / NT) k_residual_sst(De
 }
 
 // SOURKO (KOVER=0, RANS, no rotation correction) of one interior cell: SRK and
-// SEPS, and what ADDSKE adds to the k and omega residuals.
-FF_DI void sourko_cell(const DevBlock& b, size_t L, double& srk, double& som) {
+// SEPS, and what ADDSKE adds to the k and omega residuals.  SEPS goes in as
+// CROSKO's cross diffusion and comes out as the omega source: with keep it and
+// SRK are left alone, for launches that are repeated on the same state.
+FF_DI void sourko_cell(const DevBlock& b, size_t L, double& srk, double& som, bool keep = false) {
   const double pbstar = 1.0 / SST_BSTAR, persbs = 1.0 / sqrt(SST_BSTAR), eps = 1.0E-10;
   double f1 = b.a[FF_FUN1][L], onemf1 = dmax(0.0, 1.0 - f1);
   double beta = f1 * SST_BETA1 + onemf1 * SST_BETA2;
@@ -601,6 +603,7 @@ FF_DI void sourko_cell(const DevBlock& b, size_t L, double& srk, double& som) {
   double omepro = gamkom * ro * pt / (rmutrb * rom);
   double omedis = 1.0 * beta * prol * rom;
   som = som + rom * (omepro - omedis);
+  if (keep) return;
   b.a[FF_SRK][L] = srk;
   b.a[FF_SEPS][L] = som;
 }
@@ -639,8 +642,8 @@ __global__ void k_sourko_addske(DevBlock b) {
 // FT = float: the face fluxes of a coarse level in FP32 (the cells' sums
 // of their faces and the result stay FP64).
 template <int NV, int NT, int TI_, int TJ_, int TK_, bool STAGE = false, typename FT = double, bool ALT = false>
-FF_DI void residual_tile(const DevBlock& b, const ff_params& p, int level, int i0, int j0, int k0,
-                         double* res_smem) {
+FF_DI void residual_tile(const DevBlock& b, const ff_params& p, int level, int i0, int j0, int k0, double* res_smem,
+                         bool keep) {
   constexpr int TI = TI_, TJ = TJ_, TK = TK_;
   constexpr int NFK = TI * TJ * (TK + 1), NFI = (TI + 1) * TJ * TK, NFJ = TI * (TJ + 1) * TK;
   constexpr int NFT = NFK + NFI + NFJ, NC = TI * TJ * TK;
@@ -694,7 +697,7 @@ FF_DI void residual_tile(const DevBlock& b, const ff_params& p, int level, int i
     const size_t n = ix(b, I, J, K);
     const double rv = rcp(__ldg(b.a[FF_VOL] + n));
     double src[2] = {0., 0.};
-    if constexpr (NV == 7) sourko_cell(b, n, src[0], src[1]);   // SOURKO + ADDSKE
+    if constexpr (NV == 7) sourko_cell(b, n, src[0], src[1], keep);   // SOURKO + ADDSKE
 #pragma unroll
     for (int v = 0; v < NV; v++) {
       double acc = 0. - (sF[v][fk0 + TI * TJ] - sF[v][fk0]);
@@ -706,13 +709,14 @@ FF_DI void residual_tile(const DevBlock& b, const ff_params& p, int level, int i
 }
 
 // ALT: the selectable variants compiled in (the other IFLUX schemes, XXTRAA,
-// JAMESON); the plain Roe/XXTRAP forms leave them out.
+// JAMESON); the plain Roe/XXTRAP forms leave them out.  keep: see sourko_cell.
 template <int NV, int NT, int TI_ = TI, int TJ_ = TJ, int TK_ = TK, bool STAGE = false, typename FT = double,
           bool ALT = false>
-__global__ void __launch_bounds__(NT, RES_MIN_CTAS * 128 / NT) k_residual_fused(DevBlock b, ff_params p, int level) {
+__global__ void __launch_bounds__(NT, RES_MIN_CTAS * 128 / NT) k_residual_fused(DevBlock b, ff_params p, int level,
+                                                                                         int keep) {
   extern __shared__ double res_smem[];
   residual_tile<NV, NT, TI_, TJ_, TK_, STAGE, FT, ALT>(b, p, level, blockIdx.x * TI_, blockIdx.y * TJ_,
-                                                       blockIdx.z * TK_, res_smem);
+                                                       blockIdx.z * TK_, res_smem, keep != 0);
 }
 
 // Whether a block's residual on `level` needs the selectable variants.
@@ -742,7 +746,7 @@ __global__ void __launch_bounds__(NT, RES_MIN_CTAS * 128 / NT)
   while (bi + 1 < rb.nblk && t >= rb.tile0[bi + 1]) bi++;
   const int l = t - rb.tile0[bi], nx = rb.ntx[bi], ny = rb.nty[bi];
   const int ti = l % nx, tj = (l / nx) % ny, tk = l / (nx * ny);
-  residual_tile<NV, NT, TI_, TJ_, TK_, STAGE>(rb.b[bi], rb.p[bi], level, ti * TI_, tj * TJ_, tk * TK_, res_smem);
+  residual_tile<NV, NT, TI_, TJ_, TK_, STAGE>(rb.b[bi], rb.p[bi], level, ti * TI_, tj * TJ_, tk * TK_, res_smem, false);
 }
 
 inline size_t residual_fused_smem(int nv, int ti = TI, int tj = TJ, int tk = TK, bool stage = false) {

@@ -254,6 +254,10 @@ int ff_sweep_times(void *ctx, int blk, float *ms3);
 int ff_residual_shape(void *ctx, int blk);
 int ff_lusgs_kind(void *ctx, int blk);
 int ff_time_cycles(void *ctx, int blk, int ncycles, float *ms);
+/* Mean time of one launch of a stage's main kernel on the current state
+ * (reps launches).  The stage's results are those of the last launch (the
+ * sweep's are undefined); everything else, the k and omega sources among it,
+ * stays as it was. */
 int ff_time_stage(void *ctx, int blk, int stage, int reps, float *ms);
 
 /* ---- Fortran call sites ------------------------------------------------

@@ -8,7 +8,7 @@ stencil halo at the block's ghost layers are covered."""
 import numpy as np
 import pytest
 
-from finflo_b200.gpu import GpuSolver
+from finflo_b200.gpu import FF_STAGE_RESIDUAL, GpuSolver
 from oracle.oracle import Oracle
 from tests.util import flux_scale, flux_scale_sst, interior, make_pair
 
@@ -61,3 +61,23 @@ def test_residual_forms_agree_and_match_oracle(gpu_lib, sst, monkeypatch):
             scale = np.abs(res[0][n]).max()
             np.testing.assert_allclose(res[f][n], res[0][n], rtol=1e-14, atol=1e-14 * scale,
                                        err_msg=f"form {f} {n}")
+
+
+def test_timing_leaves_the_sources_alone(gpu_lib):
+    """Repeated launches (ff_time_stage, the autotuner before the first cycle)
+    do not apply SOURKO to its own result: SEPS and SRK stay as the residual
+    left them."""
+    bg, _, prm, _ = make_pair(23, 14, 10, **SST)
+    g = GpuSolver(0)
+    bid = g.add_block(bg, prm)
+    g.upload(bid)
+    g.start(bid)
+    g.statim(bid)
+    g.residu(bid, 1, 1)
+    want = g.download(bid, ["SEPS", "SRK"])
+    g.time_stage(FF_STAGE_RESIDUAL, 5, bid)
+    g.cycles(0, bid, icycle0=2)      # no cycle: the forms are timed
+    got = g.download(bid, ["SEPS", "SRK"])
+    g.close()
+    for n in want:
+        np.testing.assert_array_equal(got[n], want[n])
