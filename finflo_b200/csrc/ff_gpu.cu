@@ -328,7 +328,7 @@ int st_residu_sst(Ctx* c, BlockCtx* b, int level, int m2, int icycle, int part =
   // TURBEQ's DERFUN (m2 = 1 on level 1) or RESIKE's (m2 >= 2) of this level, EPS2KO, CROSKO
   CK(cudaMemsetAsync(b->d_red, 0, sizeof(unsigned long long), c->stream));
   k_pre_ke<<<nblk(ng, 128), 128, 0, c->stream>>>(b->db, b->prm, level, level == 1 && m2 == 1, b->d_red);
-  k_rk_roundtrip<<<nblk(b->ntot, 256), 256, 0, c->stream>>>(b->db);
+  k_rk_roundtrip<<<nblk(b->ntot, 256), 256, 0, c->stream>>>(b->db, b->d_red);
   c->nlaunch += 2;
   if (b->npatch && level == 1) {
     int maxn = 1;

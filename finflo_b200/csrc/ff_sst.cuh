@@ -56,8 +56,9 @@ FF_DI void eps2ko_cell(const DevBlock& b, const ff_params& p, size_t L, double s
 
 // DERFUN + TEMDER of T on the level's range (grad_cell), and on the interior
 // cells EPS2KO (eps2 = 1) and CROSKO: the cross diffusion into SEPS and its
-// largest positive value (FUN1KO's CDMAX; non-negative doubles order like
-// their bit patterns) into cdmax_bits.
+// largest positive value (FUN1KO's CDMAX, with the ghost cells' of
+// k_rk_roundtrip; non-negative doubles order like their bit patterns) into
+// cdmax_bits.
 __global__ void __launch_bounds__(128) k_pre_ke(DevBlock b, ff_params p, int level, int eps2,
                                                 unsigned long long* cdmax_bits) {
   int lo = level == 1 ? 0 : 1, hi = level == 1 ? 1 : 0;
@@ -102,13 +103,22 @@ __global__ void __launch_bounds__(128) k_pre_ke(DevBlock b, ff_params p, int lev
   if ((threadIdx.x & 31) == 0 && m > 0.) atomicMax(cdmax_bits, (unsigned long long)__double_as_longlong(m));
 }
 
-// CROSKO's RK = (RK / RO) RO over every cell, after its reads.
-__global__ void k_rk_roundtrip(DevBlock b) {
+// CROSKO's RK = (RK / RO) RO over every cell, after its reads, and the ghost
+// cells' part of CDMAX: FUN1KO takes the largest cross diffusion of the storage
+// from cell (1,1,1) to the last interior one, in which rows and planes of ghost
+// cells lie (zero unless the host left something in SEPS).
+__global__ void k_rk_roundtrip(DevBlock b, unsigned long long* cdmax_bits) {
   size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= (size_t)b.ntot) return;
-  const double ro = b.a[FF_RO][n], rk = b.a[FF_RK][n], re = b.a[FF_REPS][n], prol = 1. / ro;
+  const unsigned r = (unsigned)n / (unsigned)b.is, i = (unsigned)n - r * b.is, k = r / (unsigned)(b.jmax + 4),
+                 j = r - k * (b.jmax + 4);
+  const bool interior = i - 2u < (unsigned)b.imax && j - 2u < (unsigned)b.jmax && k - 2u < (unsigned)b.kmax;
+  const bool between = !interior && n > ix(b, 1, 1, 1) && n < ix(b, b.imax, b.jmax, b.kmax);
+  const double ro = b.a[FF_RO][n], rk = b.a[FF_RK][n], re = b.a[FF_REPS][n], cd = between ? b.a[FF_SEPS][n] : 0.;
+  const double prol = 1. / ro;
   b.a[FF_RK][n] = (rk * prol) * ro;
   b.a[FF_REPS][n] = (re * prol) * ro;
+  if (cd > 0.) atomicMax(cdmax_bits, (unsigned long long)__double_as_longlong(cd));
 }
 
 // FUN1KO turb3.f:7385 of one interior cell.
