@@ -260,19 +260,28 @@ void launch_residual_fused_s(cudaStream_t st, const BlockCtx* b, int level, int 
   k_residual_fused<NV, NT, I_, J_, K_, ST, FT, ALT><<<g, NT, sm, st>>>(b->db, b->prm, level, keep);
 }
 
+// The residual form a block runs on a level: the chosen one where the level's
+// kernels have it.  The selectable variants have 32x4x4 only.  FP32 has the
+// unstaged 512-thread forms: a staged choice runs unstaged, and the two-CTA
+// forms, which pay by filling FP64's waits, become 32x4x4 (us, seven equations,
+// 32x4x4 / 16x8x4 / 8x8x8: 64x32x32 cells 56.3 / 58.0 / 62.1, 90x50x34 116.4 /
+// 116.1 / 121.3, 160x96x64 554.6 / 555.5 / 579.0, with the passes before).
+int res_form(const BlockCtx* b, int level) {
+  if (!res_fused() || res_threads(b->prm.iturb >= 3) != 512 || residual_alt(b->prm, level)) return 0;
+  if (level > 1 && b->prm.res_fp32) return b->res_shape == 6 ? 6 : (b->res_shape > 6 ? 0 : b->res_shape % 3);
+  return b->res_shape;
+}
+
 template <int NV, int NT>
 void launch_residual_fused_t(cudaStream_t st, const BlockCtx* b, int level, int keep) {
-  // the form the autotuner chose for this block (512 threads only): tile
-  // shape, and the stencil staged in shared memory or not
-  const int sh = NT == 512 ? b->res_shape : 0;
-  // another IFLUX scheme, XXTRAA or JAMESON: the kernel with those variants
-  // compiled in, in the default 32x4x4 unstaged form
+  const int sh = NT == 512 ? res_form(b, level) : 0;
+  // another IFLUX scheme, XXTRAA or JAMESON: the kernel with those variants compiled in
   if (residual_alt(b->prm, level)) return launch_residual_fused_s<NV, NT, 32, 4, 4, false, double, true>(st, b, level, keep);
-  // a coarse level's face fluxes in FP32 (unstaged tiles; Roe with XXTRAP)
+  // a coarse level's face fluxes in FP32 (Roe with XXTRAP)
   if (level > 1 && b->prm.res_fp32) {
     if (NT == 512 && sh == 6) return launch_residual_fused_s<NV, NT, 8, 4, 4, false, float>(st, b, level, keep);
-    if (sh % 3 == 1) return launch_residual_fused_s<NV, NT, 16, 8, 4, false, float>(st, b, level, keep);
-    if (sh % 3 == 2) return launch_residual_fused_s<NV, NT, 8, 8, 8, false, float>(st, b, level, keep);
+    if (sh == 1) return launch_residual_fused_s<NV, NT, 16, 8, 4, false, float>(st, b, level, keep);
+    if (sh == 2) return launch_residual_fused_s<NV, NT, 8, 8, 8, false, float>(st, b, level, keep);
     return launch_residual_fused_s<NV, NT, 32, 4, 4, false, float>(st, b, level, keep);
   }
   if constexpr (NT == 512) {
@@ -920,7 +929,7 @@ int tune_ddadi(Ctx* c, BlockCtx* b, const TuneKey& key) {
 // Residual form of a block: each unstaged one of RES_FORMS (the staged ones
 // were slower on every shape tried; FINFLO_RES_SHAPE still selects them) timed
 // on the block's own level (CUDA events, after one untimed launch), the
-// fastest kept; cached per device, block shape and equation count.
+// fastest kept; cached per device, block shape, equation count and precision.
 // FINFLO_RES_SHAPE (0..8) fixes it.
 std::map<TuneKey, int> g_res_cache;
 
@@ -930,8 +939,9 @@ int tune_residual(Ctx* c, BlockCtx* b) {
   const char* e = getenv("FINFLO_RES_SHAPE");
   const int env = e ? atoi(e) : -1;
   if (env >= 0 && env < RES_NFORM) { b->res_shape = env; return 0; }
-  if (!res_fused() || res_threads(b->prm.iturb >= 3) != 512) return 0;
-  const TuneKey key{c->device, b->imax, b->jmax, b->kmax, (b->prm.iturb >= 3 ? 7 : 5) + 10 * b->level, 0, 0};
+  if (!res_fused() || res_threads(b->prm.iturb >= 3) != 512 || residual_alt(b->prm, b->level)) return 0;
+  const TuneKey key{c->device, b->imax, b->jmax, b->kmax, (b->prm.iturb >= 3 ? 7 : 5) + 10 * b->level,
+                    b->level > 1 && b->prm.res_fp32, 0};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_res_cache.find(key);
@@ -940,8 +950,8 @@ int tune_residual(Ctx* c, BlockCtx* b) {
   float best = 1e30f;
   int pick = 0;
   for (int s = 0; s < RES_NFORM; s++) {
-    if (RES_FORMS[s].staged) continue;
     b->res_shape = s;
+    if (RES_FORMS[s].staged || res_form(b, b->level) != s) continue;   // not a form of this level's kernels
     launch_residual(c->stream, b, b->level, 1);
     CK(cudaEventRecord(c->ev0, c->stream));
     for (int r = 0; r < 3; r++) launch_residual(c->stream, b, b->level, 1);
@@ -1796,6 +1806,13 @@ int ff_block_params(void* ctx, int blk, const ff_params* prm) {
   bool fp_changed = (b->prm.lusgs_fp32 != 0) != (prm->lusgs_fp32 != 0);
   bool dd_changed = (b->prm.ddadi != 0) != (prm->ddadi != 0);
   if (dd_changed) b->tuned = 0;
+  auto res_kernel = [b](const ff_params& p) {   // equation count, variants, precision
+    return (p.iturb >= 3) + 2 * residual_alt(p, b->level) + 4 * (b->level > 1 && p.res_fp32);
+  };
+  if (res_kernel(b->prm) != res_kernel(*prm)) {   // another residual kernel: its form is chosen anew
+    b->tuned = b->res_tuned = 0;
+    b->res_shape = res_rule(c, b);
+  }
   b->prm = *prm;
   if (nv_changed || fp_changed || dd_changed) {   // the sweep's kernel and buffers
     int rc = pick_sweep(c, b);
@@ -2221,7 +2238,7 @@ int ff_lusgs_kind(void* ctx, int blk) {
 int ff_residual_shape(void* ctx, int blk) {
   BlockCtx* b = getb((Ctx*)ctx, blk);
   if (!b) return -FF_ERR_ARG;
-  return b->res_shape;
+  return res_form(b, b->level);
 }
 
 int ff_cycle_launches(void* ctx, int blk) {

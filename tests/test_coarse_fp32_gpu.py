@@ -47,6 +47,52 @@ def test_coarse_residual_in_fp32(gpu_lib, sst):
         assert 0.0 < err <= 2e-5, (n, err)   # FP32 rounding: not bitwise, not more
 
 
+# FINFLO_RES_SHAPE -> the form an FP32 level runs: it has no staged and no two-CTA forms
+FP32_FORM = ("32x4x4", "16x8x4", "8x8x8", "32x4x4", "16x8x4", "8x8x8", "8x4x4", "32x4x4", "32x4x4")
+
+
+@pytest.mark.parametrize("sst", [False, True])
+def test_fp32_forms(gpu_lib, sst, monkeypatch):
+    """Every form asked for gives the same FP32 residual to FP32 rounding, and
+    ff_residual_shape names the one that runs."""
+    out = []
+    for f, want in enumerate(FP32_FORM):
+        monkeypatch.setenv("FINFLO_RES_SHAPE", str(f))
+        levels, prms, fs = case.bump_case_mg(33, 17, 17, nlev=2, **(SST if sst else {}))
+        prms[1].res_fp32 = 1
+        g = GpuSolver(0)
+        bid = g.add_levels(levels, prms)
+        for q in range(2):
+            g.upload(bid + q)
+        g.start(bid)
+        g.cycles(1, bid, icycle0=1, use_graph=False)
+        assert g.residual_shape(bid + 1) == want
+        g.statim(bid + 1)
+        g.residu(bid + 1, 2, 1)
+        out.append(g.download(bid + 1, RES7 if sst else RES5))
+        g.close()
+    for o in out[1:]:
+        for n in o:
+            assert np.abs(o[n] - out[0][n]).max() <= 2e-5 * np.abs(out[0][n]).max(), n
+
+
+def test_form_without_timing_and_after_a_change(gpu_lib):
+    """The rule's two-CTA form is not an FP32 level's; a level that turns FP32,
+    or takes another flux scheme, has the form of its new kernels."""
+    levels, prms, fs = case.bump_case_mg(193, 129, 65, nlev=2)   # the coarse level has 768 tiles of 16x4x4
+    g = GpuSolver(0)
+    bid = g.add_levels(levels, prms)
+    assert g.residual_shape(bid + 1) == "16x4x4 x2"
+    prms[1].res_fp32 = 1
+    g.set_params(bid + 1, prms[1])
+    assert g.residual_shape(bid + 1) == "32x4x4"
+    prms[1].res_fp32 = 0
+    prms[1].xxtral = 1
+    g.set_params(bid + 1, prms[1])
+    assert g.residual_shape(bid + 1) == "32x4x4"
+    g.close()
+
+
 LAM = dict(amp=0.05, inter=1, cfl=2.0, cfll=2.0)
 LAM_CYC = 5000
 
