@@ -1,6 +1,7 @@
-"""Every residual form the autotuner chooses from -- tile shapes 32x4x4,
-16x8x4, 8x8x8 cells, each with the face stencils read from global memory
-or staged in shared memory -- gives the same residual to rounding (1e-14;
+"""Every residual form -- tile shapes 32x4x4, 16x8x4, 8x8x8 cells, each with
+the face stencils read from global memory or staged in shared memory, 8x4x4 in
+one round of 512 threads, and 8x8x4 and 16x4x4 of 256 threads, two CTAs an SM
+-- gives the same residual to rounding (1e-14;
 each kernel instantiation forms its own fused multiply-adds), and that
 residual matches the oracle's (1e-12 of max(|R|, S) per cell).  The
 block sizes are not multiples of the tiles, so partial tiles and the
@@ -30,7 +31,7 @@ def _residual(form, sst, dims, monkeypatch):
     g.start(bid)
     g.cycles(4, bid, icycle0=1, use_graph=False)     # the autotuner takes the fixed form
     assert g.residual_shape(bid) == ("32x4x4", "16x8x4", "8x8x8", "32x4x4 staged", "16x8x4 staged",
-                                     "8x8x8 staged")[form]
+                                     "8x8x8 staged", "8x4x4", "8x8x4 x2", "16x4x4 x2")[form]
     d = g.download(bid)
     for n, a in d.items():
         bc.arrays[n][:] = a
@@ -55,8 +56,8 @@ def _residual(form, sst, dims, monkeypatch):
 @pytest.mark.parametrize("sst", [False, True])
 def test_residual_forms_agree_and_match_oracle(gpu_lib, sst, monkeypatch):
     dims = (38, 20, 11)      # 37 x 19 x 10 cells
-    res = [_residual(f, sst, dims, monkeypatch) for f in range(6)]
-    for f in range(1, 6):
+    res = [_residual(f, sst, dims, monkeypatch) for f in range(9)]
+    for f in range(1, 9):
         for n in res[0]:   # rounding-level: each instantiation contracts its own multiply-adds
             scale = np.abs(res[0][n]).max()
             np.testing.assert_allclose(res[f][n], res[0][n], rtol=1e-14, atol=1e-14 * scale,
