@@ -2089,8 +2089,9 @@ int ff_wall_distance(void* ctx, int blk, const double* pts, int npts) {
   if (npts > 0) CK(setup_buf(c, np3 * sizeof(double) + (size_t)(ng + nsup) * sizeof(WdBox), &dp));
   WdBox *group = (WdBox*)(dp + np3), *super = group + ng;
   cudaError_t e = cudaSuccess;
-  if (npts > 0) {
-    e = cudaMemcpyAsync(dp, pts, np3 * sizeof(double), cudaMemcpyHostToDevice, c->stream);
+  const bool scattered = wd_scattered(pts, npts);
+  if (npts > 0) e = cudaMemcpyAsync(dp, pts, np3 * sizeof(double), cudaMemcpyHostToDevice, c->stream);
+  if (!wd_plain(b->ntot, npts, scattered)) {   // the finest level has the most cells
     k_wd_boxes<<<nsup, WD_C * WD_S, 0, c->stream>>>(dp, npts, group, super);
     c->nlaunch++;
   }
@@ -2098,7 +2099,9 @@ int ff_wall_distance(void* ctx, int blk, const double* pts, int npts) {
   // the interior cells again as the mean of their children (LUMP_DIST)
   BlockCtx* fine = nullptr;
   for (BlockCtx* x = b; x && e == cudaSuccess; fine = x, x = x->coarse) {
-    k_wall_distance<<<nblk((long)x->ntot, WD_THREADS), WD_THREADS, 0, c->stream>>>(x->db, dp, npts, group, super);
+    const int nb = nblk((long)x->ntot, WD_THREADS);
+    if (wd_plain(x->ntot, npts, scattered)) k_wall_distance_all<<<nb, WD_THREADS, 0, c->stream>>>(x->db, dp, npts);
+    else k_wall_distance<<<nb, WD_THREADS, 0, c->stream>>>(x->db, dp, npts, group, super);
     c->nlaunch++;
     if (fine) {
       k_lump_distw<<<nblk((long)x->imax * x->jmax * x->kmax, 256), 256, 0, c->stream>>>(fine->db, x->db);

@@ -360,11 +360,48 @@ __global__ void k_finish_metrics(DevBlock b, const double* __restrict__ raw, Raw
 // is passed over and the result is the same to the bit.  The walk is a warp's
 // (32 consecutive cells, nearly the same groups): a group is looked at when
 // any of the 32 needs it, its points read once for all.
-constexpr int WD_THREADS = 256, WD_C = 32, WD_S = 32;
+//
+// Few points, or points in no spatial order, are compared with every cell
+// (k_wall_distance_all): the walk's votes and box distances then cost more
+// than they save (wd_plain has the lines and the times).
+constexpr int WD_THREADS = 256, WD_C = 32, WD_S = 32, WD_TP = 512;
 
 struct WdBox {
   double lo[3], hi[3];
 };
+
+// Whether the points of neighbouring groups lie anywhere: more than two fifths
+// of the pairs of (at most 32) group boxes taken evenly from the list meet.
+inline bool wd_scattered(const double* p, int np) {
+  const int ng = np / WD_C, m = min(ng, 32);
+  WdBox s[32];
+  int meet = 0;
+  for (int q = 0; q < m; q++) {
+    const double* x = p + (size_t)((long)q * ng / m) * WD_C * 3;
+    for (int c = 0; c < 3; c++) {
+      s[q].lo[c] = s[q].hi[c] = x[c];
+      for (int t = 1; t < WD_C; t++) {
+        s[q].lo[c] = x[3 * t + c] < s[q].lo[c] ? x[3 * t + c] : s[q].lo[c];
+        s[q].hi[c] = x[3 * t + c] > s[q].hi[c] ? x[3 * t + c] : s[q].hi[c];
+      }
+    }
+    for (int o = 0; o < q; o++)
+      meet += s[o].lo[0] <= s[q].hi[0] && s[q].lo[0] <= s[o].hi[0] && s[o].lo[1] <= s[q].hi[1] &&
+              s[q].lo[1] <= s[o].hi[1] && s[o].lo[2] <= s[q].hi[2] && s[q].lo[2] <= s[o].hi[2];
+  }
+  return 5 * meet > m * (m - 1);
+}
+
+// Whether a block of ntot cells compares every cell with every point.  Set-up
+// call in ms, every point / walk: 24x16x12 cells, 576 points 0.10 / 0.15;
+// 64x32x32, 1024 points 0.19 / 0.26, 4096 0.60 / 0.65; 90x50x34, 2048 0.33 /
+// 0.37, 3072 0.46 / 0.38; 128x64x64, 576 0.33 / 0.35, 1024 0.55 / 0.54, 16384
+// 8.0 / 2.2; 160x96x80, 256 0.30 / 0.31, 512 0.55 / 0.45.  The same 16384 points
+// in random order: 8.0 / 13.3, shuffled within quarters (about a third of the
+// pairs meet): 8.0 / 7.4.
+inline bool wd_plain(long ntot, int np, bool scattered) {
+  return scattered || (np <= 4096 && np * ntot <= 400000000L);
+}
 
 // boxes of the groups, one warp each, and of WD_S groups, one block of 32 warps each
 __global__ void __launch_bounds__(WD_C* WD_S) k_wd_boxes(const double* __restrict__ pts, int np, WdBox* group,
@@ -418,6 +455,28 @@ FF_DI void wd_group(const double* __restrict__ pts, int np, int g, double x, dou
   }
 }
 
+// Every cell against every point, the points staged through shared memory.
+__global__ void __launch_bounds__(WD_THREADS) k_wall_distance_all(DevBlock b, const double* __restrict__ pts, int np) {
+  __shared__ double sp[WD_TP * 3];
+  const size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool ok = n < (size_t)b.ntot;
+  const double x = ok ? b.a[FF_XC][n] : 0., y = ok ? b.a[FF_YC][n] : 0., z = ok ? b.a[FF_ZC][n] : 0.;
+  double best = 1.e8;
+  for (int t0 = 0; t0 < np; t0 += WD_TP) {
+    const int nt = min(WD_TP, np - t0);
+    __syncthreads();
+    for (int q = threadIdx.x; q < nt * 3; q += blockDim.x) sp[q] = pts[(size_t)t0 * 3 + q];
+    __syncthreads();
+    if (ok)
+      for (int t = 0; t < nt; t++) {
+        const double dx = rs(x, sp[3 * t]), dy = rs(y, sp[3 * t + 1]), dz = rs(z, sp[3 * t + 2]);
+        const double r = ra(ra(rm(dx, dx), rm(dy, dy)), rm(dz, dz));
+        if (r < best) best = r;
+      }
+  }
+  if (ok) b.a[FF_DISTW][n] = __dsqrt_rn(best);
+}
+
 __global__ void __launch_bounds__(WD_THREADS) k_wall_distance(DevBlock b, const double* __restrict__ pts, int np,
                                                               const WdBox* __restrict__ group,
                                                               const WdBox* __restrict__ super) {
@@ -427,26 +486,24 @@ __global__ void __launch_bounds__(WD_THREADS) k_wall_distance(DevBlock b, const 
   const double x = b.a[FF_XC][m], y = b.a[FF_YC][m], z = b.a[FF_ZC][m];
   const int ng = (np + WD_C - 1) / WD_C, nsup = (ng + WD_S - 1) / WD_S;
   double best = 1.e8;
-  if (np > 0) {
-    // a first guess: the nearest group of the nearest super-group
-    int s0 = 0, g0;
-    double near = __longlong_as_double(0x7ff0000000000000LL);
-    for (int s = 0; s < nsup; s++) {
-      const double d = wd_bound(super + s, x, y, z);
-      if (d < near) { near = d; s0 = s; }
-    }
-    near = __longlong_as_double(0x7ff0000000000000LL);
-    g0 = s0 * WD_S;
-    for (int g = s0 * WD_S; g < min(ng, (s0 + 1) * WD_S); g++) {
-      const double d = wd_bound(group + g, x, y, z);
-      if (d < near) { near = d; g0 = g; }
-    }
-    wd_group(pts, np, g0, x, y, z, best);
-    for (int s = 0; s < nsup; s++) {
-      if (!__any_sync(0xffffffffu, wd_bound(super + s, x, y, z) <= best)) continue;
-      for (int g = s * WD_S; g < min(ng, (s + 1) * WD_S); g++)
-        if (__any_sync(0xffffffffu, wd_bound(group + g, x, y, z) <= best)) wd_group(pts, np, g, x, y, z, best);
-    }
+  // a first guess: the nearest group of the nearest super-group
+  int s0 = 0, g0;
+  double near = __longlong_as_double(0x7ff0000000000000LL);
+  for (int s = 0; s < nsup; s++) {
+    const double d = wd_bound(super + s, x, y, z);
+    if (d < near) { near = d; s0 = s; }
+  }
+  near = __longlong_as_double(0x7ff0000000000000LL);
+  g0 = s0 * WD_S;
+  for (int g = s0 * WD_S; g < min(ng, (s0 + 1) * WD_S); g++) {
+    const double d = wd_bound(group + g, x, y, z);
+    if (d < near) { near = d; g0 = g; }
+  }
+  wd_group(pts, np, g0, x, y, z, best);
+  for (int s = 0; s < nsup; s++) {
+    if (!__any_sync(0xffffffffu, wd_bound(super + s, x, y, z) <= best)) continue;
+    for (int g = s * WD_S; g < min(ng, (s + 1) * WD_S); g++)
+      if (__any_sync(0xffffffffu, wd_bound(group + g, x, y, z) <= best)) wd_group(pts, np, g, x, y, z, best);
   }
   if (ok) b.a[FF_DISTW][n] = __dsqrt_rn(best);
 }
