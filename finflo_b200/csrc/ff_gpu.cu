@@ -31,8 +31,9 @@ struct BlockCtx {
   ff_params prm{};
   // LU-SGS, warp wavefront (the default sweep): the records of the upper and
   // the lower sweep, the edge words between tiles and the tile counters, in
-  // the precision lusgs_fp32 asks.  flow_static: the records' face normals
-  // are filled (0 after an allocation or a change of the metrics).
+  // the precision lusgs_fp32 asks (one allocation, at fup).  flow_static: the
+  // records' face normals are filled (0 after an allocation or a change of the
+  // metrics).
   void *fup = nullptr, *flo = nullptr, *fedge = nullptr;
   unsigned* fticket = nullptr;
   FlowGeom fg{};
@@ -504,21 +505,26 @@ int alloc_sweep(Ctx* c, BlockCtx* b) {
   b->sw_static = 0;
   b->flow_static = 0;
   drop(b->sw); drop(b->swl); drop(b->dwp); drop(b->sw32); drop(b->swl32); drop(b->dwp32);
-  drop(b->fup); drop(b->flo); drop(b->fedge);
+  drop(b->fup);
+  b->flo = b->fedge = nullptr;
+  b->fticket = nullptr;
   if (b->prm.ddadi) return 0;
   const bool f32 = b->prm.lusgs_fp32 != 0;
   if (b->use_lines) {
     const int nv = b->prm.iturb >= 3 ? 7 : 5;
     const size_t el = f32 ? sizeof(float) : sizeof(double);
     const size_t nr = flow_rec_len(b->fg, nv) * el, ne = flow_edge_len(b->fg, nv) * el;
-    CK(cudaMalloc(&b->fup, nr));
-    CK(cudaMalloc(&b->flo, nr));
-    CK(cudaMalloc(&b->fedge, ne));
-    if (!b->fticket) CK(cudaMalloc(&b->fticket, 2 * sizeof(unsigned)));
-    CK(cudaMemsetAsync(b->fup, 0, nr, c->stream));
-    CK(cudaMemsetAsync(b->flo, 0, nr, c->stream));
+    // in one piece, the zeroed part in front (four allocations with a fill each
+    // took a tenth of adding a small block); nr and the counters' 256 bytes
+    // leave every part aligned for the bulk copies
+    const size_t nz = 2 * nr + 256;
+    CK(cudaMalloc(&b->fup, nz + ne));
+    char* base = (char*)b->fup;
+    b->flo = base + nr;
+    b->fticket = (unsigned*)(base + 2 * nr);
+    b->fedge = base + nz;
+    CK(cudaMemsetAsync(base, 0, nz, c->stream));
     CK(cudaMemsetAsync(b->fedge, 0xff, ne, c->stream));
-    CK(cudaMemsetAsync(b->fticket, 0, 2 * sizeof(unsigned), c->stream));
     return 0;
   }
   if (f32) {
@@ -1688,7 +1694,7 @@ int ff_destroy(void* ctx) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
     cudaFree(b->base); cudaFree(b->d_patch);
     cudaFree(b->sw); cudaFree(b->swl); cudaFree(b->dwp); cudaFree(b->sw32); cudaFree(b->swl32); cudaFree(b->dwp32);
-    cudaFree(b->fup); cudaFree(b->flo); cudaFree(b->fedge); cudaFree(b->fticket);
+    cudaFree(b->fup);
     cudaFree(b->d_red);
     delete b;
   }
