@@ -496,6 +496,13 @@ void drop(T*& p) {
   p = nullptr;
 }
 
+void drop_sweep(BlockCtx* b) {
+  drop(b->sw); drop(b->swl); drop(b->dwp); drop(b->sw32); drop(b->swl32); drop(b->dwp32);
+  drop(b->fup);
+  b->flo = b->fedge = nullptr;
+  b->fticket = nullptr;
+}
+
 // The buffers of the block's LU-SGS sweep in its precision and equation
 // count (none for DDADI, whose sweeps work in place).  Records start as
 // zeros (slots without a cell stay so), edge words as the mark of a word not
@@ -504,10 +511,7 @@ int alloc_sweep(Ctx* c, BlockCtx* b) {
   const size_t ns = b->ns;
   b->sw_static = 0;
   b->flow_static = 0;
-  drop(b->sw); drop(b->swl); drop(b->dwp); drop(b->sw32); drop(b->swl32); drop(b->dwp32);
-  drop(b->fup);
-  b->flo = b->fedge = nullptr;
-  b->fticket = nullptr;
+  drop_sweep(b);
   if (b->prm.ddadi) return 0;
   const bool f32 = b->prm.lusgs_fp32 != 0;
   if (b->use_lines) {
@@ -581,6 +585,17 @@ int coop_sweep_n(Ctx* c, BlockCtx* b, int upper, bool fp32, int threads) {
 
 int coop_sweep(Ctx* c, BlockCtx* b, int upper, bool fp32) {
   return coop_sweep_n(c, b, upper, fp32, b->coop_threads);
+}
+
+// Whether the sweep's buffers are there: not after an ff_block_params that
+// could not allocate them.
+bool sweep_ready(const BlockCtx* b) {
+  if (b->prm.ddadi) return true;
+  return b->use_lines ? b->fup != nullptr : (b->prm.lusgs_fp32 ? b->dwp32 != nullptr : b->dwp != nullptr);
+}
+int need_sweep(Ctx* c, const BlockCtx* b) {
+  if (sweep_ready(b)) return 0;
+  return fail(c, FF_ERR_CUDA, "no memory for the sweep's data at the last ff_block_params");
 }
 
 constexpr int kMaxDev = 64;
@@ -812,9 +827,13 @@ void sweep_static(Ctx* c, BlockCtx* b, bool fp32) {
 }
 
 // Before a capture: the metric-only sweep data of every block that lacks it.
-void fill_static(Ctx* c) {
-  for (auto* b : c->blocks)
+int fill_static(Ctx* c) {
+  for (auto* b : c->blocks) {
+    int rc = need_sweep(c, b);
+    if (rc) return rc;
     if (!b->prm.ddadi) sweep_static(c, b, b->prm.lusgs_fp32 != 0);
+  }
+  return 0;
 }
 
 // Every captured cycle and phase of the context.
@@ -984,6 +1003,8 @@ int tune_sweep(Ctx* c, BlockCtx* b) {
                     b->prm.ddadi != 0};
   if (b->prm.ddadi) return tune_ddadi(c, b, key);
   if (b->use_lines || b->use_pipe) return 0;
+  int rc = need_sweep(c, b);
+  if (rc) return rc;
   const bool fp32 = b->prm.lusgs_fp32 != 0;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -1002,8 +1023,7 @@ int tune_sweep(Ctx* c, BlockCtx* b) {
     float bt = 0.f;
     for (int rep = 0; rep < 4; rep++) {   // rep 0 warms up
       CK(cudaEventRecord(c->ev0, c->stream));
-      int rc = coop_sweep_n(c, b, 1, fp32, threads[k]);
-      if (rc) return rc;
+      if ((rc = coop_sweep_n(c, b, 1, fp32, threads[k]))) return rc;
       CK(cudaEventRecord(c->ev1, c->stream));
       CK(cudaEventSynchronize(c->ev1));
       float ms = 0.f;
@@ -1121,10 +1141,11 @@ void st_imps_post(Ctx* c, BlockCtx* b, bool divide_cp) {
 }
 
 int st_imps(Ctx* c, BlockCtx* b, int level, bool divide_cp) {
+  int rc = need_sweep(c, b);
+  if (rc) return rc;
   // the warp wavefront takes the time step and the conversion in k_flow_coef
   if (b->prm.ddadi || !b->use_lines) st_imps_pre(c, b);
   bool fp32 = b->prm.lusgs_fp32 != 0;
-  int rc;
   if (b->prm.ddadi) {
     if ((rc = ddadi_sweeps(c, b))) return rc;
   } else {
@@ -1693,8 +1714,7 @@ int ff_destroy(void* ctx) {
   for (auto* b : c->blocks) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
     cudaFree(b->base); cudaFree(b->d_patch);
-    cudaFree(b->sw); cudaFree(b->swl); cudaFree(b->dwp); cudaFree(b->sw32); cudaFree(b->swl32); cudaFree(b->dwp32);
-    cudaFree(b->fup);
+    drop_sweep(b);
     cudaFree(b->d_red);
     delete b;
   }
@@ -1819,16 +1839,19 @@ int ff_block_params(void* ctx, int blk, const ff_params* prm) {
     b->tuned = b->res_tuned = 0;
     b->res_shape = res_rule(c, b);
   }
+  drop_graphs(c);   // captured cycles of any block may include this one (multigrid levels)
+  const ff_params old = b->prm;
   b->prm = *prm;
-  if (nv_changed || fp_changed || dd_changed) {   // the sweep's kernel and buffers
+  if (nv_changed || fp_changed || dd_changed || !sweep_ready(b)) {   // the sweep's kernel and buffers
     int rc = pick_sweep(c, b);
-    if (rc || (rc = alloc_sweep(c, b))) return rc;
+    if (rc || (rc = alloc_sweep(c, b))) {   // the parameters stay; the next call allocates again
+      b->prm = old;
+      drop_sweep(b);
+      cudaGetLastError();
+      return rc;
+    }
   }
   if (nv_changed || fp_changed) b->tuned = 0;
-  // captured cycles of any block may include this one (multigrid levels)
-  for (auto* x : c->blocks)
-    if (x->graph) { cudaGraphExecDestroy(x->graph); x->graph = nullptr; }
-  drop_phase_graphs(c);
   return 0;
 }
 
@@ -2190,7 +2213,7 @@ int ff_cycles(void* ctx, int blk, int ncycles, int icycle0, double* hist, int us
     if (!b->graph || b->graph_fp32 != want) {
       if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
       cudaGraph_t g;
-      fill_static(c);
+      if ((rc = fill_static(c))) return rc;
       CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
       long n0 = c->nlaunch;
       rc = run_cycle(c, b, 2);
@@ -2308,7 +2331,7 @@ int ff_mb_phase(void* ctx, int phase, int icycle, int use_graph) {
   } else {
     if (!c->phase_graph[gi]) {
       cudaGraph_t g;
-      fill_static(c);
+      if ((rc = fill_static(c))) return rc;
       CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
       rc = mb_phase(c, phase, 2);
       cudaError_t e = cudaStreamEndCapture(c->stream, &g);
@@ -2365,7 +2388,7 @@ int ff_cycles_all(void* ctx, int ncycles, int icycle0, double* hist, int use_gra
     if (!c->mb_graph || c->mb_graph_n != nb) {
       if (c->mb_graph) { cudaGraphExecDestroy(c->mb_graph); c->mb_graph = nullptr; }
       cudaGraph_t g;
-      fill_static(c);
+      if ((rc = fill_static(c))) return rc;
       CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
       long n0 = c->nlaunch;
       rc = mb_cycle(c, 2);
@@ -2420,7 +2443,7 @@ int ff_time_stage(void* ctx, int blk, int stage, int reps, float* ms) {
   if (!b || !ms || reps < 1) return fail(c, FF_ERR_ARG, "ff_time_stage");
   if (stage == FF_STAGE_SWEEP) {   // the sweep's kernel choice and (LU-SGS) its data in the sweep layout
     int rc = tune_sweep(c, b);
-    if (rc) return rc;
+    if (rc || (rc = need_sweep(c, b))) return rc;
     if (!b->prm.ddadi) sweep_coef(c, b, 1, b->prm.lusgs_fp32 != 0);
   }
   CK(cudaEventRecord(c->ev0, c->stream));
