@@ -1177,6 +1177,15 @@ void launch_prolong(Ctx* c, BlockCtx* cc, BlockCtx* f) {
   c->nlaunch++;
 }
 
+// FIN of a coarse level in a V-cycle, with the equation of state where a
+// coarser level follows.
+void launch_fin_coarse(Ctx* c, BlockCtx* cc) {
+  const int nb = nblk(cc->ntot, 256);
+  if (cc->coarse) k_fin_coarse<true><<<nb, 256, 0, c->stream>>>(cc->db, cc->prm, 2);
+  else k_fin_coarse<false><<<nb, 256, 0, c->stream>>>(cc->db, cc->prm, 2);
+  c->nlaunch++;
+}
+
 int one_cycle(Ctx* c, BlockCtx* b, int icycle) {
   int rc;
   const bool sst = b->prm.iturb >= 3;
@@ -1245,8 +1254,7 @@ int mg_body(Ctx* c, BlockCtx* b, int icycle, bool own, int part = 0) {
     k_forcing<<<nblk(cc->ntot, 256), 256, 0, c->stream>>>(cc->db, 2, sst);
     c->nlaunch++;
     if ((rc = st_imps(c, cc, (int)m + 1, false))) return rc;
-    k_fin_coarse<<<nblk(cc->ntot, 256), 256, 0, c->stream>>>(cc->db, cc->prm, 2, cc->coarse != nullptr);
-    c->nlaunch++;
+    launch_fin_coarse(c, cc);
   }
   for (size_t m = lv.size() - 1; m >= 1; m--) {
     launch_prolong(c, lv[m], lv[m - 1]);
@@ -1455,8 +1463,7 @@ int mb_mg_body_ls(Ctx* c, int icycle) {
     });
     if (rc || (rc = ls_imps(c, cs, (int)m + 1, false))) return rc;
     rc = fork_n(c, (int)cs.size(), [&](int n) {
-      k_fin_coarse<<<nblk(cs[n]->ntot, 256), 256, 0, c->stream>>>(cs[n]->db, cs[n]->prm, 2, cs[n]->coarse != nullptr);
-      c->nlaunch++;
+      launch_fin_coarse(c, cs[n]);
       return 0;
     });
     if (rc) return rc;
@@ -2172,7 +2179,7 @@ int ff_fin(void* ctx, int blk, double* dromax) {
   k_reset_acc<<<1, 32, 0, c->stream>>>(c->d_resi, c->d_dromax);
   c->nlaunch++;
   if (b->level > 1) {   // coarse level: FIN with the coarse limits (ns3c.f:1935-1990)
-    k_fin_coarse<<<nblk(b->ntot, 256), 256, 0, c->stream>>>(b->db, b->prm, 1, 0);
+    k_fin_coarse<false><<<nblk(b->ntot, 256), 256, 0, c->stream>>>(b->db, b->prm, 1);
     c->nlaunch++;
     if (dromax) *dromax = 0.0;
     CK(cudaGetLastError());
