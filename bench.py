@@ -48,14 +48,13 @@ WORKLOADS = {
 
 
 # DRAM bytes (read + write) of one launch of the dominant kernel, from one
-# ncu capture of the same workload (profiles/k_residual_fused_sstmg128x64x64_full.md:
-# 244.6 MB read + 25.4 MB written, 16x8x4-cell tiles).
-TRAFFIC = {"sst-mg": 270.0e6}
+# ncu capture of a block of the workload's size (16x4x4-cell tiles, two CTAs an
+# SM: 254.4 MB read + 28.5 MB written).
+TRAFFIC = {"sst-mg": 282.9e6}
 # DRAM bytes (read + write) per cell of one FP64 LU-SGS sweep
 # (k_flow_sweep<double,7>) in the multi-block cycle, from an ncu capture of
-# the same eight-block case at 256x128x64 cells (profiles/
-# k_flow_sweep_8blk_256x128x64_dram.md); a launch's traffic scales with its
-# block's cells
+# the same eight-block case at 256x128x64 cells; a launch's traffic scales
+# with its block's cells
 SWEEP_TRAFFIC_PER_CELL = 281.0
 
 
@@ -309,7 +308,7 @@ def run_ours(args):
         chosen = f"pipelined tile wavefront, {lk // 100} tiles"
     else:
         chosen = f"cooperative hyperplane, {lk // 100} threads/CTA"
-    sweep = dict(g.sweep_tuning(bid), chosen=chosen, ms_per_sweep=ms_sweep)
+    sweep = dict(chosen=chosen, ms_per_sweep=ms_sweep)
     if args.ddadi:   # the tuner's PRED+CORR time per direction
         t = g.sweep_tuning(bid)
         sweep = dict(chosen=chosen, ms_per_stage=ms_sweep, ms_k=t["pipe_ms"], ms_i=t["lines_ms"],
@@ -345,7 +344,8 @@ def run_ours(args):
                    "l2": "state resident in HBM; per-cycle working set above L2 at the default size",
                    "lusgs_sweep": sweep},
         "gpu_launches": launches,
-        "roofline": {"bound": "hbm", "kernel": "k_residual_fused<7,512>" if prms[0].iturb >= 3 else "k_residual_fused<5,512>",
+        "roofline": {"bound": "hbm", "kernel": f"k_residual_fused<{7 if prms[0].iturb >= 3 else 5}>, "
+                                               f"tiles of {g.residual_shape(bid)} cells",
                      "achieved": achieved, "peak": peak, "peak_kind": pkind, "unit": "GB/s",
                      "frac": achieved / peak,
                      "traffic": TRAFFIC.get(args.workload) if not args.grid else None,
@@ -649,7 +649,7 @@ def run_large(args):
                      "frac": achieved_sweep / peak,
                      "traffic": None if fp32 else SWEEP_TRAFFIC_PER_CELL * fine_cells[big], "ms_per_launch": ms_sweep,
                      "bytes_per_cell": sweep_bpc, "cells": fine_cells[big]},
-        "residual": {"kernel": "k_residual_fused<7,512> (largest block, alone)", "ms_per_launch": ms_res,
+        "residual": {"kernel": "k_residual_fused<7> (largest block, alone)", "ms_per_launch": ms_res,
                      "tile": g.residual_shape(big * nlev),
                      "bytes_per_cell": 328.0, "achieved_gbs": achieved, "frac": achieved / peak},
         "e2e": {"value": e2e, "unit": "cell-iters/s", "h2d_bytes_per_step": h2d // max(1, nsteps_e2e),

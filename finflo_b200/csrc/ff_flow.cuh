@@ -24,8 +24,9 @@
 // 0.134 ms).  Loading the next record into registers a step ahead made the
 // step longer (0.156 ms at 16 x 8), as did a step barrier split into arrival
 // and wait on an mbarrier.  One sweep, B200: 128x64x64 cells, seven equations,
-// 0.114 ms in FP64 and 0.099 ms in FP32 (cluster lines 0.588 ms); 64x32x32,
-// five equations, 0.046 ms (0.223 ms); 248x136x72, seven, 0.249 ms.
+// 0.118 ms in FP64 and 0.103 ms in FP32 (cluster lines 0.588 ms); 64x32x32,
+// five equations, 0.047 ms (0.223 ms); 248x136x72, seven, 0.251 ms (the mean of
+// a hundred in a row; the shapes above were timed in one run of their own).
 //
 // Between CTAs the products of the edge lines go through global memory (L2)
 // and carry their own arrival: every word of the edge buffer holds a mark (all

@@ -63,11 +63,10 @@ struct BlockCtx {
   int pipe_tk = 0;              // its tile height along k (8, 16 or 32 lines)
   bool pipe_stage = false;
   PipeGeom pg{};
-  float pipe_ms = 0.f;          // measured upper sweep of the pipelined kernel
   int tuned = 0;                // sweep kind chosen by tune_sweep
   int res_shape = 0;            // residual form (RES_FORMS), chosen by tune_residual
   int res_tuned = 0;
-  float sweep_ms[2] = {0.f, 0.f};   // measured upper sweep: lines, best hyperplane
+  float hyp_ms = 0.f;           // measured upper sweep of the hyperplane kernel
   DevBlock db{};
   cudaGraphExec_t graph = nullptr;
   int graph_fp32 = -1;
@@ -874,7 +873,7 @@ void sweep_coef(Ctx* c, BlockCtx* b, int upper, bool fp32) {
 // GPU, at the fastest of 64/128/256 threads per CTA, timed here) run only
 // where FINFLO_LUSGS=pipe|hyperplane asks for them: both were slower on every
 // block shape tried (128x64x64 SST, FP64, one sweep: warp wavefront
-// 0.114 ms, pipelined 0.74 ms, hyperplanes 2.2 ms).
+// 0.118 ms, pipelined 0.74 ms, hyperplanes 2.2 ms).
 // DDADI kernel shapes: the prefetch depth and CTA size of the one thread
 // per line kernels, and the (lines per CTA, cells per chunk) of the
 // producer/consumer kernels the autotuner chooses from.
@@ -895,8 +894,8 @@ struct TuneKey {
   }
 };
 struct TuneVal {
-  int use_pipe, use_lines, coop_threads, dd_cfg;
-  float pipe_ms, lines_ms, hyp_ms;
+  int coop_threads = 0, dd_cfg = 0;   // hyperplane sweep; DDADI forms (i, j, k as decimal digits)
+  float ms[3] = {0.f, 0.f, 0.f};      // hyperplane sweep; DDADI i, j, k
 };
 std::map<TuneKey, TuneVal> g_tune_cache;
 std::mutex g_tune_mu;
@@ -920,7 +919,7 @@ int tune_ddadi(Ctx* c, BlockCtx* b, const TuneKey& key) {
     if (it != g_tune_cache.end()) {
       const int packed = it->second.dd_cfg;
       b->dd_cfg[1] = packed / 100; b->dd_cfg[2] = (packed / 10) % 10; b->dd_cfg[3] = packed % 10;
-      b->dd_ms[1] = it->second.pipe_ms; b->dd_ms[2] = it->second.lines_ms; b->dd_ms[3] = it->second.hyp_ms;
+      for (int d = 1; d <= 3; d++) b->dd_ms[d] = it->second.ms[d - 1];
       return 0;
     }
   }
@@ -946,8 +945,8 @@ int tune_ddadi(Ctx* c, BlockCtx* b, const TuneKey& key) {
     b->dd_ms[d] = best_ms;
   }
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  g_tune_cache[key] = TuneVal{0, 0, 0, b->dd_cfg[1] * 100 + b->dd_cfg[2] * 10 + b->dd_cfg[3],
-                              b->dd_ms[1], b->dd_ms[2], b->dd_ms[3]};
+  g_tune_cache[key] = TuneVal{0, b->dd_cfg[1] * 100 + b->dd_cfg[2] * 10 + b->dd_cfg[3],
+                              {b->dd_ms[1], b->dd_ms[2], b->dd_ms[3]}};
   return 0;
 }
 
@@ -1011,7 +1010,7 @@ int tune_sweep(Ctx* c, BlockCtx* b) {
     auto it = g_tune_cache.find(key);
     if (it != g_tune_cache.end()) {
       b->coop_threads = it->second.coop_threads;
-      b->sweep_ms[1] = it->second.hyp_ms;
+      b->hyp_ms = it->second.ms[0];
       return 0;
     }
   }
@@ -1035,10 +1034,10 @@ int tune_sweep(Ctx* c, BlockCtx* b) {
   int herr = 0;
   CK(cudaMemcpy(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (herr) return fail(c, FF_ERR_TIMEOUT, "sweep autotune: a bounded wait gave up");
-  b->sweep_ms[1] = best;
+  b->hyp_ms = best;
   b->coop_threads = best_t;
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  g_tune_cache[key] = TuneVal{0, 0, best_t, 0, 0.f, 0.f, best};
+  g_tune_cache[key] = TuneVal{best_t, 0, {best, 0.f, 0.f}};
   return 0;
 }
 
@@ -1377,8 +1376,7 @@ int fork_join(Ctx* c, int nb, F fn) {
 }
 
 // fn(n) for n < cnt on side streams, forked from and joined back into the
-// context stream, with no sweep inside (the lockstep cycle's per-block
-// stages between its batched sweeps).
+// context stream (the lockstep cycle's per-block stages, sweeps included).
 template <typename F>
 int fork_n(Ctx* c, int cnt, F fn) {
   if (cnt <= 1) return cnt == 1 ? fn(0) : 0;
@@ -2246,8 +2244,8 @@ int ff_cycles(void* ctx, int blk, int ncycles, int icycle0, double* hist, int us
 int ff_sweep_tuning(void* ctx, int blk, float* ms2) {
   BlockCtx* b = getb((Ctx*)ctx, blk);
   if (!b || !ms2) return FF_ERR_ARG;
-  ms2[0] = b->sweep_ms[0];
-  ms2[1] = b->sweep_ms[1];
+  ms2[0] = 0.f;
+  ms2[1] = b->hyp_ms;
   return 0;
 }
 
@@ -2259,9 +2257,8 @@ int ff_sweep_times(void* ctx, int blk, float* ms3) {
     ms3[0] = b->dd_ms[3]; ms3[1] = b->dd_ms[1]; ms3[2] = b->dd_ms[2];
     return 0;
   }
-  ms3[0] = b->pipe_ms;
-  ms3[1] = b->sweep_ms[0];
-  ms3[2] = b->sweep_ms[1];
+  ms3[0] = ms3[1] = 0.f;
+  ms3[2] = b->hyp_ms;
   return 0;
 }
 

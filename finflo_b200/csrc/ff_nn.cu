@@ -7,10 +7,13 @@
 //                 elected thread per CTA, operands staged in shared memory
 //                 in the canonical K-major core-matrix layout, completion
 //                 through an mbarrier, accumulator read back with
-//                 tcgen05.ld); split-K with FP32 atomics for the weight
-//                 gradients, whose reduction runs over all voxels.
-//   element-wise  SiLU backward, column sums (bias gradients), transposes,
-//                 casts, mean-squared-error gradient, Adam.
+//                 tcgen05.ld): k_gemm_rows for many rows against one small
+//                 matrix, else k_gemm_bf16 (with split-K and FP32 atomics
+//                 where a caller asks for it; the network does not).
+//   ffnn_wgrad    G[N,K] += X[R,N]^T Y[R,K], the weight gradients.
+//   element-wise  SiLU backward and mean-squared-error gradient, each also
+//                 with the bias gradient in the same pass (the network's
+//                 form), column sums, transposes, casts, Adam.
 //
 // Every device wait is bounded: on time-out the kernel sets the error word,
 // waits (bounded) for its own tensor-core work, frees its tensor memory and

@@ -16,12 +16,12 @@ constexpr double SST_SIGRK1 = 0.85, SST_SIGOM1 = 0.5, SST_BETA2 = 0.0828, SST_SI
 
 // ---- before the face pass -------------------------------------------------
 // The steps of TURBEQ and RESIKE before the face fluxes in two kernels and one
-// of two arrays (they were eight): what bounds them is memory, and DERFUN, CROSKO and TEMDER of k
-// and omega each read the twelve face-metric arrays, the volume and the
-// thicknesses.  128x64x64 cells, one level-1 pass: k_grad 57.4, k_eps2ko 10.7,
+// of two arrays (they were eight): what bounds them is memory, and DERFUN,
+// CROSKO and TEMDER of k and omega each read the twelve face-metric arrays, the
+// volume and the thicknesses.  128x64x64 cells, one level-1 pass: k_grad 57.4, k_eps2ko 10.7,
 // k_crosko 27.8, k_rk_roundtrip 7.0, k_cdmax 6.7, k_fun1ko 11.2, k_prodke 11.0,
-// k_temder_ke 73.8 us before; k_pre_ke 62.9, k_temder_fun 35.9 us now.  The two are
-// apart because FUN1KO needs the largest cross diffusion of the block and
+// k_temder_ke 73.8 us before; k_pre_ke 63.5, k_rk_roundtrip 7.9, k_temder_fun 39.3
+// us now.  The two are apart because FUN1KO needs the largest cross diffusion of the block and
 // TEMDER the wall ghosts REFCEN fills in between.
 //
 // CROSKO divides RK and REPS by RO in place and multiplies them back, which
@@ -630,18 +630,20 @@ __global__ void k_sourko_addske(DevBlock b) {
   b.a[FF_DEPS][L] = b.a[FF_DEPS][L] + som;
 }
 
-// RESIDU/RESIKE for a 32x4x4 tile with all three directions' faces in one
-// work list: the k, i and j faces (640 + 528 + 640) are computed by NT
+// RESIDU/RESIKE for a tile with all three directions' faces in one work list:
+// the k, i and j faces (640 + 528 + 640 of a 32x4x4 tile) are computed by NT
 // threads into one shared-memory face buffer with a single barrier, then
 // each cell sums its six faces in the reference order (k, i, j, then
 // 1/VOL, SWEEP res3c.f:992 / SWEEPK res3c.f:1342).  Against one barrier per
-// direction this balances the face work over the threads (8 rounds for the
-// 1808 faces at 256 threads, against 3 + 3 + 3) and drops two barriers.
+// direction this balances the face work over the threads and drops two
+// barriers.
 //
-// The tile shape (TI_ x TJ_ x TK_ cells, 512 of them) is a template
-// parameter: 32x4x4, 16x8x4 and 8x8x8 trade i-direction coalescing against
-// the faces computed per cell (3.53, 3.44, 3.38); the autotuner picks one
-// per block shape.
+// The tile shape (TI_ x TJ_ x TK_ cells) and the threads are template
+// parameters; RES_FORMS lists the forms, the autotuner or res_rule picks one
+// per block: 512 cells trade i-direction coalescing against the faces
+// computed per cell (32x4x4 3.53, 16x8x4 3.44, 8x8x8 3.38), 256 cells on 256
+// threads (8x8x4 and 16x4x4, 3.5 and 3.56) put two CTAs on an SM, 8x4x4 (3.63)
+// is one round of 512 threads.
 //
 // STAGE: the MUSCL variables (RO, U, V, W, P(, RK, REPS)) of the tile's
 // cells and of the two cells beyond each of its six faces are first copied

@@ -232,14 +232,13 @@ int ff_time_cycles_all(void *ctx, int ncycles, float *ms, int *launches_per_cycl
 int ff_cycle_launches(void *ctx, int blk);
 /* LU-SGS sweep kernel of a block: 1 + 100*CTAs = line wavefront of warps
  * (the default), 2 + 100*threads_per_CTA = cooperative hyperplane kernel. */
-/* The measured upper-sweep times in ms {lines, fastest cooperative
- * hyperplane} of a block, zero for a kernel that was not timed: the line
- * wavefront is taken without timing it, the hyperplane kernel's CTA size is
- * timed at the first ff_cycles call where FINFLO_LUSGS asks for it. */
+/* The measured upper-sweep time of a block in ms, {0, cooperative hyperplane}:
+ * the hyperplane kernel's CTA size is timed at the first ff_cycles call where
+ * FINFLO_LUSGS asks for that kernel (0 otherwise); the line wavefront is taken
+ * without timing it (ff_time_stage times one). */
 int ff_sweep_tuning(void *ctx, int blk, float *ms2);
-/* The measured upper-sweep times in ms {pipelined tile wavefront, lines,
- * fastest cooperative hyperplane} (zero where not timed).  LU-SGS kind 3 +
- * 100*tiles = the pipelined tile wavefront.
+/* The same as {0, 0, cooperative hyperplane}.  LU-SGS kind 3 + 100*tiles = the
+ * pipelined tile wavefront.
  * DDADI blocks (prm->ddadi = 1): the tuned PRED+CORR time per direction
  * {k, i, j}, and kind 4 + 100*(1000 + 100*fk + 10*fi + fj) with f the
  * chosen producer/consumer form per direction (0: 32 lines x 4 cells per

@@ -196,8 +196,8 @@ def test_fp32_lusgs_converges_to_fp64_answer(gpu_lib):
 
 @pytest.mark.parametrize("dims", [(33, 33, 33), (17, 65, 65)])
 def test_line_and_hyperplane_sweeps_agree(gpu_lib, dims, monkeypatch):
-    """The cluster line-wavefront LU-SGS and the cooperative hyperplane kernel
-    solve the same triangular systems."""
+    """The line-wavefront LU-SGS and the cooperative hyperplane kernel solve the
+    same triangular systems."""
     g1, b1, bg1, o, bc, prm = _setup(*dims)
     assert g1.lusgs_kind(b1) % 100 == 1
     monkeypatch.setenv("FINFLO_LUSGS", "hyperplane")
