@@ -644,10 +644,12 @@ def run_large(args):
         "gpu_launches": per_cycle * args.steps,
         # one upper LU-SGS sweep of the largest block, timed alone (the residual, beside it, has the
         # larger share of the cycle since the sweep became a wavefront of warps)
-        "roofline": {"bound": "hbm", "kernel": "k_flow_sweep<double,7> (upper sweep, largest block)",
+        "roofline": {"bound": "hbm",
+                     "kernel": "k_ddadi_pc (all line sweeps, largest block)" if args.ddadi else
+                               f"k_flow_sweep<{'float' if fp32 else 'double'},7> (upper sweep, largest block)",
                      "achieved": achieved_sweep, "peak": peak, "peak_kind": pkind, "unit": "GB/s",
                      "frac": achieved_sweep / peak,
-                     "traffic": None if fp32 else SWEEP_TRAFFIC_PER_CELL * fine_cells[big], "ms_per_launch": ms_sweep,
+                     "traffic": None if fp32 or args.ddadi else SWEEP_TRAFFIC_PER_CELL * fine_cells[big], "ms_per_launch": ms_sweep,
                      "bytes_per_cell": sweep_bpc, "cells": fine_cells[big]},
         "residual": {"kernel": "k_residual_fused<7> (largest block, alone)", "ms_per_launch": ms_res,
                      "tile": g.residual_shape(big * nlev),
