@@ -1847,7 +1847,10 @@ int ff_block_params(void* ctx, int blk, const ff_params* prm) {
   drop_graphs(c);   // captured cycles of any block may include this one (multigrid levels)
   const ff_params old = b->prm;
   b->prm = *prm;
-  if (nv_changed || fp_changed || dd_changed || !sweep_ready(b)) {   // the sweep's kernel and buffers
+  // the sweep's kernel and buffers; a change to DDADI keeps them, for a host that goes back and forth
+  if (b->prm.ddadi) {
+    if (nv_changed || fp_changed) drop_sweep(b);
+  } else if (nv_changed || fp_changed || !sweep_ready(b)) {
     int rc = pick_sweep(c, b);
     if (rc || (rc = alloc_sweep(c, b))) {   // the parameters stay; the next call allocates again
       b->prm = old;
