@@ -127,6 +127,19 @@ int fail(Ctx* c, int code, const char* what, cudaError_t e = cudaSuccess) {
     if (e_ != cudaSuccess) return fail(c, FF_ERR_CUDA, #call, e_); \
   } while (0)
 
+// Device memory; where there is none left, the set-up scratch that the context
+// keeps is given back first (the set-up calls are synchronous: nothing uses it).
+template <typename T>
+cudaError_t dev_malloc(Ctx* c, T** p, size_t bytes) {
+  cudaError_t e = cudaMalloc((void**)p, bytes);
+  if (e != cudaErrorMemoryAllocation || !c->setup) return e;
+  cudaGetLastError();
+  cudaFree(c->setup);
+  c->setup = nullptr;
+  c->setup_bytes = 0;
+  return cudaMalloc((void**)p, bytes);
+}
+
 inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 
 BlockCtx* getb(Ctx* c, int blk) {
@@ -521,7 +534,7 @@ int alloc_sweep(Ctx* c, BlockCtx* b) {
     // took a tenth of adding a small block); nr and the counters' 256 bytes
     // leave every part aligned for the bulk copies
     const size_t nz = 2 * nr + 256;
-    CK(cudaMalloc(&b->fup, nz + ne));
+    CK(dev_malloc(c, &b->fup, nz + ne));
     char* base = (char*)b->fup;
     b->flo = base + nr;
     b->fticket = (unsigned*)(base + 2 * nr);
@@ -531,13 +544,13 @@ int alloc_sweep(Ctx* c, BlockCtx* b) {
     return 0;
   }
   if (f32) {
-    CK(cudaMalloc(&b->sw32, sizeof(float) * SW_N * ns));
-    CK(cudaMalloc(&b->swl32, sizeof(float) * SW_N * ns));
-    CK(cudaMalloc(&b->dwp32, sizeof(float) * 7 * ns));
+    CK(dev_malloc(c, &b->sw32, sizeof(float) * SW_N * ns));
+    CK(dev_malloc(c, &b->swl32, sizeof(float) * SW_N * ns));
+    CK(dev_malloc(c, &b->dwp32, sizeof(float) * 7 * ns));
   } else {
-    CK(cudaMalloc(&b->sw, sizeof(double) * SW_N * ns));
-    CK(cudaMalloc(&b->swl, sizeof(double) * SW_N * ns));
-    CK(cudaMalloc(&b->dwp, sizeof(double) * 7 * ns));
+    CK(dev_malloc(c, &b->sw, sizeof(double) * SW_N * ns));
+    CK(dev_malloc(c, &b->swl, sizeof(double) * SW_N * ns));
+    CK(dev_malloc(c, &b->dwp, sizeof(double) * 7 * ns));
   }
   return 0;
 }
@@ -1317,12 +1330,12 @@ int ensure_conn(Ctx* c) {
   if (c->d_blocks) cudaFree(c->d_blocks);
   if (c->d_conn) cudaFree(c->d_conn);
   c->d_blocks = nullptr; c->d_conn = nullptr;
-  CK(cudaMalloc(&c->d_blocks, sizeof(DevBlock) * max(1, nb)));
+  CK(dev_malloc(c, &c->d_blocks, sizeof(DevBlock) * max(1, nb)));
   CK(cudaMemcpy(c->d_blocks, tab.data(), sizeof(DevBlock) * nb, cudaMemcpyHostToDevice));
   c->nconn = (int)items.size();
   c->maxconn = maxn;
   if (c->nconn) {
-    CK(cudaMalloc(&c->d_conn, sizeof(ConnItem) * c->nconn));
+    CK(dev_malloc(c, &c->d_conn, sizeof(ConnItem) * c->nconn));
     CK(cudaMemcpy(c->d_conn, items.data(), sizeof(ConnItem) * c->nconn, cudaMemcpyHostToDevice));
   }
   while (c->side.size() < c->tops.size()) {
@@ -1662,7 +1675,7 @@ int run_cycle(Ctx* c, BlockCtx* b, int icycle) {
 int ensure_hist(Ctx* c, int n) {
   if (n <= c->hist_cap) return 0;
   if (c->d_hist) cudaFree(c->d_hist);
-  CK(cudaMalloc(&c->d_hist, sizeof(double) * 6 * n));
+  CK(dev_malloc(c, &c->d_hist, sizeof(double) * 6 * n));
   c->hist_cap = n;
   for (auto* b : c->blocks)
     if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
@@ -1686,13 +1699,13 @@ int ff_create(void** out, int device) {
   *out = nullptr;
   CK(cudaSetDevice(device));
   CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-  CK(cudaMalloc(&c->d_bar, 2 * sizeof(unsigned)));
+  CK(dev_malloc(c, &c->d_bar, 2 * sizeof(unsigned)));
   CK(cudaMemsetAsync(c->d_bar, 0, 2 * sizeof(unsigned), c->stream));
-  CK(cudaMalloc(&c->d_err, sizeof(int)));
+  CK(dev_malloc(c, &c->d_err, sizeof(int)));
   CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-  CK(cudaMalloc(&c->d_resi, 16 * sizeof(double)));
-  CK(cudaMalloc(&c->d_dromax, sizeof(unsigned long long)));
-  CK(cudaMalloc(&c->d_hist_pos, sizeof(int)));
+  CK(dev_malloc(c, &c->d_resi, 16 * sizeof(double)));
+  CK(dev_malloc(c, &c->d_dromax, sizeof(unsigned long long)));
+  CK(dev_malloc(c, &c->d_hist_pos, sizeof(int)));
   CK(cudaMemsetAsync(c->d_hist_pos, 0, sizeof(int), c->stream));
   CK(cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device));
   CK(cudaDeviceGetAttribute(&c->smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
@@ -1785,15 +1798,15 @@ static int block_add(Ctx* c, int imax, int jmax, int kmax, int npatch, const ff_
     }
   }
   b->patch_own = patches_own(b);
-  CK(cudaMalloc(&b->base, sizeof(double) * b->slot_stride * FF_NSLOTS));
+  CK(dev_malloc(c, &b->base, sizeof(double) * b->slot_stride * FF_NSLOTS));
   CK(cudaMemsetAsync(b->base, 0, sizeof(double) * b->slot_stride * FF_NSLOTS, c->stream));
   if (npatch) {
-    CK(cudaMalloc(&b->d_patch, sizeof(ff_patch) * npatch));
+    CK(dev_malloc(c, &b->d_patch, sizeof(ff_patch) * npatch));
     CK(cudaMemcpyAsync(b->d_patch, patches, sizeof(ff_patch) * npatch, cudaMemcpyHostToDevice, c->stream));
   }
   b->ns = sw_size(imax, jmax, kmax);
   b->fg = flow_geom(imax, jmax, kmax);
-  CK(cudaMalloc(&b->d_red, sizeof(unsigned long long) * 2));
+  CK(dev_malloc(c, &b->d_red, sizeof(unsigned long long) * 2));
   b->db.imax = imax; b->db.jmax = jmax; b->db.kmax = kmax;
   b->db.is = imax + 4; b->db.il = (imax + 4) * (jmax + 4); b->db.ntot = b->ntot;
   b->db.npatch = npatch; b->db.patch = b->d_patch;
@@ -2315,7 +2328,7 @@ int ff_halo_plan(void* ctx, int nitems, const ff_halo_item* items, double* send_
   if (c->d_halo) cudaFree(c->d_halo);
   c->d_halo = nullptr;
   if (nitems) {
-    CK(cudaMalloc(&c->d_halo, sizeof(HaloItem) * nitems));
+    CK(dev_malloc(c, &c->d_halo, sizeof(HaloItem) * nitems));
     CK(cudaMemcpy(c->d_halo, h.data(), sizeof(HaloItem) * nitems, cudaMemcpyHostToDevice));
   }
   c->nhalo = nitems; c->halo_maxn = maxn; c->halo_pack = pk; c->halo_unpack = up;

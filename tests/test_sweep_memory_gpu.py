@@ -19,14 +19,14 @@ NAMES = ["DRO", "DM", "DN", "DW", "DE"]
 
 
 @contextlib.contextmanager
-def _full_device():
-    """The device's free memory taken up to some 16 MB (the driver's own needs)."""
-    held, n = [], torch.cuda.mem_get_info()[0] - (16 << 20)
+def _full_device(spare=16 << 20):
+    """The device's free memory taken up to a few MB more than `spare` (the driver's own needs)."""
+    held, n = [], torch.cuda.mem_get_info()[0] - spare
     try:
-        while n >= 1 << 22:
+        while n >= 1 << 21:
             try:
                 held.append(torch.empty(n, dtype=torch.uint8, device="cuda"))
-                n = torch.cuda.mem_get_info()[0] - (16 << 20)
+                n = torch.cuda.mem_get_info()[0] - spare
             except torch.OutOfMemoryError:
                 n //= 2
         yield
@@ -104,4 +104,24 @@ def test_change_of_equations_without_memory(gpu_lib):
     got = g.download(bid, NAMES)
     for n in NAMES:
         np.testing.assert_array_equal(got[n], want[n])
+    g.close()
+
+
+def test_a_block_takes_the_memory_of_the_setup_scratch(gpu_lib):
+    """The set-up calls keep their scratch; a block that needs it gets it."""
+    from finflo_b200 import case, grid
+    nodes = grid.bump_nodes(97, 65, 65)
+    big, _, prm, _ = make_pair(97, 65, 65)
+    g = GpuSolver(0)
+    bid = g.add_block(big, prm)
+    g.block_metrics(bid, *nodes)          # keeps 3 x (nodes + extended nodes) = 21 MB
+    small, sprm, _ = case.bump_case(16, 9, 9)
+    g.add_block(small, sprm)
+    g.sync()
+    with _full_device(spare=1 << 20):
+        mid, mprm, _ = case.bump_case(25, 17, 17)   # 9 MB of arrays and records
+        nid = g.add_block(mid, mprm)
+        g.upload(nid)
+        g.start(nid)
+        assert np.isfinite(g.download(nid, ["RO"])["RO"]).all()
     g.close()
